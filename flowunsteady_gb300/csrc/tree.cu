@@ -9,9 +9,9 @@
 //      particles whose codes differ is split at the first 3-bit Morton digit
 //      where they differ (so no single-child chains), children are appended
 //      with an atomic counter; cells are contiguous ranges of sorted particles;
-//   3. upward pass, deepest generation first: leaves take their bounding box,
-//      largest core and moments (order P) from their particles, parents from
-//      their children (box union; moments shifted to the parent centre);
+//   3. upward pass: leaves take their bounding box, largest core and moments
+//      (order P) from their particles, then, deepest generation first, parents
+//      from their children (box union; moments shifted to the parent centre);
 //   4. targets are taken in groups of 64 consecutive particles of the Morton
 //      order (compact boxes, one full CTA each).  The walk for a group is
 //      split over the subtrees of a frontier of at most 73 cells (the leaves
@@ -51,9 +51,9 @@
 namespace vpm {
 
 constexpr int kMaxGen = 23;        // root + at most 21 Morton digits (+1 spare)
-// Device counters: cells, leaves, error flags, target groups, then the first
+// Device counters: cells, leaves, error flags, finished blocks of the running split, then the first
 // cell of every generation (generation g starts at counters[kGenBase + g]).
-constexpr int kCntCells = 0, kCntLeaves = 1, kCntFlags = 2, kCntGroups = 3, kGenBase = 4;
+constexpr int kCntCells = 0, kCntLeaves = 1, kCntFlags = 2, kCntDone = 3, kGenBase = 4;
 constexpr int kNumCounters = kGenBase + kMaxGen + 2;
 constexpr int kStack = 256;        // traversal stack (cells)
 // Target group size (consecutive particles of the Morton order).  32-particle
@@ -86,7 +86,7 @@ struct FmmWork {
   int* counters = nullptr;    // see kCntCells .. kGenBase
   int64_t meta_cap = 0;       // (group, frontier cell) walk slots
   float4* ggeom = nullptr;    // target-group boxes (centre, radius), FP32
-  float4* cgeom = nullptr;    // walk records, two per cell (see cell_walk_kernel)
+  float4* cgeom = nullptr;    // walk records, two per cell (see write_cell_geom)
   int* front = nullptr;       // frontier cells (walk roots)
   unsigned long long* pairs = nullptr;   // [0] near source pairs, [1] far (target, cell) pairs
   double* box = nullptr;      // bounding cube: min x y z, size
@@ -230,7 +230,7 @@ __global__ void tree_init_kernel(int64_t n, int* lo, int* hi, int* counters) {
   counters[kCntCells] = 1;
   counters[kCntLeaves] = 0;
   counters[kCntFlags] = 0;
-  counters[kCntGroups] = 0;
+  counters[kCntDone] = 0;
   counters[kGenBase + 0] = 0;   // generation 0 is the root
   counters[kGenBase + 1] = 1;
 }
@@ -245,68 +245,73 @@ __device__ __forceinline__ int lower_bound_code(const uint64_t* codes, int lo, i
   return lo;
 }
 
-// Split or close the cells of generation g.
+// Split or close the cells of generation g, eight lanes per cell: lane v finds
+// where Morton digit v begins, so that the seven binary searches of a cell (16
+// to 20 dependent loads each) run side by side.  One thread per cell walked them
+// one after another: 38 µs a generation at N = 60,000 against 12 µs.  The last
+// block to finish closes generation g + 1, which ends where the cells appended
+// here end (a launch of its own before).
 __global__ void tree_split_kernel(int g, int ncrit, int64_t cell_cap, const uint64_t* __restrict__ codes,
                                   int* lo, int* hi, int* child, int* nchild, int* leaves,
                                   int* counters) {
   const int begin = counters[kGenBase + g], end = counters[kGenBase + g + 1];
-  for (int cell = begin + int(blockIdx.x * blockDim.x + threadIdx.x); cell < end;
-       cell += int(gridDim.x * blockDim.x)) {
-    const int a = lo[cell], b = hi[cell];
-    const uint64_t first = codes[a], last = codes[b - 1];
-    if (b - a <= ncrit || first == last) {
-      child[cell] = -1;
-      nchild[cell] = 0;
-      leaves[atomicAdd(&counters[kCntLeaves], 1)] = cell;
-      continue;
+  const int lane = threadIdx.x & 31, v = lane & 7, base = lane & ~7;
+  const int per = int(blockDim.x) / 8;
+  for (int c0 = begin + int(blockIdx.x) * per; c0 < end; c0 += int(gridDim.x) * per) {
+    const int cell = c0 + int(threadIdx.x) / 8;
+    const bool valid = cell < end;
+    int a = 0, b = 0;
+    uint64_t first = 0, last = 0;
+    if (valid) {
+      a = lo[cell];
+      b = hi[cell];
+      first = codes[a];
+      last = codes[b - 1];
     }
-    const int bit = 63 - __clzll((long long)(first ^ last));   // highest differing bit
-    const int shift = (bit / 3) * 3;                            // its Morton digit
-    const uint64_t prefix = first & ~((uint64_t(8) << shift) - 1);
-    int bounds[9];
-    bounds[0] = a;
-    bounds[8] = b;
-    for (int v = 1; v < 8; ++v) bounds[v] = lower_bound_code(codes, a, b, prefix | (uint64_t(v) << shift));
-    int nc = 0;
-    for (int v = 0; v < 8; ++v) nc += bounds[v + 1] > bounds[v];
-    const int first_child = atomicAdd(&counters[kCntCells], nc);
-    if (first_child + nc > cell_cap) {
-      atomicOr(&counters[kCntFlags], 1);
-      child[cell] = -1;
-      nchild[cell] = 0;
-      continue;
+    const bool split = valid && b - a > ncrit && first != last;
+    int bound = a;
+    if (split && v > 0) {
+      const int bit = 63 - __clzll((long long)(first ^ last));   // highest differing bit
+      const int shift = (bit / 3) * 3;                            // its Morton digit
+      const uint64_t prefix = first & ~((uint64_t(8) << shift) - 1);
+      bound = lower_bound_code(codes, a, b, prefix | (uint64_t(v) << shift));
     }
-    int k = first_child;
-    for (int v = 0; v < 8; ++v) {
-      if (bounds[v + 1] > bounds[v]) {
-        lo[k] = bounds[v];
-        hi[k] = bounds[v + 1];
-        ++k;
-      }
+    int next = __shfl_down_sync(0xffffffffu, bound, 1);
+    if (v == 7) next = b;
+    const bool some = split && next > bound;
+    const unsigned mask = (__ballot_sync(0xffffffffu, some) >> base) & 0xffu;
+    const int nc = __popc(mask);
+    int first_child = 0;
+    if (valid && v == 0) {
+      if (split) first_child = atomicAdd(&counters[kCntCells], nc);
+      else leaves[atomicAdd(&counters[kCntLeaves], 1)] = cell;
     }
-    child[cell] = first_child;
-    nchild[cell] = nc;
+    first_child = __shfl_sync(0xffffffffu, first_child, base);
+    const bool fits = split && first_child + nc <= cell_cap;
+    if (some && fits) {
+      const int k = first_child + __popc(mask & ((1u << v) - 1u));
+      lo[k] = bound;
+      hi[k] = next;
+    }
+    if (valid && v == 0) {
+      child[cell] = fits ? first_child : -1;
+      nchild[cell] = fits ? nc : 0;
+      if (split && !fits) atomicOr(&counters[kCntFlags], 1);
+    }
   }
-}
-
-// Generation g+1 ends where the cells appended while splitting generation g end.
-__global__ void tree_advance_kernel(int g, int* counters) {
-  counters[kGenBase + g + 2] = counters[kCntCells];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&counters[kCntDone], 1) == int(gridDim.x) - 1) {
+      counters[kGenBase + g + 2] = atomicAdd(&counters[kCntCells], 0);
+      counters[kCntDone] = 0;
+    }
+  }
 }
 
 // ------------------------------------------------------------ upward pass --
 // Cell geometry record (8 doubles): box min x y z, box max x y z, σmax, unused.
 constexpr int kGeom = 8;
-
-// Binomial coefficient, iteratively: a recursive form becomes a recursive
-// device call wherever the loops around it are not fully unrolled, and
-// recursion has no static stack bound.
-__host__ __device__ constexpr int binom(int n, int k) {
-  if (k < 0 || k > n) return 0;
-  int r = 1;
-  for (int i = 1; i <= k; ++i) r = r * (n - k + i) / i;
-  return r;
-}
 
 __device__ __forceinline__ void cell_centre(const double* g, double& cx, double& cy, double& cz,
                                             double& r) {
@@ -317,167 +322,278 @@ __device__ __forceinline__ void cell_centre(const double* g, double& cx, double&
   r = sqrt(ex * ex + ey * ey + ez * ez);
 }
 
-// Binomial coefficients C(n, k) for n, k <= 6 (the largest order is 6), as a
-// table: the moment shift's loops are too large to unroll completely, and a
-// binomial formed at run time costs integer divisions in its innermost loop.
-__constant__ double c_binom[7][7] = {
-    {1, 0, 0, 0, 0, 0, 0},   {1, 1, 0, 0, 0, 0, 0},    {1, 2, 1, 0, 0, 0, 0},
-    {1, 3, 3, 1, 0, 0, 0},   {1, 4, 6, 4, 1, 0, 0},    {1, 5, 10, 10, 5, 1, 0},
-    {1, 6, 15, 20, 15, 6, 1}};
+// Smallest and largest of a double over the warp, on the order-preserving integer
+// image of its bits: FP64 comparisons would queue on GB300's FP64 pipe (about two
+// operations per SM and cycle).
+__device__ __forceinline__ long long order_key(double x) {
+  const long long b = __double_as_longlong(x);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+__device__ __forceinline__ double order_value(long long k) {
+  return __longlong_as_double(k ^ ((k >> 63) & 0x7fffffffffffffffll));
+}
+__device__ __forceinline__ bool is_nan(double x) {
+  return (__double_as_longlong(x) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+}
+__device__ __forceinline__ long long warp_min_key(long long k) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) k = min(k, __shfl_xor_sync(0xffffffffu, k, o));
+  return k;
+}
+__device__ __forceinline__ long long warp_max_key(long long k) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) k = max(k, __shfl_xor_sync(0xffffffffu, k, o));
+  return k;
+}
 
-// Cells of generation g: leaves from their particles, parents from their
-// children (which belong to later generations, already done).  One thread per
-// (cell, vorticity component m): the three threads of a cell form the same box;
-// the one with m = 0 writes it.
+// Bounding box of the particles [lo, hi) of the sorted rows, by one warp; every
+// lane gets it in g[0..5], and the largest core (sorted row 6) in g[6].
+__device__ __forceinline__ void warp_box(const double* __restrict__ sorted, int64_t ldw, int64_t lo,
+                                         int64_t hi, double (&g)[8]) {
+  long long mn[3], mx[3], ms = order_key(0.0);
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    mn[d] = order_key(INFINITY);
+    mx[d] = order_key(-INFINITY);
+  }
+  for (int64_t i = lo + (threadIdx.x & 31); i < hi; i += 32) {
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const double x = sorted[d * ldw + i];
+      if (is_nan(x)) continue;   // a diverged particle does not widen the box
+      const long long k = order_key(x);
+      mn[d] = min(mn[d], k);
+      mx[d] = max(mx[d], k);
+    }
+    const double sg = sorted[6 * ldw + i];
+    if (!is_nan(sg)) ms = max(ms, order_key(sg));
+  }
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    g[d] = order_value(warp_min_key(mn[d]));
+    g[3 + d] = order_value(warp_max_key(mx[d]));
+  }
+  g[6] = order_value(warp_max_key(ms));
+  g[7] = 0.0;
+}
+
+// Exponents (a, b, c) of every multi-index |k| <= 6 in graded order, packed as
+// a | b << 4 | c << 8 (computed at compile time).
+struct MidxTable {
+  short v[ncoef(6)];
+};
+constexpr MidxTable make_midx_table() {
+  MidxTable t{};
+  for (int n = 0; n <= 6; ++n)
+    for (int a = n; a >= 0; --a)
+      for (int b = n - a; b >= 0; --b) t.v[midx(a, b, n - a - b)] = short(a | b << 4 | (n - a - b) << 8);
+  return t;
+}
+__constant__ MidxTable c_midx = make_midx_table();
+__constant__ double c_fact[7] = {1, 1, 2, 6, 24, 120, 720};
+__constant__ double c_ifact[7] = {1, 1, 0.5, 1.0 / 6, 1.0 / 24, 1.0 / 120, 1.0 / 720};
+
+// What the upward kernels write for a cell: its box, FP64 moments, their FP32 copy
+// (momf, where given) and its walk record.
+struct CellOut {
+  double* geom;
+  double* mom;
+  float* momf;
+  float4* walk;
+};
+
+// Walk record of a cell, two float4 read together by the traversal:
+//   rec[2c]     = centre x, y, z and radius (FP32, inflated by 1e-6 of the
+//                 coordinates' magnitude so that rounding cannot shrink it);
+//   rec[2c + 1] = largest core (FP32), then as integer bits: the first child
+//                 (or the first particle of a leaf), the end of the cell's
+//                 particle range, the number of children (0 for a leaf).
+__device__ __forceinline__ void write_cell_geom(const CellOut& o, int cell, const double (&g)[8],
+                                                int first, int end, int nc) {
+  double* gc = o.geom + int64_t(cell) * kGeom;
+#pragma unroll
+  for (int d = 0; d < 8; ++d) gc[d] = g[d];
+  double cx, cy, cz, r;
+  cell_centre(g, cx, cy, cz, r);
+  const double pad = 1e-6 * (fabs(cx) + fabs(cy) + fabs(cz) + r);
+  o.walk[2 * int64_t(cell)] = make_float4(float(cx), float(cy), float(cz), float(r + pad));
+  o.walk[2 * int64_t(cell) + 1] = make_float4(float(g[6]), __int_as_float(first),
+                                              __int_as_float(end), __int_as_float(nc));
+}
+
+// The upward pass is FP64 sums of a few thousand terms per cell, on a pipe that
+// retires about two of them per SM and cycle: what matters is that a cell's sums
+// run side by side and not as one thread's chain.  One thread per (cell, component)
+// took 1.66 ms of a treecode evaluation at N = 60,000 (eight launches of 160 to
+// 300 µs, each the length of one chain); these two kernels take 0.26 ms (leaves
+// 51 µs, a generation of parents 22 to 61 µs).
+//
+// Leaves, one warp each: lane = particle forms the box and the monomials
+// (y - c)^k, then lane = (component, k) sums Γ^m (y - c)^k over the particles in
+// their order.
+constexpr int kLeafWarps = 4;
 template <int P>
-__global__ void tree_upward_kernel(int g, const int* __restrict__ counters, const int* __restrict__ lo,
-                                   const int* __restrict__ hi, const int* __restrict__ child,
-                                   const int* __restrict__ nchild, const double* __restrict__ sorted,
-                                   int64_t ldw, double* geom, double* mom) {
-  constexpr int NC = ncoef(P);
-  const int begin = counters[kGenBase + g], end = counters[kGenBase + g + 1];
-  const int64_t nwork = int64_t(end - begin) * 3;
-  for (int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < nwork;
-       t += int64_t(gridDim.x) * blockDim.x) {
-    const int cell = begin + int(t / 3), m = int(t % 3);
-    double* gc = geom + int64_t(cell) * kGeom;
-    const int nc = nchild[cell];
-    double bx[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
-    double smax = 0.0;
-    bool bad = false;
-    if (nc == 0) {
-      for (int i = lo[cell]; i < hi[cell]; ++i) {
+__global__ void __launch_bounds__(32 * kLeafWarps) tree_leaf_kernel(
+    int nleaves, const int* __restrict__ leaves, const int* __restrict__ lo,
+    const int* __restrict__ hi, const double* __restrict__ sorted, int64_t ldw, CellOut out) {
+  constexpr int NC = ncoef(P), ROUNDS = (3 * NC + 31) / 32;
+  constexpr int CH = P > 4 ? 16 : 32;   // particles staged at a time
+  __shared__ double s_pw[kLeafWarps][CH][NC], s_g[kLeafWarps][CH][3];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int l = int(blockIdx.x) * kLeafWarps + wid;
+  if (l >= nleaves) return;
+  const int cell = leaves[l], a = lo[cell], b = hi[cell];
+  double g[8];
+  warp_box(sorted, ldw, a, b, g);
+  if (lane == 0) write_cell_geom(out, cell, g, a, b, 0);
+  double cx, cy, cz, rad;
+  cell_centre(g, cx, cy, cz, rad);
+  double acc[ROUNDS];
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          const double x = sorted[d * ldw + i];
-          bx[d] = fmin(bx[d], x);
-          bx[3 + d] = fmax(bx[3 + d], x);
-        }
-        smax = fmax(smax, sorted[6 * ldw + i]);
-      }
-    } else {
-      for (int k = 0; k < nc; ++k) {
-        if (child[cell] + k >= counters[kCntCells]) {
-          atomicOr(const_cast<int*>(&counters[kCntFlags]), 32);
-          bad = true;
-          break;
-        }
-        const double* gk = geom + int64_t(child[cell] + k) * kGeom;
+  for (int r = 0; r < ROUNDS; ++r) acc[r] = 0.0;
+  for (int i0 = a; i0 < b; i0 += CH) {
+    const int cnt = min(CH, b - i0);
+    __syncwarp();
+    if (lane < cnt) {
+      const int i = i0 + lane;
+      double pw[NC];
+      monomials<P, double>(sorted[i] - cx, sorted[ldw + i] - cy, sorted[2 * ldw + i] - cz, pw);
 #pragma unroll
-        for (int d = 0; d < 3; ++d) {
-          bx[d] = fmin(bx[d], gk[d]);
-          bx[3 + d] = fmax(bx[3 + d], gk[3 + d]);
-        }
-        smax = fmax(smax, gk[6]);
+      for (int k = 0; k < NC; ++k) s_pw[wid][lane][k] = pw[k];
+#pragma unroll
+      for (int m = 0; m < 3; ++m) s_g[wid][lane][m] = sorted[(3 + m) * ldw + i];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int r = 0; r < ROUNDS; ++r) {
+      const int e = lane + 32 * r;
+      if (e < 3 * NC) {
+        const int m = e / NC, k = e - m * NC;
+        for (int i = 0; i < cnt; ++i) acc[r] += s_g[wid][i][m] * s_pw[wid][i][k];
       }
     }
-    if (m == 0) {
+  }
 #pragma unroll
-      for (int d = 0; d < 6; ++d) gc[d] = bx[d];
-      gc[6] = smax;
-      gc[7] = 0.0;
+  for (int r = 0; r < ROUNDS; ++r) {
+    const int e = lane + 32 * r;
+    if (e < 3 * NC) {
+      out.mom[int64_t(cell) * 3 * NC + e] = acc[r];
+      if (out.momf) out.momf[int64_t(cell) * 3 * NC + e] = float(acc[r]);
     }
-    double cx, cy, cz, rad;
-    {
-      double b8[8] = {bx[0], bx[1], bx[2], bx[3], bx[4], bx[5], smax, 0.0};
-      cell_centre(b8, cx, cy, cz, rad);
-    }
-    double* mc = mom + int64_t(cell) * 3 * NC;
-    double acc[NC];
-#pragma unroll
-    for (int k = 0; k < NC; ++k) acc[k] = 0.0;
-    if (nc == 0) {
-      for (int i = lo[cell]; i < hi[cell]; ++i) {
-        double pw[NC];
-        monomials<P, double>(sorted[i] - cx, sorted[ldw + i] - cy, sorted[2 * ldw + i] - cz, pw);
-        const double gm = sorted[(3 + m) * ldw + i];
-#pragma unroll
-        for (int k = 0; k < NC; ++k) acc[k] += gm * pw[k];
-      }
-    } else if (!bad) {
-      for (int q = 0; q < nc; ++q) {
-        const int ch = child[cell] + q;
-        double qx, qy, qz, qr;
-        cell_centre(geom + int64_t(ch) * kGeom, qx, qy, qz, qr);
-        double tp[NC];
-        monomials<P, double>(qx - cx, qy - cy, qz - cz, tp);
-        const double* mq = mom + int64_t(ch) * 3 * NC + m * NC;
-        // (y - c)^k = Σ_{j<=k} C(k, j) (y - c_q)^j (c_q - c)^{k-j}
-#pragma unroll
-        for (int n = 0; n <= P; ++n)
-#pragma unroll
-          for (int a = n; a >= 0; --a)
-#pragma unroll
-            for (int b = n - a; b >= 0; --b) {
-              const int c = n - a - b;
-              double s = 0.0;
-#pragma unroll
-              for (int ja = 0; ja <= a; ++ja)
-#pragma unroll
-                for (int jb = 0; jb <= b; ++jb)
-#pragma unroll
-                  for (int jc = 0; jc <= c; ++jc)
-                    s += c_binom[a][ja] * c_binom[b][jb] * c_binom[c][jc] *
-                         tp[midx(a - ja, b - jb, c - jc)] * mq[midx(ja, jb, jc)];
-              acc[midx(a, b, c)] += s;
-            }
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < NC; ++k) mc[m * NC + k] = acc[k];
   }
 }
 
-__global__ void moments_to_f32_kernel(int64_t n, const double* __restrict__ a, float* b) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i < n) b[i] = float(a[i]);
+// Parents of generation g from their children (of later generations, already
+// done), one CTA per cell.  The moment shift
+//   M_k/k! = Σ_{children q} Σ_{j<=k} (M_j^q/j!) (c_q - c)^{k-j}/(k-j)!
+// runs with one thread per (coefficient slot, child slot); kUpSlots child slots
+// are summed in order at the end.
+constexpr int kUpSlots = 4, kUpThreads = 128;
+template <int P>
+__global__ void __launch_bounds__(kUpThreads * kUpSlots) tree_upward_kernel(
+    int g, int* counters, const int* __restrict__ hi, const int* __restrict__ child,
+    const int* __restrict__ nchild, CellOut out) {
+  constexpr int NC = ncoef(P), NE = 3 * NC;
+  __shared__ double s_m[8][NE], s_t[8][NC], s_box[8][8], s_geom[8];
+  __shared__ double s_sum[kUpSlots - 1][NE];
+  const int tid = threadIdx.x, slot = tid / kUpThreads, tl = tid - slot * kUpThreads;
+  const int begin = counters[kGenBase + g], end = counters[kGenBase + g + 1];
+  const int total = counters[kCntCells];
+  for (int cell = begin + int(blockIdx.x); cell < end; cell += int(gridDim.x)) {
+    int nc = nchild[cell];
+    const int ch = child[cell];
+    if (nc == 0) continue;   // a leaf: done by tree_leaf_kernel
+    if (nc > 8 || ch < 0 || ch + nc > total) {   // outside the tree: record, skip
+      if (tid == 0) atomicOr(&counters[kCntFlags], 32);
+      continue;
+    }
+    __syncthreads();   // the previous cell is done with shared memory
+    if (tid < 8 * nc) s_box[tid >> 3][tid & 7] = out.geom[int64_t(ch + (tid >> 3)) * kGeom + (tid & 7)];
+    for (int e = tid; e < nc * NE; e += blockDim.x) {
+      const int q = e / NE, r = e - q * NE;
+      const int x = c_midx.v[r % NC];
+      s_m[q][r] = out.mom[int64_t(ch) * NE + e] *
+                  (c_ifact[x & 15] * c_ifact[(x >> 4) & 15] * c_ifact[x >> 8]);
+    }
+    __syncthreads();
+    if (tid < 7) {
+      double v = s_box[0][tid];
+      for (int q = 1; q < nc; ++q) {
+        const double u = s_box[q][tid];
+        v = (tid < 3 ? order_key(u) < order_key(v) : order_key(u) > order_key(v)) ? u : v;
+      }
+      s_geom[tid] = v;
+    }
+    if (tid == 7) s_geom[7] = 0.0;
+    __syncthreads();
+    // (c_q - c)^k / k!
+    for (int e = tid; e < nc * NC; e += blockDim.x) {
+      const int q = e / NC, k = e - q * NC, x = c_midx.v[k];
+      double f = 1.0;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const int ex = (x >> (4 * d)) & 15;
+        const double dd = 0.5 * (s_box[q][d] + s_box[q][3 + d]) - 0.5 * (s_geom[d] + s_geom[3 + d]);
+        double w = c_ifact[ex];
+        for (int i = 0; i < ex; ++i) w *= dd;
+        f *= w;
+      }
+      s_t[q][k] = f;
+    }
+    if (tid == 0) {
+      double gg[8];
+#pragma unroll
+      for (int d = 0; d < 8; ++d) gg[d] = s_geom[d];
+      write_cell_geom(out, cell, gg, ch, hi[cell], nc);
+    }
+    __syncthreads();
+    for (int e0 = 0; e0 < NE; e0 += kUpThreads) {
+      const int e = e0 + tl;
+      double acc = 0.0;
+      int x = 0;
+      if (e < NE) {
+        const int m = e / NC;
+        x = c_midx.v[e - m * NC];
+        const int a = x & 15, b = (x >> 4) & 15, c = x >> 8;
+        for (int q = slot; q < nc; q += kUpSlots) {
+          const double* mq = s_m[q] + m * NC;
+          const double* tq = s_t[q];
+          for (int ja = 0; ja <= a; ++ja)
+            for (int jb = 0; jb <= b; ++jb)
+              for (int jc = 0; jc <= c; ++jc)
+                acc += tq[midx(a - ja, b - jb, c - jc)] * mq[midx(ja, jb, jc)];
+        }
+        if (slot > 0) s_sum[slot - 1][e] = acc;
+      }
+      __syncthreads();
+      if (slot == 0 && e < NE) {
+#pragma unroll
+        for (int q = 0; q < kUpSlots - 1; ++q) acc += s_sum[q][e];
+        acc *= c_fact[x & 15] * c_fact[(x >> 4) & 15] * c_fact[x >> 8];
+        out.mom[int64_t(cell) * NE + e] = acc;
+        if (out.momf) out.momf[int64_t(cell) * NE + e] = float(acc);
+      }
+    }
+  }
 }
 
 // -------------------------------------------------------------- traversal --
 // Targets are taken in groups of kTreeBlock consecutive particles of the Morton
 // order (the last one shorter): compact boxes, full CTAs.  Each group's box
-// (centre, radius) and each cell's (centre, radius) and largest core go to
-// FP32 records for the walk; radii are inflated by 1e-6 of the coordinates'
-// magnitude so that rounding cannot shrink them.
+// (centre, radius) goes to an FP32 record for the walk, by one warp per group;
+// radii are inflated by 1e-6 of the coordinates' magnitude so that rounding
+// cannot shrink them.
 __global__ void group_geom_kernel(int64_t n, const double* __restrict__ sorted, int64_t ldw,
                                   float4* ggeom) {
-  const int64_t g = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t g = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32;
   const int64_t a = g * kTreeBlock;
   if (a >= n) return;
-  const int64_t b = a + kTreeBlock < n ? a + kTreeBlock : n;
-  double bx[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
-  for (int64_t i = a; i < b; ++i)
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      const double x = sorted[d * ldw + i];
-      bx[d] = fmin(bx[d], x);
-      bx[3 + d] = fmax(bx[3 + d], x);
-    }
+  double bx[8];
+  warp_box(sorted, ldw, a, a + kTreeBlock < n ? a + kTreeBlock : n, bx);
   double cx, cy, cz, r;
   cell_centre(bx, cx, cy, cz, r);
   const double pad = 1e-6 * (fabs(cx) + fabs(cy) + fabs(cz) + r);
-  ggeom[g] = make_float4(float(cx), float(cy), float(cz), float(r + pad));
-}
-
-// Walk record of cell c, two float4 read together by the traversal:
-//   rec[2c]     = centre x, y, z and radius (FP32, inflated as above);
-//   rec[2c + 1] = largest core (FP32), then as integer bits: the first child
-//                 (or the first particle of a leaf), the end of a leaf's
-//                 particle range, the number of children (0 for a leaf).
-__global__ void cell_walk_kernel(int ncells, const double* __restrict__ geom,
-                                 const int* __restrict__ lo, const int* __restrict__ hi,
-                                 const int* __restrict__ child, const int* __restrict__ nchild,
-                                 float4* rec) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncells) return;
-  double cx, cy, cz, r;
-  cell_centre(geom + int64_t(c) * kGeom, cx, cy, cz, r);
-  const double pad = 1e-6 * (fabs(cx) + fabs(cy) + fabs(cz) + r);
-  rec[2 * c] = make_float4(float(cx), float(cy), float(cz), float(r + pad));
-  const int nc = nchild[c];
-  rec[2 * c + 1] = make_float4(float(geom[int64_t(c) * kGeom + 6]),
-                               __int_as_float(nc == 0 ? lo[c] : child[c]), __int_as_float(hi[c]),
-                               __int_as_float(nc));
+  if ((threadIdx.x & 31) == 0) ggeom[g] = make_float4(float(cx), float(cy), float(cz), float(r + pad));
 }
 
 // One thread per (target group g, frontier cell j), t = g·nfront + j: the
@@ -1313,11 +1429,20 @@ cudaError_t reserve_particles(FmmWork* w, int64_t n) {
   return cudaSuccess;
 }
 
+// Leaves, then the parents generation by generation, the deepest first; returns
+// the launches.
 template <int P>
-void launch_upward(FmmWork* w, int g, int ncells_in_gen, int64_t ldw, cudaStream_t st) {
-  const int grid = std::max(1, std::min((3 * ncells_in_gen + 63) / 64, 4096));
-  tree_upward_kernel<P><<<grid, 64, 0, st>>>(g, w->counters, w->lo, w->hi, w->child, w->nchild,
-                                             w->sorted, ldw, w->geom, w->mom);
+int launch_upward(FmmWork* w, int nleaves, int last_gen, bool f64, int64_t ldw, cudaStream_t st) {
+  const CellOut out = {w->geom, w->mom, f64 ? nullptr : w->momf, w->cgeom};
+  tree_leaf_kernel<P><<<(nleaves + kLeafWarps - 1) / kLeafWarps, 32 * kLeafWarps, 0, st>>>(
+      nleaves, w->leaves, w->lo, w->hi, w->sorted, ldw, out);
+  int launches = 1;
+  for (int g = last_gen - 1; g >= 0; --g, ++launches) {
+    const int ncells_in_gen = w->h_counters[kGenBase + g + 1] - w->h_counters[kGenBase + g];
+    tree_upward_kernel<P><<<std::min(ncells_in_gen, 4096), kUpThreads * kUpSlots, 0, st>>>(
+        g, w->counters, w->hi, w->child, w->nchild, out);
+  }
+  return launches;
 }
 
 template <int P, int Q>
@@ -1437,9 +1562,8 @@ cudaError_t fmm_eval(vpm_ctx* c, int kernel, int prec, int p, int ncrit, double 
   for (int g = 0; g < kMaxGen - 1; ++g) {
     tree_split_kernel<<<split_grid, 256, 0, st>>>(g, ncrit, w->cell_cap, codes, w->lo, w->hi,
                                                   w->child, w->nchild, w->leaves, w->counters);
-    tree_advance_kernel<<<1, 1, 0, st>>>(g, w->counters);
   }
-  if ((e = launched(1 + 2 * (kMaxGen - 1))) != cudaSuccess) return e;
+  if ((e = launched(1 + (kMaxGen - 1))) != cudaSuccess) return e;
   int* hc = w->h_counters;
   e = cudaMemcpyAsync(hc, w->counters, sizeof(int) * kNumCounters, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -1454,14 +1578,22 @@ cudaError_t fmm_eval(vpm_ctx* c, int kernel, int prec, int p, int ncrit, double 
   int nfront = 0;
   {
     const int g2 = hc[kGenBase + 2], g3 = hc[kGenBase + 3];
-    std::vector<int> nch(g2);
+    std::vector<int> nch(g2), first(g3);
     e = cudaMemcpy(nch.data(), w->nchild, sizeof(int) * g2, cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess)
+      e = cudaMemcpy(first.data(), w->lo, sizeof(int) * g3, cudaMemcpyDeviceToHost);
     if (e != cudaSuccess) return e;
     int hf[kMaxFront];
     for (int cidx = 0; cidx < g2 && nfront < kMaxFront; ++cidx)
       if (nch[cidx] == 0) hf[nfront++] = cidx;
     const int leaves01 = nfront;
     for (int cidx = g2; cidx < g3 && nfront < kMaxFront; ++cidx) hf[nfront++] = cidx;
+    // Cells of a generation are numbered as the atomic counter handed them out;
+    // the roots go in Morton order, so that the lists (and the order of every
+    // sum over them) are the same in every evaluation.
+    auto morton = [&](int x, int y) { return first[x] < first[y]; };
+    std::sort(hf, hf + leaves01, morton);
+    std::sort(hf + leaves01, hf + nfront, morton);
     if (nfront == 0 || nfront != leaves01 + (g3 - g2)) {   // at most 9 + 64 by construction
       *why = "tree frontier larger than expected";
       return cudaErrorInvalidValue;
@@ -1493,24 +1625,13 @@ cudaError_t fmm_eval(vpm_ctx* c, int kernel, int prec, int p, int ncrit, double 
   int last_gen = 0;
   for (int g = 0; g < kMaxGen; ++g)
     if (hc[kGenBase + g + 1] > hc[kGenBase + g]) last_gen = g;
-  for (int g = last_gen; g >= 0; --g) {
-    const int cnt = hc[kGenBase + g + 1] - hc[kGenBase + g];
-    if (cnt <= 0) continue;
-    if (p == 2) launch_upward<2>(w, g, cnt, ldw, st);
-    else if (p == 4) launch_upward<4>(w, g, cnt, ldw, st);
-    else launch_upward<6>(w, g, cnt, ldw, st);
-    if ((e = launched(1)) != cudaSuccess) return e;
-  }
-  if (!f64) {
-    const int64_t nm = int64_t(ncells) * 3 * NC;
-    moments_to_f32_kernel<<<int((nm + 255) / 256), 256, 0, st>>>(nm, w->mom, w->momf);
-    if ((e = launched(1)) != cudaSuccess) return e;
-  }
-
-  cell_walk_kernel<<<(ncells + 255) / 256, 256, 0, st>>>(ncells, w->geom, w->lo, w->hi, w->child,
-                                                         w->nchild, w->cgeom);
-  group_geom_kernel<<<(ngroups + 127) / 128, 128, 0, st>>>(n, w->sorted, ldw, w->ggeom);
-  if ((e = launched(2)) != cudaSuccess) return e;
+  // (The deepest generation holds only leaves.)
+  if (p == 2) e = launched(launch_upward<2>(w, nleaves, last_gen, f64, ldw, st));
+  else if (p == 4) e = launched(launch_upward<4>(w, nleaves, last_gen, f64, ldw, st));
+  else e = launched(launch_upward<6>(w, nleaves, last_gen, f64, ldw, st));
+  if (e != cudaSuccess) return e;
+  group_geom_kernel<<<(ngroups + 7) / 8, 256, 0, st>>>(n, w->sorted, ldw, w->ggeom);
+  if ((e = launched(1)) != cudaSuccess) return e;
 
   // 4. interaction lists: count, scan, fill
   stage = "traversal";

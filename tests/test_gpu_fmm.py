@@ -206,3 +206,26 @@ def test_sfs_passes_from_treecode_match_direct(analytic):
     assert rel_l2(U1, U0) <= 1e-4 and rel_l2(J1, J0) <= 1e-4
     assert rel_l2(E1, E0) <= 1e-3, rel_l2(E1, E0)
     assert rel_l2(C1[:, 0], C0[:, 0]) <= (1e-2 if analytic else 1e-12), rel_l2(C1[:, 0], C0[:, 0])
+
+
+@pytest.mark.parametrize("n,ncrit,p", [(1, 50, 4), (33, 1, 2), (700, 33, 4), (1500, 64, 6),
+                                       (5000, 50, 6), (5000, 1, 4)])
+def test_upward_pass_at_the_edges_of_its_warps_and_slots(oracle, n, ncrit, p):
+    # Leaves below, at and above a warp of particles, one-particle leaves, parents
+    # with few and many children, every order.  With θ = 0.2 a term of the
+    # expansion in R/d of order p + 1 is left out, at most (p + 3)² θ^(p+1) of the
+    # field for J (two derivatives of order p + 3); a moment of a lower order that
+    # is missing or misplaced shows at θ^1 .. θ^p.
+    X, G, S = uniform_box(n, seed_index=142)
+    S = S * 1e-3    # so that the cores keep no cell from being far
+    U0, J0 = oracle.uj_direct(1, X, G, S)
+    bound = (p + 3) ** 2 * 0.2 ** (p + 1)
+    with Ctx(n) as c:
+        c.set(X, G, S)
+        U, J = eval_fmm(c, 1, L.PREC_FP64, fmm(p=p, ncrit=ncrit, theta=0.2))
+        U2, J2 = eval_fmm(c, 1, L.PREC_FP64, fmm(p=p, ncrit=ncrit, theta=0.2))
+        if n >= 5000:
+            assert stats(c)[2] > 0
+    assert np.array_equal(U, U2) and np.array_equal(J, J2)
+    if n > 1:
+        assert rel_l2(U, U0) <= bound and rel_l2(J, J0) <= bound
