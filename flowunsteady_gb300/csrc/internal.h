@@ -108,8 +108,6 @@ struct Shape {
 // Launch one pair pass (grid chosen by the caller through args/n_items).
 cudaError_t launch_pair(int pass, int kernel, int precision, Shape shape, const PairArgs& a,
                         int grid, cudaStream_t st);
-// Dynamic shared memory of a shape (bytes).
-size_t pair_smem_bytes(int pass, int precision, Shape shape);
 // Clusters of `cluster` CTAs of a shape that fit on the device at once (0: the
 // shape cannot run as such clusters; only FP32C shapes do).
 int pair_max_active_clusters(int pass, int kernel, int precision, Shape shape, int cluster);
@@ -144,15 +142,14 @@ cudaError_t launch_reduce(int pass, int kernel, int precision, const double* par
                           int scalar_chunks, int64_t t_begin, int64_t t_end, double* u,
                           double* j, double* dj, int64_t ldo, cudaStream_t st);
 
-// The D passes live in pair_d.cu; launch_pair/launch_reduce/pair_ctas_per_sm/
-// pair_smem_bytes forward to these for PASS_UJD and PASS_ZETAD.
+// The D passes live in pair_d.cu; launch_pair/launch_reduce/pair_ctas_per_sm
+// forward to these for PASS_UJD and PASS_ZETAD.
 cudaError_t launch_pair_d(int pass, int kernel, int precision, Shape shape, const PairArgs& a,
                           int grid, cudaStream_t st);
 cudaError_t launch_reduce_d(int pass, int kernel, int precision, const double* part, int64_t ldp,
                             const int64_t* foff, const int32_t* fchunks, int nfields,
                             int scalar_chunks, int64_t t_begin, int64_t t_end, double* u,
                             double* j, double* dj, int64_t ldo, cudaStream_t st);
-size_t pair_smem_bytes_d(int pass, int precision, Shape shape);
 int pair_ctas_per_sm_d(int pass, int kernel, int precision, Shape shape);
 
 }  // namespace vpm

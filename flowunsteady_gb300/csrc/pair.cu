@@ -10,12 +10,6 @@ bool pair_shape_supported(int precision, Shape s) {
   return (s.block == 128 && (s.tpt == 2 || s.tpt == 4)) || (s.block == 256 && s.tpt == 2);
 }
 
-size_t pair_smem_bytes(int pass, int precision, Shape s) {
-  if (pass == PASS_UJ) return smem_of<PASS_UJ>(precision, s);
-  if (pass == PASS_ZETA) return smem_of<PASS_ZETA>(precision, s);
-  return pair_smem_bytes_d(pass, precision, s);
-}
-
 int pair_ctas_per_sm(int pass, int kernel, int precision, Shape s) {
   if (pass == PASS_UJ) return ctas_per_sm<PASS_UJ>(kernel, precision, s);
   if (pass == PASS_ZETA) return ctas_per_sm<PASS_ZETA>(kernel, precision, s);

@@ -4,10 +4,6 @@
 
 namespace vpm {
 
-size_t pair_smem_bytes_d(int pass, int precision, Shape s) {
-  return pass == PASS_UJD ? smem_of<PASS_UJD>(precision, s) : smem_of<PASS_ZETAD>(precision, s);
-}
-
 int pair_ctas_per_sm_d(int pass, int kernel, int precision, Shape s) {
   return pass == PASS_UJD ? ctas_per_sm<PASS_UJD>(kernel, precision, s)
                           : ctas_per_sm<PASS_ZETAD>(kernel, precision, s);

@@ -35,6 +35,7 @@
 #include <type_traits>
 
 #include "internal.h"
+#include "pair_f64.cuh"
 #include "update.h"
 #include "vpm_device.cuh"
 
@@ -52,8 +53,10 @@ struct PairTraits {
   static constexpr int kNval = nval_of(PASS);
   static constexpr bool kUJ = PASS == PASS_UJ || PASS == PASS_UJD;
   static constexpr bool kD = PASS == PASS_UJD || PASS == PASS_ZETAD;
-  // shared quads per source: (x, a), (Γ, b), and for ζ passes v_q (and w_q)
-  static constexpr int kQuads = kUJ ? 2 : (PASS == PASS_ZETA ? 3 : 4);
+  // shared quads per source: (x, a), (Γ, b), for ζ passes v_q (and w_q), for the
+  // FP64 U/J passes further constants of the source
+  static constexpr int kQuads =
+      kUJ ? (PREC == VPM_PREC_FP64 ? 3 : 2) : (PASS == PASS_ZETA ? 3 : 4);
   // The FP32 passes read packed source records (pack_sources_kernel for U/J,
   // pack_zeta_sources_kernel for ζ); the plain U/J pass stages them with bulk
   // copies.
@@ -72,13 +75,28 @@ __host__ __device__ constexpr size_t box_bytes(int block) {
   return PREC == VPM_PREC_FP64 ? 0 : size_t(block / 32) * 4 * 16;
 }
 
-template <int PASS, int PREC>
+// FP64 Gaussian-erf: the core table (U/J) and the exponential's (ζ, α-derivatives).
+template <int PASS, int KERNEL, int PREC>
+__host__ __device__ constexpr size_t core_table_doubles() {
+  return PREC == VPM_PREC_FP64 && KERNEL == VPM_KERNEL_GAUSSIANERF && PairTraits<PASS, PREC>::kUJ
+             ? size_t(kCoreRows) * kCoreCoef
+             : 0;
+}
+template <int PASS, int KERNEL, int PREC>
+__host__ __device__ constexpr size_t exp2_table_doubles() {
+  return PREC == VPM_PREC_FP64 && KERNEL == VPM_KERNEL_GAUSSIANERF && PASS != PASS_UJ
+             ? size_t(kExp2Rows)
+             : 0;
+}
+
+template <int PASS, int KERNEL, int PREC>
 __host__ __device__ constexpr size_t smem_bytes(int block, int tpt) {
   using Tr = PairTraits<PASS, PREC>;
   size_t src = size_t(block) * Tr::kQuads * sizeof(Quad<typename Tr::R>);
   size_t fold = Tr::kComp ? size_t(block) * tpt * Tr::kNval * 2 * sizeof(float) : 0;
   size_t stage = Tr::kTma ? size_t(block) * Tr::kRecBytes + 16 : 0;
-  return src + box_bytes<PASS, PREC>(block) + fold + stage;
+  size_t tables = 8 * (core_table_doubles<PASS, KERNEL, PREC>() + exp2_table_doubles<PASS, KERNEL, PREC>());
+  return src + box_bytes<PASS, PREC>(block) + fold + stage + tables;
 }
 
 // Minimum resident CTAs requested from the compiler: caps the FP32 U/J kernels
@@ -160,6 +178,19 @@ __device__ __forceinline__ void finish_f32_sums(double* v) {
     if constexpr (KERNEL == VPM_KERNEL_GAUSSIANERF) {
 #pragma unroll
       for (int w = 3; w < 11; ++w) v[w] *= kGaussAScale;
+    }
+    v[11] = -(v[3] + v[7]);
+    if constexpr (PASS == PASS_UJD) v[23] = -(v[15] + v[19]);
+  }
+}
+
+// FP64 U/J passes: likewise, Gaussian-erf A sums hold p/(-3).
+template <int PASS, int KERNEL>
+__device__ __forceinline__ void finish_f64_sums(double* v) {
+  if constexpr (PASS == PASS_UJ || PASS == PASS_UJD) {
+    if constexpr (KERNEL == VPM_KERNEL_GAUSSIANERF) {
+#pragma unroll
+      for (int w = 3; w < 11; ++w) v[w] *= -3.0;
     }
     v[11] = -(v[3] + v[7]);
     if constexpr (PASS == PASS_UJD) v[23] = -(v[15] + v[19]);
@@ -321,6 +352,13 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
   float4* stage = reinterpret_cast<float4*>(smem_raw + kQuadBytes + kBoxBytes +
                                             (COMP ? size_t(BLOCK) * T * NV * 2 * sizeof(float) : 0));
   uint64_t* bar = reinterpret_cast<uint64_t*>(stage + size_t(BLOCK) * 3);
+  // FP64 Gaussian-erf tables, once per CTA (the first tile's barrier publishes them).
+  double* core_tab = reinterpret_cast<double*>(smem_raw + kQuadBytes);
+  double* exp2_tab = core_tab + core_table_doubles<PASS, KERNEL, PREC>();
+  if constexpr (core_table_doubles<PASS, KERNEL, PREC>() > 0)
+    stage_table(core_tab, d_core_table.v, kCoreRows * kCoreCoef);
+  if constexpr (exp2_table_doubles<PASS, KERNEL, PREC>() > 0)
+    stage_table(exp2_tab, d_exp2_table.v, kExp2Rows);
   __shared__ int s_item;
   __shared__ int s_last;
 
@@ -538,11 +576,12 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
           const double sig = a.ss[jj] * a.sigma_scale;
           qa.x = R(px - cx); qa.y = R(py - cy); qa.z = R(pz - cz);
           qb.x = R(a.gs[jj]); qb.y = R(a.gs[a.lds + jj]); qb.z = R(a.gs[2 * a.lds + jj]);
-          if (Tr::kUJ) {
-            source_consts<KERNEL, R>(sig, qa.w, qb.w);
+          if constexpr (Tr::kUJ) {
+            if constexpr (F32) source_consts<KERNEL, R>(sig, qa.w, qb.w);
+            else uj_consts_f64<KERNEL, PASS == PASS_UJD>(sig, qa.w, qb.w, qc.x, qc.y, qc.z, qc.w);
           } else {
             if constexpr (F32) zeta_consts_f32<KERNEL>(sig, qa.w, qb.w, qc.w);
-            else zeta_consts<KERNEL, R>(sig, qa.w, qb.w);
+            else zeta_consts_f64<KERNEL>(sig, qa.w, qb.w, qc.w);
             if (a.vs) {
               qc.x = R(a.vs[jj]); qc.y = R(a.vs[a.lds + jj]); qc.z = R(a.vs[2 * a.lds + jj]);
             }
@@ -554,13 +593,24 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
           // Padding source: zero strength, unit core.
           qa.x = qa.y = qa.z = R(0);
           qb.x = qb.y = qb.z = R(0);
-          if (Tr::kUJ) source_consts<KERNEL, R>(1.0, qa.w, qb.w);
-          else if constexpr (F32) zeta_consts_f32<KERNEL>(1.0, qa.w, qb.w, qc.w);
-          else zeta_consts<KERNEL, R>(1.0, qa.w, qb.w);
+          if constexpr (Tr::kUJ) {
+            if constexpr (F32) source_consts<KERNEL, R>(1.0, qa.w, qb.w);
+            else uj_consts_f64<KERNEL, PASS == PASS_UJD>(1.0, qa.w, qb.w, qc.x, qc.y, qc.z, qc.w);
+          } else if constexpr (F32) {
+            zeta_consts_f32<KERNEL>(1.0, qa.w, qb.w, qc.w);
+          } else {
+            zeta_consts_f64<KERNEL>(1.0, qa.w, qb.w, qc.w);
+          }
+        }
+        if constexpr (!F32 && !Tr::kUJ && KERNEL == VPM_KERNEL_GAUSSIANERF) {
+          // ζ = b 2^{r² a}: b goes into the strengths.
+          qb.x *= qb.w; qb.y *= qb.w; qb.z *= qb.w;
+          qc.x *= qb.w; qc.y *= qb.w; qc.z *= qb.w;
+          qd.x *= qb.w; qd.y *= qb.w; qd.z *= qb.w;
         }
         tileA[tid] = qa;
         tileB[tid] = qb;
-        if (!Tr::kUJ) tileC[tid] = qc;
+        if (Tr::kQuads > 2) tileC[tid] = qc;
         if (PASS == PASS_ZETAD) tileD[tid] = qd;
         if constexpr (F32) warp_source_box(qa.x, qa.y, qa.z, qa.w, jj < s1, sbox + 2 * warp);
         __syncthreads();
@@ -649,34 +699,49 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
           }
         }
       } else if constexpr (Tr::kUJ) {
-        // FP64 U/J (and DJ).
+        // FP64 U/J (and DJ).  Warps without a target only stage.
+        if (t0 + (tid & ~31) < t1) {
 #pragma unroll 2
-        for (int js = 0; js < cnt; ++js) {
-          const Quad<R> sa = tileA[js];
-          const Quad<R> sb = tileB[js];
+          for (int js = 0; js < cnt; ++js) {
+            const Quad<R> sa = tileA[js];
+            const Quad<R> sb = tileB[js];
+            const Quad<R> sc = tileC[js];
 #pragma unroll
-          for (int k = 0; k < T; ++k) {
-            const R dx = tx[k] - sa.x, dy = ty[k] - sa.y, dz = tz[k] - sa.z;
-            const R r2 = dx * dx + dy * dy + dz * dz;
-            R q, p;
-            pair_qp<KERNEL>(r2, sa.w, sb.w, q, p);
-            const R c0 = dy * sb.z - dz * sb.y;
-            const R c1 = dz * sb.x - dx * sb.z;
-            const R c2 = dx * sb.y - dy * sb.x;
-            acc[k][0] += q * c0; acc[k][1] += q * c1; acc[k][2] += q * c2;
-            const R p0 = p * c0, p1 = p * c1, p2 = p * c2;
-            acc[k][3] += p0 * dx; acc[k][4] += p0 * dy; acc[k][5] += p0 * dz;
-            acc[k][6] += p1 * dx; acc[k][7] += p1 * dy; acc[k][8] += p1 * dz;
-            acc[k][9] += p2 * dx; acc[k][10] += p2 * dy; acc[k][11] += p2 * dz;
-            acc[k][12] += q * sb.x; acc[k][13] += q * sb.y; acc[k][14] += q * sb.z;
-            if constexpr (PASS == PASS_UJD) {
-              R dq, dp;
-              pair_dqp_f64<KERNEL>(r2, sa.w, sb.w, dq, dp);
-              const R e0 = dp * c0, e1 = dp * c1, e2 = dp * c2;
-              acc[k][15] += e0 * dx; acc[k][16] += e0 * dy; acc[k][17] += e0 * dz;
-              acc[k][18] += e1 * dx; acc[k][19] += e1 * dy; acc[k][20] += e1 * dz;
-              acc[k][21] += e2 * dx; acc[k][22] += e2 * dy; acc[k][23] += e2 * dz;
-              acc[k][24] += dq * sb.x; acc[k][25] += dq * sb.y; acc[k][26] += dq * sb.z;
+            for (int k = 0; k < T; ++k) {
+              const R dx = tx[k] - sa.x, dy = ty[k] - sa.y, dz = tz[k] - sa.z;
+              R q, p, dq = 0, dp = 0;
+              if constexpr (KERNEL == VPM_KERNEL_GAUSSIANERF) {
+                const R r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+                uj_f64_gauss(r2, sa.w, sb.w, sc.x, core_tab, q, p);
+                if constexpr (PASS == PASS_UJD) {
+                  const R e = is_zero_f64(r2) ? 0.0 : exp2_f64(r2, sc.y, exp2_tab);
+                  dq = -sc.z * e;
+                  dp = sc.w * e;
+                }
+              } else {
+                const bool self = coincident_f64(dx, dy, dz);
+                const R rs = rsqrt(fma(dx, dx, fma(dy, dy, fma(dz, dz, sa.w))));
+                const R rs2 = rs * rs;
+                const R rs3 = rs2 * rs;
+                const R rs5 = rs3 * rs2;
+                const R rs7 = rs5 * rs2;
+                q = self ? 0.0 : fma(sb.w, rs5, rs3);
+                p = fma(sc.x, rs7, rs5);
+                if constexpr (PASS == PASS_UJD) {
+                  dq = self ? 0.0 : sc.y * rs7;
+                  dp = self ? 0.0 : sc.z * (rs7 * rs2);
+                }
+              }
+              accum_pair_f64(dx, dy, dz, q, p, sb.x, sb.y, sb.z, acc[k]);
+              if constexpr (PASS == PASS_UJD) {
+                const R gx = sb.x, gy = sb.y, gz = sb.z;
+                const R c0 = dy * gz - dz * gy, c1 = dz * gx - dx * gz, c2 = dx * gy - dy * gx;
+                const R e0 = dp * c0, e1 = dp * c1, e2 = dp * c2;
+                acc[k][15] += e0 * dx; acc[k][16] += e0 * dy; acc[k][17] += e0 * dz;
+                acc[k][18] += e1 * dx; acc[k][19] += e1 * dy; acc[k][20] += e1 * dz;
+                acc[k][21] += e2 * dx; acc[k][22] += e2 * dy;
+                acc[k][24] += dq * gx; acc[k][25] += dq * gy; acc[k][26] += dq * gz;
+              }
             }
           }
         }
@@ -721,30 +786,35 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
           }
         }
       } else {
-        // ζ passes, FP64.
+        // ζ passes, FP64 (Gaussian-erf: the strengths carry ζ(0)/σ³).
+        if (t0 + (tid & ~31) < t1) {
 #pragma unroll 2
-        for (int js = 0; js < cnt; ++js) {
-          const Quad<R> sa = tileA[js];
-          const Quad<R> sb = tileB[js];
-          const Quad<R> sc = tileC[js];
+          for (int js = 0; js < cnt; ++js) {
+            const Quad<R> sa = tileA[js];
+            const Quad<R> sb = tileB[js];
+            const Quad<R> sc = tileC[js];
 #pragma unroll
-          for (int k = 0; k < T; ++k) {
-            const R dx = tx[k] - sa.x, dy = ty[k] - sa.y, dz = tz[k] - sa.z;
-            const R r2 = dx * dx + dy * dy + dz * dz;
-            if constexpr (PASS == PASS_ZETA) {
-              const R z = pair_zeta<KERNEL>(r2, sa.w, sb.w);
+            for (int k = 0; k < T; ++k) {
+              const R dx = tx[k] - sa.x, dy = ty[k] - sa.y, dz = tz[k] - sa.z;
+              const R r2 = fma(dx, dx, fma(dy, dy, dz * dz));
+              R z, dzz = 0;
+              if constexpr (KERNEL == VPM_KERNEL_GAUSSIANERF) {
+                z = is_zero_f64(r2) ? 0.0 : exp2_f64(r2, sa.w, exp2_tab);
+                if constexpr (PASS == PASS_ZETAD) dzz = z * fma(r2, sc.w, -3.0);
+              } else if constexpr (PASS == PASS_ZETA) {
+                z = pair_zeta<KERNEL>(r2, sa.w, sb.w);
+              } else {
+                pair_zeta_d<KERNEL>(r2, sa.w, sb.w, z, dzz);
+              }
               acc[k][0] += z * sb.x; acc[k][1] += z * sb.y; acc[k][2] += z * sb.z;
               acc[k][3] += z * sc.x; acc[k][4] += z * sc.y; acc[k][5] += z * sc.z;
-            } else {
-              const Quad<R> sd = tileD[js];
-              R z, dzz;
-              pair_zeta_d<KERNEL>(r2, sa.w, sb.w, z, dzz);
-              acc[k][0] += z * sb.x; acc[k][1] += z * sb.y; acc[k][2] += z * sb.z;
-              acc[k][3] += z * sc.x; acc[k][4] += z * sc.y; acc[k][5] += z * sc.z;
-              acc[k][6] += dzz * sb.x; acc[k][7] += dzz * sb.y; acc[k][8] += dzz * sb.z;
-              acc[k][9] += dzz * sc.x + z * sd.x;
-              acc[k][10] += dzz * sc.y + z * sd.y;
-              acc[k][11] += dzz * sc.z + z * sd.z;
+              if constexpr (PASS == PASS_ZETAD) {
+                const Quad<R> sd = tileD[js];
+                acc[k][6] += dzz * sb.x; acc[k][7] += dzz * sb.y; acc[k][8] += dzz * sb.z;
+                acc[k][9] += dzz * sc.x + z * sd.x;
+                acc[k][10] += dzz * sc.y + z * sd.y;
+                acc[k][11] += dzz * sc.z + z * sd.z;
+              }
             }
           }
         }
@@ -808,6 +878,7 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
         }
       }
       if constexpr (F32) finish_f32_sums<PASS, KERNEL>(v);
+      else finish_f64_sums<PASS, KERNEL>(v);
       if (slot >= 0) {
         const uint64_t pol = l2_policy(a.tile_done != nullptr);
 #pragma unroll
@@ -925,7 +996,7 @@ PairFn fn_ready() {
   static bool once = [] {
     cudaFuncSetAttribute(pair_kernel<PASS, KERNEL, PREC, BLOCK, T, CLU>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(smem_bytes<PASS, PREC>(BLOCK, T)));
+                         int(smem_bytes<PASS, KERNEL, PREC>(BLOCK, T)));
     // Clusters of up to 16 CTAs (beyond the portable 8) for the split-source form.
     if (CLU)
       cudaFuncSetAttribute(pair_kernel<PASS, KERNEL, PREC, BLOCK, T, CLU>,
@@ -984,11 +1055,14 @@ PairFn pick_cluster(int kernel, int prec, Shape s) {
 }
 
 template <int PASS>
-size_t smem_of(int precision, Shape s) {
+size_t smem_of(int kernel, int precision, Shape s) {
+  constexpr int W = VPM_KERNEL_WINCKELMANS, G = VPM_KERNEL_GAUSSIANERF;
   switch (precision) {
-    case VPM_PREC_FP64: return smem_bytes<PASS, VPM_PREC_FP64>(s.block, s.tpt);
-    case VPM_PREC_FP32: return smem_bytes<PASS, VPM_PREC_FP32>(s.block, s.tpt);
-    default: return smem_bytes<PASS, VPM_PREC_FP32C>(s.block, s.tpt);
+    case VPM_PREC_FP64:
+      return kernel == W ? smem_bytes<PASS, W, VPM_PREC_FP64>(s.block, s.tpt)
+                         : smem_bytes<PASS, G, VPM_PREC_FP64>(s.block, s.tpt);
+    case VPM_PREC_FP32: return smem_bytes<PASS, G, VPM_PREC_FP32>(s.block, s.tpt);
+    default: return smem_bytes<PASS, G, VPM_PREC_FP32C>(s.block, s.tpt);
   }
 }
 
@@ -997,7 +1071,7 @@ int ctas_per_sm(int kernel, int precision, Shape s) {
   PairFn f = pick_kernel<PASS>(kernel, precision, s);
   if (!f) return 0;
   int n = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, s.block, smem_of<PASS>(precision, s)) !=
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, f, s.block, smem_of<PASS>(kernel, precision, s)) !=
       cudaSuccess)
     return 0;
   return n;
@@ -1034,11 +1108,11 @@ cudaError_t launch(int kernel, int precision, Shape s, const PairArgs& a, int gr
         int64_t(grid) != int64_t(a.n_tb) * a.n_chunk || a.n_chunk != a.cluster)
       return cudaErrorInvalidConfiguration;
     cudaLaunchAttribute attr;
-    cudaLaunchConfig_t cfg = cluster_config(grid, s.block, smem_of<PASS>(precision, s), st,
+    cudaLaunchConfig_t cfg = cluster_config(grid, s.block, smem_of<PASS>(kernel, precision, s), st,
                                             a.cluster, &attr);
     return cudaLaunchKernelEx(&cfg, f, a);
   }
-  f<<<grid, s.block, smem_of<PASS>(precision, s), st>>>(a);
+  f<<<grid, s.block, smem_of<PASS>(kernel, precision, s), st>>>(a);
   return cudaGetLastError();
 }
 
@@ -1049,7 +1123,7 @@ int max_active_clusters(int kernel, int precision, Shape s, int cluster) {
   PairFn f = pick_cluster<PASS>(kernel, precision, s);
   if (!f) return 0;
   cudaLaunchAttribute attr;
-  cudaLaunchConfig_t cfg = cluster_config(cluster, s.block, smem_of<PASS>(precision, s), nullptr,
+  cudaLaunchConfig_t cfg = cluster_config(cluster, s.block, smem_of<PASS>(kernel, precision, s), nullptr,
                                           cluster, &attr);
   int n = 0;
   if (cudaOccupancyMaxActiveClusters(&n, f, &cfg) != cudaSuccess) {
