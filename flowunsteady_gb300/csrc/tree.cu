@@ -13,9 +13,9 @@
 //      (order P) from their particles, then, deepest generation first, parents
 //      from their children (box union; moments shifted to the parent centre);
 //   4. targets are taken in groups of 64 consecutive particles of the Morton
-//      order (compact boxes, one full CTA each).  The walk for a group is
-//      split over the subtrees of a frontier of at most 73 cells (the leaves
-//      of generations 0-1 and generation 2), one thread per (group, subtree):
+//      order (compact boxes).  The walk for a group is split over the subtrees of a
+//      frontier of at most 73 cells (the leaves of generations 0-1 and generation
+//      2), one thread per (subtree, group):
 //      a cell s is far for group t when (R_t + R_s) < θ·d and
 //      d - R_t - R_s >= sigma_factor·σmax_s (d = distance of the centres, FP32
 //      boxes), then it is evaluated from its moments; otherwise its leaves are
@@ -24,13 +24,13 @@
 //      as large as the group are marked for them;
 //   5. local expansions (FP32, P = 4): the marked cells' moments turned into
 //      one local expansion of ψ per group (M2L, tree.cuh);
-//   6. the direct near field: one CTA per group over its near ranges, with the
+//   6. the direct near field: runs of tiles of a group's near ranges, with the
 //      regularised kernels of the direct sum (FP32 pair routines on positions
 //      relative to the group's first particle, or FP64);
 //   7. the far field: one thread per target over the unmarked far cells of its
-//      group (M2P, tree.cuh), added to the near field; results go to the
-//      original order; then the local expansion at every target (L2P) is
-//      added to them.
+//      group (M2P, tree.cuh); 5 and 7 run beside 6 on a second stream;
+//   8. near field, far field and the local expansion at every target (L2P)
+//      added, in the original order.
 // The far field uses the singular kernel, as FLOWVPM's nonzero_sigma=false;
 // sigma_factor keeps regularised pairs out of it (Gaussian-erf: beyond 7.1 σ
 // the kernels agree to FP32 rounding).
@@ -55,7 +55,6 @@ constexpr int kMaxGen = 23;        // root + at most 21 Morton digits (+1 spare)
 // cell of every generation (generation g starts at counters[kGenBase + g]).
 constexpr int kCntCells = 0, kCntLeaves = 1, kCntFlags = 2, kCntDone = 3, kGenBase = 4;
 constexpr int kNumCounters = kGenBase + kMaxGen + 2;
-constexpr int kStack = 256;        // traversal stack (cells)
 // Target group size (consecutive particles of the Morton order).  32-particle
 // groups were measured at N = 1M too: at θ = 0.4 they take 0.131 s instead of
 // 0.142 s but lose accuracy (rel-L2 U 5.3e-5, J 1.46e-5 against 4.4e-5, 1.15e-5),
@@ -64,21 +63,29 @@ constexpr int kTreeBlock = 64;     // threads of the far CTAs = group size
 constexpr int kMaxFront = 1 + 8 + 64;   // walk roots: leaves of generations 0-1, generation 2
 
 // ------------------------------------------------------------- workspace --
+// Interaction lists of a target group: far cells (M2P), near source ranges, cells of
+// its local expansion.
+enum ListKind { LIST_FAR = 0, LIST_NEAR = 1, LIST_LOC = 2, kListKinds = 3 };
+
 struct FmmWork {
   int64_t cap = 0;            // particles
   int64_t cell_cap = 0;       // cells (2·cap + 8 bounds any octree of cap points)
   int64_t mom_cells = 0;      // cells the moment buffers hold
   int mom_p = -1;
-  int64_t list_cap = 0;       // interaction list entries
+  int64_t far_cap = 0, near_cap = 0, loc_cap_list = 0;   // interaction list entries
   // particles in Morton order
   uint64_t *codes = nullptr, *codes_alt = nullptr;
   int *idx = nullptr, *perm = nullptr;
   double* sorted = nullptr;   // X 3, Γ 3, σ 1 rows of length cap
   float4* rec = nullptr;      // packed FP32 source records of the sorted particles
-  double* near_raw = nullptr; // up to 27 raw near-field sums per sorted particle
+  // raw near-field sums, kTreeBlock targets per row, NV rows per near item
+  double* near_raw = nullptr;
+  size_t near_raw_cap = 0;    // doubles
+  double* pot = nullptr;      // far-field U 3, J 9 per sorted particle (FP32 or FP64 rows)
   float* vw = nullptr;        // v_q, w_q rows of the ζ passes in Morton order, FP32
   // cells
   int *lo = nullptr, *hi = nullptr, *child = nullptr, *nchild = nullptr;
+  int* skip = nullptr;        // the cell after this one's subtree in Morton order (-1: none)
   double* geom = nullptr;     // per cell: box min x y z, box max x y z, σmax, unused
   double* mom = nullptr;      // per cell: 3·ncoef(P) FP64 moments
   float* momf = nullptr;      // FP32 copy
@@ -91,19 +98,24 @@ struct FmmWork {
   unsigned long long* pairs = nullptr;   // [0] near source pairs, [1] far (target, cell) pairs
   double* box = nullptr;      // bounding cube: min x y z, size
   double* box_part = nullptr; // per-block min/max partials
-  // interaction lists
-  int *nfar = nullptr, *nnear = nullptr, *ofar = nullptr, *onear = nullptr;
+  // interaction lists, one per target group, group g's at gbase[q][g] .. + gtot[q][g]
+  int* wcnt = nullptr;        // per (frontier cell, group): kListKinds counts, then offsets in the group
+  int* gtot = nullptr;        // kListKinds + 1 rows: list lengths; near sources
+  int* gbase = nullptr;       // kListKinds + 1 rows: list starts; first near item
+  int* gorder = nullptr;      // groups by decreasing far list
+  long long* totals = nullptr;   // see group_scan_kernel
   int* far_list = nullptr;    // far cell ids per target group (M2P at every target)
-  int *nloc = nullptr, *oloc = nullptr;   // local-expansion list counts, offsets
-  int* loc_list = nullptr;    // far cell ids per target group taken by its local expansion
-  int64_t loc_list_cap = 0;
   int2* near_list = nullptr;  // near source ranges [x, y) per target group
+  int* loc_list = nullptr;    // far cell ids per target group taken by its local expansion
+  cudaStream_t aux = nullptr; // far field and local expansions, beside the near field
+  cudaEvent_t fork = nullptr, join = nullptr;
   void* cub_tmp = nullptr;
   size_t cub_bytes = 0;
   int h_counters[kNumCounters];
   // statistics of the last evaluation
   int64_t last_cells = 0, last_leaves = 0, last_groups = 0, last_far = 0, last_near = 0;
-  int64_t last_nfront = 0, last_n = -1;
+  int64_t last_n = -1;
+  int64_t last_items = 0;    // near items
   unsigned long long h_pairs[3] = {0, 0, 0};
   float* loc = nullptr;       // per target group: 3·ncoef(Q) local coefficients
   int64_t loc_cap = 0;
@@ -111,11 +123,14 @@ struct FmmWork {
 
 void fmm_free(FmmWork* w) {
   if (!w) return;
-  void* ptrs[] = {w->codes, w->codes_alt, w->idx, w->perm, w->sorted, w->rec, w->near_raw,
-                  w->vw, w->lo, w->hi, w->child, w->nchild, w->geom, w->mom, w->momf, w->leaves,
-                  w->ggeom, w->cgeom, w->front, w->pairs, w->counters, w->box, w->box_part,
-                  w->nfar, w->nnear, w->ofar, w->onear, w->far_list, w->near_list, w->cub_tmp,
-                  w->loc, w->nloc, w->oloc, w->loc_list};
+  void* ptrs[] = {w->codes, w->codes_alt, w->idx, w->perm, w->sorted, w->rec, w->near_raw, w->pot,
+                  w->vw, w->lo, w->hi, w->child, w->nchild, w->skip, w->geom, w->mom, w->momf,
+                  w->leaves, w->ggeom, w->cgeom, w->front, w->pairs, w->counters, w->box,
+                  w->box_part, w->wcnt, w->gtot, w->gbase, w->gorder, w->totals, w->far_list,
+                  w->near_list, w->cub_tmp, w->loc, w->loc_list};
+  if (w->aux) cudaStreamDestroy(w->aux);
+  if (w->fork) cudaEventDestroy(w->fork);
+  if (w->join) cudaEventDestroy(w->join);
   for (void* p : ptrs) cudaFree(p);
   delete w;
 }
@@ -224,9 +239,10 @@ __global__ void gather_kernel(int64_t n, const int* __restrict__ perm, const dou
 }
 
 // ------------------------------------------------------------- tree build --
-__global__ void tree_init_kernel(int64_t n, int* lo, int* hi, int* counters) {
+__global__ void tree_init_kernel(int64_t n, int* lo, int* hi, int* skip, int* counters) {
   lo[0] = 0;
   hi[0] = int(n);
+  skip[0] = -1;
   counters[kCntCells] = 1;
   counters[kCntLeaves] = 0;
   counters[kCntFlags] = 0;
@@ -252,7 +268,7 @@ __device__ __forceinline__ int lower_bound_code(const uint64_t* codes, int lo, i
 // block to finish closes generation g + 1, which ends where the cells appended
 // here end (a launch of its own before).
 __global__ void tree_split_kernel(int g, int ncrit, int64_t cell_cap, const uint64_t* __restrict__ codes,
-                                  int* lo, int* hi, int* child, int* nchild, int* leaves,
+                                  int* lo, int* hi, int* child, int* nchild, int* skip, int* leaves,
                                   int* counters) {
   const int begin = counters[kGenBase + g], end = counters[kGenBase + g + 1];
   const int lane = threadIdx.x & 31, v = lane & 7, base = lane & ~7;
@@ -292,6 +308,7 @@ __global__ void tree_split_kernel(int g, int ncrit, int64_t cell_cap, const uint
       const int k = first_child + __popc(mask & ((1u << v) - 1u));
       lo[k] = bound;
       hi[k] = next;
+      skip[k] = k + 1 < first_child + nc ? k + 1 : skip[cell];
     }
     if (valid && v == 0) {
       child[cell] = fits ? first_child : -1;
@@ -400,16 +417,18 @@ struct CellOut {
   double* mom;
   float* momf;
   float4* walk;
+  const int* skip;
 };
 
 // Walk record of a cell, two float4 read together by the traversal:
 //   rec[2c]     = centre x, y, z and radius (FP32, inflated by 1e-6 of the
 //                 coordinates' magnitude so that rounding cannot shrink it);
 //   rec[2c + 1] = largest core (FP32), then as integer bits: the first child
-//                 (or the first particle of a leaf), the end of the cell's
-//                 particle range, the number of children (0 for a leaf).
+//                 (or the first particle of a leaf), the end of a leaf's
+//                 particle range (-1: not a leaf), and the cell after this one's
+//                 subtree in Morton order (-1: none).
 __device__ __forceinline__ void write_cell_geom(const CellOut& o, int cell, const double (&g)[8],
-                                                int first, int end, int nc) {
+                                                int first, int end) {
   double* gc = o.geom + int64_t(cell) * kGeom;
 #pragma unroll
   for (int d = 0; d < 8; ++d) gc[d] = g[d];
@@ -418,7 +437,7 @@ __device__ __forceinline__ void write_cell_geom(const CellOut& o, int cell, cons
   const double pad = 1e-6 * (fabs(cx) + fabs(cy) + fabs(cz) + r);
   o.walk[2 * int64_t(cell)] = make_float4(float(cx), float(cy), float(cz), float(r + pad));
   o.walk[2 * int64_t(cell) + 1] = make_float4(float(g[6]), __int_as_float(first),
-                                              __int_as_float(end), __int_as_float(nc));
+                                              __int_as_float(end), __int_as_float(o.skip[cell]));
 }
 
 // The upward pass is FP64 sums of a few thousand terms per cell, on a pipe that
@@ -445,7 +464,7 @@ __global__ void __launch_bounds__(32 * kLeafWarps) tree_leaf_kernel(
   const int cell = leaves[l], a = lo[cell], b = hi[cell];
   double g[8];
   warp_box(sorted, ldw, a, b, g);
-  if (lane == 0) write_cell_geom(out, cell, g, a, b, 0);
+  if (lane == 0) write_cell_geom(out, cell, g, a, b);
   double cx, cy, cz, rad;
   cell_centre(g, cx, cy, cz, rad);
   double acc[ROUNDS];
@@ -491,8 +510,8 @@ __global__ void __launch_bounds__(32 * kLeafWarps) tree_leaf_kernel(
 constexpr int kUpSlots = 4, kUpThreads = 128;
 template <int P>
 __global__ void __launch_bounds__(kUpThreads * kUpSlots) tree_upward_kernel(
-    int g, int* counters, const int* __restrict__ hi, const int* __restrict__ child,
-    const int* __restrict__ nchild, CellOut out) {
+    int g, int* counters, const int* __restrict__ child, const int* __restrict__ nchild,
+    CellOut out) {
   constexpr int NC = ncoef(P), NE = 3 * NC;
   __shared__ double s_m[8][NE], s_t[8][NC], s_box[8][8], s_geom[8];
   __shared__ double s_sum[kUpSlots - 1][NE];
@@ -544,7 +563,7 @@ __global__ void __launch_bounds__(kUpThreads * kUpSlots) tree_upward_kernel(
       double gg[8];
 #pragma unroll
       for (int d = 0; d < 8; ++d) gg[d] = s_geom[d];
-      write_cell_geom(out, cell, gg, ch, hi[cell], nc);
+      write_cell_geom(out, cell, gg, ch, -1);
     }
     __syncthreads();
     for (int e0 = 0; e0 < NE; e0 += kUpThreads) {
@@ -596,75 +615,215 @@ __global__ void group_geom_kernel(int64_t n, const double* __restrict__ sorted, 
   if ((threadIdx.x & 31) == 0) ggeom[g] = make_float4(float(cx), float(cy), float(cz), float(r + pad));
 }
 
-// One thread per (target group g, frontier cell j), t = g·nfront + j: the
-// walk of the subtree below frontier cell j for group g.  FILL = false counts
-// the far cells and near source ranges, FILL = true writes them at the
-// scanned offsets (same order); a group's lists are the concatenation over j.
-// Near leaves that continue the previous near range in Morton order extend it.
+// One thread per (frontier cell j, target group g), t = j·ngroups + g: the walk of
+// the subtree below frontier cell j for group g, in Morton order.  A warp holds 32
+// neighbouring groups on one subtree, so its lanes visit nearly the same cells, and
+// each cell's record leads to both the cell inside it and the one after it (no
+// stack).  FILL = false counts the far cells, near source ranges, local-expansion
+// cells and near sources; FILL = true writes them at the scanned offsets (same
+// order); a group's lists are the concatenation over j.  Near leaves that continue
+// the previous near range in Morton order extend it.
+// With one lane per subtree of one group and a stack of cells in local memory the
+// two passes took 205 + 209 µs at N = 60,000; this form takes 133 + 144 µs.
 template <bool FILL>
-__global__ void traverse_kernel(int64_t nthreads, int nfront, const int* __restrict__ front,
+__global__ void traverse_kernel(int ngroups, int nfront, const int* __restrict__ front,
                                 const float4* __restrict__ ggeom, const float4* __restrict__ walk,
-                                float theta, float sfac, int mark_local, int* nfar,
-                                int* nnear, int* nloc, const int* __restrict__ ofar,
-                                const int* __restrict__ onear, const int* __restrict__ oloc,
-                                int* far_list, int2* near_list, int* loc_list, int* counters,
-                                int ncells) {
+                                float theta, float sfac, int mark_local, int* wcnt, int* nsrc,
+                                const int* __restrict__ gbase, int* far_list, int2* near_list,
+                                int* loc_list, int* counters, int ncells) {
+  const int64_t nwalk = int64_t(ngroups) * nfront;
   const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (t >= nthreads) return;
-  const int64_t g = t / nfront;
+  if (t >= nwalk) return;
+  const int g = int(t % ngroups);
   const float4 tg = ggeom[g];
-  int stack[kStack];
-  int sp = 0;
-  stack[sp++] = front[t % nfront];
-  int cf = 0, cn = 0, cl = 0, last_hi = -1;
-  const int of = FILL ? ofar[t] : 0, on = FILL ? onear[t] : 0, ol = FILL && mark_local ? oloc[t] : 0;
-  while (sp > 0) {
-    const int s = stack[--sp];
-    if (s < 0 || s >= ncells) {
+  int cf = 0, cn = 0, cl = 0, cs = 0, last_hi = -1;
+  int of = 0, on = 0, ol = 0;
+  if (FILL) {
+    of = gbase[g] + wcnt[t];
+    on = gbase[ngroups + g] + wcnt[nwalk + t];
+    if (mark_local) ol = gbase[2 * ngroups + g] + wcnt[2 * nwalk + t];
+  }
+  int s = front[t / ngroups];
+  int stop = -1;
+  for (int visits = 0; s != stop || visits == 0; ++visits) {
+    if (s < 0 || s >= ncells || visits >= ncells) {   // cannot happen: the walk left the tree
       atomicOr(&counters[kCntFlags], 16);
       break;
     }
-    const float4 cs = walk[2 * s], ck = walk[2 * s + 1];
-    const int first = __float_as_int(ck.y), end = __float_as_int(ck.z), nc = __float_as_int(ck.w);
-    const float dx = tg.x - cs.x, dy = tg.y - cs.y, dz = tg.z - cs.z;
+    const float4 cs4 = walk[2 * s], ck = walk[2 * s + 1];
+    const int first = __float_as_int(ck.y), end = __float_as_int(ck.z), next = __float_as_int(ck.w);
+    if (visits == 0) stop = next;
+    const float dx = tg.x - cs4.x, dy = tg.y - cs4.y, dz = tg.z - cs4.z;
     const float d = sqrtf(dx * dx + dy * dy + dz * dz);
-    if (tg.w + cs.w < theta * d && d - tg.w - cs.w >= sfac * ck.x) {
+    if (tg.w + cs4.w < theta * d && d - tg.w - cs4.w >= sfac * ck.x) {
       // Cells at least as large as the group go to its local expansion.
-      if (mark_local && cs.w >= tg.w) {
+      if (mark_local && cs4.w >= tg.w) {
         if (FILL) loc_list[ol + cl] = s;
         ++cl;
       } else {
         if (FILL) far_list[of + cf] = s;
         ++cf;
       }
-    } else if (nc == 0) {
+    } else if (end >= 0) {   // a leaf
       if (cn > 0 && first == last_hi) {
         if (FILL) near_list[on + cn - 1].y = end;
       } else {
         if (FILL) near_list[on + cn] = make_int2(first, end);
         ++cn;
       }
+      cs += end - first;
       last_hi = end;
     } else {
-      const int c0 = first;
-      if (sp + nc > kStack) {   // cannot happen for 21 Morton levels (7·21 + 1 entries)
-        atomicOr(&counters[kCntFlags], 2);
-        break;
-      }
-      for (int k = nc - 1; k >= 0; --k) stack[sp++] = c0 + k;
+      s = first;
+      continue;
     }
+    s = next;
   }
   if (!FILL) {
-    nfar[t] = cf;
-    nnear[t] = cn;
-    if (mark_local) nloc[t] = cl;
+    wcnt[t] = cf;
+    wcnt[nwalk + t] = cn;
+    wcnt[2 * nwalk + t] = cl;
+    nsrc[t] = cs;
   }
 }
 
+// Lengths of group g's lists and its near sources (gtot rows), and in wcnt the
+// offset of every subtree's part in the group's list: one warp per group, lane =
+// frontier cell.
+__global__ void group_lists_kernel(int ngroups, int nfront, int* wcnt, const int* __restrict__ nsrc,
+                                   int* gtot) {
+  const int g = int((int64_t(blockIdx.x) * blockDim.x + threadIdx.x) / 32), lane = threadIdx.x & 31;
+  if (g >= ngroups) return;
+  const int64_t nwalk = int64_t(ngroups) * nfront;
+  for (int q = 0; q <= kListKinds; ++q) {
+    int carry = 0;
+    for (int j0 = 0; j0 < nfront; j0 += 32) {
+      const int j = j0 + lane;
+      const int64_t t = int64_t(j) * ngroups + g;
+      const int v = j >= nfront ? 0 : q < kListKinds ? wcnt[q * nwalk + t] : nsrc[t];
+      int incl = v;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+      }
+      if (j < nfront && q < kListKinds) wcnt[q * nwalk + t] = carry + incl - v;
+      carry += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) gtot[int64_t(q) * ngroups + g] = carry;
+  }
+}
+
+// Starts of the groups' lists and of their near items, and the groups by decreasing
+// far list (within 64 steps of the longest), by one block.
+//   totals[0..2]  list lengths;  totals[3]  near items;  totals[4]  tiles of an item;
+//   totals[5]     near sources over all groups.
+// Near items are runs of whole fold groups (kItemTiles tiles) of one group's near
+// tiles, of equal length: the shortest for which the field has about kNearItems of
+// them beside one per group.  gbase row 3 holds each group's first item.
+constexpr int kScanThreads = 1024;
+constexpr int kItemTiles = 16;               // tiles between two folds (near_tile_kernel)
+constexpr long long kNearItems = 16 * 3 * 152;   // about 16 waves of near CTAs
+
+__device__ __forceinline__ int near_tiles(int sources, int ranges) {
+  return sources / 128 + (ranges + 127) / 128;   // at most: every 128 ranges end a tile
+}
+
+__global__ void __launch_bounds__(kScanThreads) group_scan_kernel(int ngroups, const int* __restrict__ gtot,
+                                                                 int* gbase, int* gorder,
+                                                                 int whole_groups, long long* totals) {
+  __shared__ long long s_part[32], s_carry[4];
+  __shared__ int s_max, s_hist[64];
+  __shared__ long long s_tiles;
+  const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+  if (tid == 0) s_max = 0;
+  if (tid < 64) s_hist[tid] = 0;
+  if (tid < 4) s_carry[tid] = 0;
+  __syncthreads();
+  long long tiles = 0, srcs = 0;
+  int fmax_ = 0;
+  for (int g = tid; g < ngroups; g += kScanThreads) {
+    const int n = gtot[int64_t(kListKinds) * ngroups + g];
+    srcs += n;
+    tiles += near_tiles(n, gtot[int64_t(LIST_NEAR) * ngroups + g]);
+    fmax_ = max(fmax_, gtot[g]);
+  }
+  auto block_sum = [&](long long v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if (lane == 0) s_part[wid] = v;
+    __syncthreads();
+    long long r = 0;
+    for (int w = 0; w < kScanThreads / 32; ++w) r += s_part[w];
+    return r;
+  };
+  tiles = block_sum(tiles);
+  srcs = block_sum(srcs);
+  atomicMax(&s_max, fmax_);
+  if (tid == 0) {
+    const long long want = (tiles + kNearItems - 1) / kNearItems;
+    s_tiles = whole_groups ? (1ll << 40) : max(1ll, (want + kItemTiles - 1) / kItemTiles) * kItemTiles;
+    totals[4] = s_tiles;
+    totals[5] = srcs;
+  }
+  __syncthreads();
+  const long long per = s_tiles;
+  const int fmx = s_max;
+  for (int g0 = 0; g0 < ngroups; g0 += kScanThreads) {
+    const int g = g0 + tid;
+    const bool live = g < ngroups;
+    const int far = live ? gtot[g] : 0;
+    const int rng = live ? gtot[int64_t(LIST_NEAR) * ngroups + g] : 0;
+    const int loc = live ? gtot[int64_t(LIST_LOC) * ngroups + g] : 0;
+    const int src = live ? gtot[int64_t(kListKinds) * ngroups + g] : 0;
+    const long long nt = near_tiles(src, rng);
+    const long long vals[4] = {far, rng, loc, live ? max(1ll, (nt + per - 1) / per) : 0ll};
+    if (live) atomicAdd(&s_hist[63 - int(int64_t(far) * 63 / max(fmx, 1))], 1);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      long long incl = vals[q];
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const long long u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+      }
+      __syncthreads();
+      if (lane == 31) s_part[wid] = incl;
+      __syncthreads();
+      long long before = s_carry[q], all = 0;
+      for (int w = 0; w < kScanThreads / 32; ++w) {
+        if (w < wid) before += s_part[w];
+        all += s_part[w];
+      }
+      if (live) gbase[int64_t(q) * ngroups + g] = int(before + incl - vals[q]);
+      __syncthreads();
+      if (tid == 0) s_carry[q] += all;
+    }
+  }
+  __syncthreads();
+  if (tid < 4) totals[tid] = s_carry[tid];
+  if (tid == 0) {   // starts of the order's steps
+    int at = 0;
+    for (int b = 0; b < 64; ++b) {
+      const int n = s_hist[b];
+      s_hist[b] = at;
+      at += n;
+    }
+  }
+  __syncthreads();
+  for (int g = tid; g < ngroups; g += kScanThreads)
+    gorder[atomicAdd(&s_hist[63 - int(int64_t(gtot[g]) * 63 / max(fmx, 1))], 1)] = g;
+}
+
 // --------------------------------------------------------------- near field --
-// One CTA of kNearThreads threads per target group against every particle of
-// its near source ranges, with the pair routines of the direct sum
-// (vpm_device.cuh) on T targets per thread:
+// Groups' near fields differ a hundredfold (a group that straddles a jump of the
+// Morton curve has a box as large as the wake and nearly every particle near it), so
+// the work is dealt in items of equal length (group_scan_kernel) and not in groups:
+// with one CTA per group the longest one, 60,000 sources at N = 60,000 against
+// 11,000 on average, set the launch's 2.0 ms; items take 1.11 ms.  One CTA of kNearThreads threads per
+// item: its run of the tiles of the group's near source ranges, with the pair
+// routines of the direct sum (vpm_device.cuh) on T targets per thread:
 //   - the group's kTreeBlock targets are held as TQ = kTreeBlock/T target sets of T targets
 //     (target t = tq + TQ·k), each set by SL = kNearThreads/TQ threads, one per
 //     source slice;
@@ -680,7 +839,9 @@ __global__ void traverse_kernel(int64_t nthreads, int nfront, const int* __restr
 //   - FP32 sums are folded into (hi, lo) pairs (Knuth's TwoSum) every
 //     kNearFoldSources sources of a thread; the epilogue forms every target's raw
 //     sums in FP64 as the slices' (hi + lo) in slice order.
-// Raw sums go to raw[k·ldr + i] in Morton order:
+// Raw sums of target t of item i go to raw[(i·NV + k)·kTreeBlock + t]; the reader adds
+// a group's items in order.  An item starts at a fold, so that the FP32 sums are
+// those of one CTA that walks the whole group:
 //   PASS_UJ    U 3, A 9, W 3 (Gaussian-erf A sums hold p/(-3), as the direct
 //              pass's do);
 //   PASS_UJD   those plus DA 9, DW 3 (Gaussian-erf: Dq, Dp vanish beyond the
@@ -713,16 +874,17 @@ struct NearShape {
 
 template <int KERNEL, int PASS>
 __global__ void __launch_bounds__(kNearThreads, NearShape<PASS>::kMinBlocks) near_tile_kernel(
-    int nfront, const int* __restrict__ onear, const int* __restrict__ nnear,
-    const int2* __restrict__ near_list, const float4* __restrict__ rec,
-    const float* __restrict__ vw, int64_t ldv, double* raw, int64_t ldr, int64_t n,
-    int* counters, unsigned long long* pairs) {
+    int ngroups, const int* __restrict__ gbase, const int* __restrict__ gtot,
+    const long long* __restrict__ totals, const int2* __restrict__ near_list,
+    const float4* __restrict__ rec, const float* __restrict__ vw, int64_t ldv, double* raw,
+    int64_t n, int* counters, unsigned long long* pairs) {
   using Sh = NearShape<PASS>;
   constexpr int T = Sh::T, TQ = Sh::TQ, SL = Sh::SL, NV = Sh::NV;
   constexpr bool UJ = Sh::UJ;
   constexpr bool D = PASS == PASS_UJD || PASS == PASS_ZETAD;
   constexpr int PER = kNearThreads / SL;              // staged sources per thread and tile
   constexpr int FOLD_TILES = kNearFoldSources / PER;  // tiles between two folds
+  static_assert(kItemTiles % FOLD_TILES == 0, "items start at folds");
   static_assert(kNearThreads == 128 && kNearThreads % TQ == 0 && kTreeBlock <= kNearThreads,
                 "four-warp scan below; whole target sets");
   extern __shared__ __align__(16) unsigned char near_smem[];
@@ -736,10 +898,23 @@ __global__ void __launch_bounds__(kNearThreads, NearShape<PASS>::kMinBlocks) nea
 
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   const int tq = tid % TQ, sl = tid / TQ;
-  const int a = int(blockIdx.x) * kTreeBlock, b = int(min(int64_t(a) + kTreeBlock, n));
+  const int item = int(blockIdx.x);
+  if (item >= totals[3]) return;
+  int grp = 0;   // the last group whose first item is <= item
+  {
+    const int* first = gbase + int64_t(kListKinds) * ngroups;
+    int hi_g = ngroups - 1;
+    while (grp < hi_g) {
+      const int mid = (grp + hi_g + 1) >> 1;
+      if (first[mid] <= item) grp = mid;
+      else hi_g = mid - 1;
+    }
+  }
+  const long long w0 = (item - gbase[int64_t(kListKinds) * ngroups + grp]) * totals[4],
+                  w1 = w0 + totals[4];   // its tiles
+  const int a = grp * kTreeBlock, b = int(min(int64_t(a) + kTreeBlock, n));
   const float4 o0 = rec[3 * int64_t(a)], o1 = rec[3 * int64_t(a) + 1];
-  const int64_t t0s = int64_t(blockIdx.x) * nfront, t1s = t0s + nfront - 1;
-  const int l0 = onear[t0s], ln = onear[t1s] + nnear[t1s] - l0;
+  const int l0 = gbase[int64_t(LIST_NEAR) * ngroups + grp], ln = gtot[int64_t(LIST_NEAR) * ngroups + grp];
 
   float tx[T], ty[T], tz[T];
 #pragma unroll
@@ -777,10 +952,11 @@ __global__ void __launch_bounds__(kNearThreads, NearShape<PASS>::kMinBlocks) nea
   };
 
   int tiles = 0;
+  long long tile0 = 0;   // first tile of the chunk of ranges
   // The near ranges, kNearThreads at a time: their lengths' prefix sums in
   // shared memory; the concatenated sources are then staged in full tiles, each
   // slot finding its range by binary search.
-  for (int rc0 = 0; rc0 < ln; rc0 += kNearThreads) {
+  for (int rc0 = 0; rc0 < ln && tile0 < w1; rc0 += kNearThreads) {
     const int nr = min(kNearThreads, ln - rc0);
     int len = 0;
     __syncthreads();   // previous chunk's tiles consumed
@@ -806,8 +982,13 @@ __global__ void __launch_bounds__(kNearThreads, NearShape<PASS>::kMinBlocks) nea
     if (tid == 0) s_pref[0] = 0;
     __syncthreads();
     const int total = s_pref[nr];
-    if (tid == 0 && pairs) atomicAdd(&pairs[0], (unsigned long long)total * (unsigned long long)(b - a));
-    for (int q0 = 0; q0 < total; q0 += kNearThreads) {
+    const int chunk_tiles = (total + kNearThreads - 1) / kNearThreads;
+    const int q_begin = int(min((long long)chunk_tiles, max(0ll, w0 - tile0))) * kNearThreads;
+    const int q_end = int(min((long long)total, max(0ll, w1 - tile0) * kNearThreads));
+    tile0 += chunk_tiles;
+    if (tid == 0 && pairs && q_end > q_begin)
+      atomicAdd(&pairs[0], (unsigned long long)(q_end - q_begin) * (unsigned long long)(b - a));
+    for (int q0 = q_begin; q0 < q_end; q0 += kNearThreads) {
       const int q = q0 + tid;
       float4 qa = make_float4(kNearPadX, kNearPadX, kNearPadX, 0.f);
       float4 qb = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -894,24 +1075,55 @@ __global__ void __launch_bounds__(kNearThreads, NearShape<PASS>::kMinBlocks) nea
           if (w == 19) d11 = v;
           if (w == 23) v = -(d00 + d11);
         }
-        raw[w * ldr + i] = v;
+        raw[(int64_t(item) * NV + w) * kTreeBlock + tid] = v;
       }
     }
   }
 }
 
 template <int KERNEL, int PASS>
-void launch_near(int ngroups, int nfront, const FmmWork* w, const float* vw, int64_t ldv,
-                 int64_t ldr, int64_t n, unsigned long long* pairs, cudaStream_t st) {
+void launch_near(int ngroups, int64_t items, const FmmWork* w, const float* vw, int64_t ldv,
+                 int64_t n, unsigned long long* pairs, cudaStream_t st) {
   static const bool once = [] {
     cudaFuncSetAttribute(near_tile_kernel<KERNEL, PASS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          int(NearShape<PASS>::kSmem));
     return true;
   }();
   (void)once;
-  near_tile_kernel<KERNEL, PASS><<<ngroups, kNearThreads, NearShape<PASS>::kSmem, st>>>(
-      nfront, w->onear, w->nnear, w->near_list, w->rec, vw, ldv, w->near_raw, ldr, n, w->counters,
-      pairs);
+  near_tile_kernel<KERNEL, PASS><<<int(items), kNearThreads, NearShape<PASS>::kSmem, st>>>(
+      ngroups, w->gbase, w->gtot, w->totals, w->near_list, w->rec, vw, ldv, w->near_raw, n,
+      w->counters, pairs);
+}
+
+// Raw sum k of target t of a group: its near items in order.
+template <int NV>
+__device__ __forceinline__ double near_sum(const double* __restrict__ raw, int item0, int item1, int k,
+                                           int t) {
+  double v = 0.0;
+  for (int i = item0; i < item1; ++i) v += raw[(int64_t(i) * NV + k) * kTreeBlock + t];
+  return v;
+}
+__device__ __forceinline__ void group_items(const int* __restrict__ gbase,
+                                            const long long* __restrict__ totals, int ngroups, int g,
+                                            int& item0, int& item1) {
+  const int* first = gbase + int64_t(kListKinds) * ngroups;
+  item0 = first[g];
+  item1 = g + 1 < ngroups ? first[g + 1] : int(totals[3]);
+}
+
+// ζ sums of the near items to the original order.
+template <int NV>
+__global__ void __launch_bounds__(kTreeBlock) zeta_scatter_kernel(
+    int64_t n, int ngroups, const int* __restrict__ gbase, const long long* __restrict__ totals,
+    const double* __restrict__ raw, const int* __restrict__ perm, double* dst, int64_t ldd) {
+  const int64_t i = int64_t(blockIdx.x) * kTreeBlock + threadIdx.x;
+  if (i >= n) return;
+  int item0, item1;
+  group_items(gbase, totals, ngroups, int(blockIdx.x), item0, item1);
+  const int64_t o = perm[i];
+#pragma unroll 1
+  for (int k = 0; k < NV; ++k)
+    dst[k * ldd + o] = near_sum<NV>(raw, item0, item1, k, threadIdx.x);
 }
 
 // Rows of a Morton-ordered array back to the original order.
@@ -950,16 +1162,16 @@ __global__ void gather_rows_f32_kernel(int64_t n, int rows, const int* __restric
 // first particle; pairs with r = 0 skipped as in the direct FP64 sum).
 template <int KERNEL>
 __global__ void __launch_bounds__(kTreeBlock) near_f64_kernel(
-    int nfront, const int* __restrict__ onear, const int* __restrict__ nnear,
+    int ngroups, const int* __restrict__ gbase, const int* __restrict__ gtot,
     const int2* __restrict__ near_list, const double* __restrict__ sorted, int64_t ldw, double* raw,
-    int64_t ldr, int64_t n, int* counters) {
+    int64_t n, int* counters) {
   __shared__ double sx[kTreeBlock], sy[kTreeBlock], sz[kTreeBlock], sa_[kTreeBlock];
   __shared__ double sg0[kTreeBlock], sg1[kTreeBlock], sg2[kTreeBlock], sb_[kTreeBlock];
   const int tid = threadIdx.x;
   const int a = int(blockIdx.x) * kTreeBlock, b = int(min(int64_t(a) + kTreeBlock, n));
   const double cx = sorted[a], cy = sorted[ldw + a], cz = sorted[2 * ldw + a];
-  const int64_t t0s = int64_t(blockIdx.x) * nfront, t1s = t0s + nfront - 1;
-  const int l0 = onear[t0s], ln = onear[t1s] + nnear[t1s] - l0;
+  const int l0 = gbase[int64_t(LIST_NEAR) * ngroups + blockIdx.x];
+  const int ln = gtot[int64_t(LIST_NEAR) * ngroups + blockIdx.x];
   for (int t0 = a; t0 < b; t0 += kTreeBlock) {
     const int i = t0 + tid;
     double tx = 0.0, ty = 0.0, tz = 0.0;
@@ -1014,7 +1226,7 @@ __global__ void __launch_bounds__(kTreeBlock) near_f64_kernel(
     }
     if (i < b) {
 #pragma unroll
-      for (int k = 0; k < 15; ++k) raw[k * ldr + i] = acc[k];
+      for (int k = 0; k < 15; ++k) raw[(int64_t(blockIdx.x) * 15 + k) * kTreeBlock + tid] = acc[k];
     }
   }
 }
@@ -1073,8 +1285,8 @@ __device__ __forceinline__ float inv_fact3(int a, int b, int c) {
 }
 
 template <int P, int Q>
-__global__ void __launch_bounds__(32) m2l_kernel(int nfront, const int* __restrict__ oloc,
-                                                 const int* __restrict__ nloc,
+__global__ void __launch_bounds__(32) m2l_kernel(int ngroups, const int* __restrict__ gbase,
+                                                 const int* __restrict__ gtot,
                                                  const int* __restrict__ loc_list,
                                                  const double* __restrict__ geom,
                                                  const float* __restrict__ momf,
@@ -1131,8 +1343,7 @@ __global__ void __launch_bounds__(32) m2l_kernel(int nfront, const int* __restri
 #pragma unroll
   for (int q = 0; q < SLOTS; ++q) Lacc[q][0] = Lacc[q][1] = Lacc[q][2] = 0.f;
 
-  const int64_t t0s = int64_t(g) * nfront, t1s = t0s + nfront - 1;
-  const int f0 = oloc[t0s], fn = oloc[t1s] + nloc[t1s] - f0;
+  const int f0 = gbase[int64_t(LIST_LOC) * ngroups + g], fn = gtot[int64_t(LIST_LOC) * ngroups + g];
   for (int base = 0; base < fn; base += CH) {
     const int cnt = min(CH, fn - base);
     if (lane < cnt) {
@@ -1241,10 +1452,11 @@ __global__ void __launch_bounds__(32) m2l_kernel(int nfront, const int* __restri
 }
 
 // ---------------------------------------------------------------- far field --
-// One thread per target (CTA per target group): the moments of the group's far
-// cells at the target (M2P; the cells of the group's local expansion are on
-// their own list, and l2p_kernel adds them afterwards), plus the near-field
-// raw sums; U and J are written at the target's original index.
+// One thread per target (CTA per target group, the longest far lists first: they
+// are ten times the average, and one that starts last runs alone): the moments of
+// the group's far cells at the target (M2P; the cells of the group's local expansion
+// are on their own list).  U and J of the far field, without the 1/(4π), go to rows
+// of pot in Morton order; finish_kernel adds the other parts.
 // The group's far cells are taken kFarChunk at a time: the CTA stages their
 // moments and centres in shared memory with coalesced loads, then every thread
 // reads them from there (broadcast) for its target.
@@ -1253,26 +1465,25 @@ __host__ __device__ constexpr int far_chunk() {
   return 12288 / int(3 * ncoef(P) * sizeof(M)) > 0 ? 12288 / int(3 * ncoef(P) * sizeof(M)) : 1;
 }
 
-template <int P, int KERNEL, typename R, typename M, bool D>
+template <int P, typename R, typename M>
 __global__ void __launch_bounds__(kTreeBlock) far_kernel(
-    int64_t n, int nfront,
-    const int* __restrict__ ofar, const int* __restrict__ nfar, const int* __restrict__ far_list,
+    int64_t n, int ngroups, const int* __restrict__ gorder, const int* __restrict__ gbase,
+    const int* __restrict__ gtot, const int* __restrict__ far_list,
     const double* __restrict__ geom, const M* __restrict__ mom, const double* __restrict__ sorted,
-    int64_t ldw, const double* __restrict__ raw, int64_t ldr, const int* __restrict__ perm,
-    double* U, double* J, double* DJ, int64_t ldo, int ncells, int* counters,
+    int64_t ldw, R* __restrict__ pot, int64_t ldp, int ncells, int* counters,
     unsigned long long* pairs) {
   constexpr int NC = ncoef(P), ROWM = 3 * NC, FCH = far_chunk<P, M>();
   __shared__ M smom[FCH * ROWM];
   __shared__ R sctr[FCH][3];
-  const int a = int(blockIdx.x) * kTreeBlock, b = int(min(int64_t(a) + kTreeBlock, n));
+  const int g = gorder[blockIdx.x];
+  const int a = g * kTreeBlock, b = int(min(int64_t(a) + kTreeBlock, n));
   // Targets and cell centres relative to the group's first target, formed in
   // FP64 once per target and once per staged cell, so that the evaluations
   // subtract in R (GB300's FP64 pipe retires about two operations per SM and
   // cycle; three FP64 differences and conversions per evaluation cost more
   // than the FP32 work they feed).
   const double ox = sorted[a], oy = sorted[ldw + a], oz = sorted[2 * ldw + a];
-  const int64_t t0s = int64_t(blockIdx.x) * nfront, t1s = t0s + nfront - 1;
-  const int f0 = ofar[t0s], fn = ofar[t1s] + nfar[t1s] - f0;
+  const int f0 = gbase[g], fn = gtot[g];
   if (threadIdx.x == 0) atomicAdd(&pairs[1], (unsigned long long)fn * (unsigned long long)(b - a));
   const int i = a + int(threadIdx.x);
   const bool active = i < b;
@@ -1312,113 +1523,117 @@ __global__ void __launch_bounds__(kTreeBlock) far_kernel(
     if (!active) return;
     R uf[3], jf[9];
     curl_from_potential<R>(dp, dd, uf, jf);
-    double v[15];
 #pragma unroll
-    for (int k = 0; k < 15; ++k) v[k] = raw[k * ldr + i];
-    const double w = kInv4Pi, kp = kp_to_qr<KERNEL>();
-    const int64_t o = perm[i];
-    U[o] = -w * v[0] + w * double(uf[0]);
-    U[ldo + o] = -w * v[1] + w * double(uf[1]);
-    U[2 * ldo + o] = -w * v[2] + w * double(uf[2]);
-    const double w0 = v[12], w1 = v[13], w2 = v[14];
-    const double jn[9] = {kp * v[3],      kp * v[4] + w2, kp * v[5] - w1,
-                          kp * v[6] - w2, kp * v[7],      kp * v[8] + w0,
-                          kp * v[9] + w1, kp * v[10] - w0, kp * v[11]};
+    for (int k = 0; k < 3; ++k) pot[k * ldp + i] = uf[k];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) J[k * ldo + o] = -w * jn[k] + w * double(jf[k]);
-    if constexpr (D) {   // α-derivative: near field only (see near_tile_kernel)
-      const double d0 = raw[24 * ldr + i], d1 = raw[25 * ldr + i], d2 = raw[26 * ldr + i];
-      const double* a9 = raw + 15 * ldr + i;
-      const double jd[9] = {kp * a9[0],          kp * a9[ldr] + d2,     kp * a9[2 * ldr] - d1,
-                            kp * a9[3 * ldr] - d2, kp * a9[4 * ldr],    kp * a9[5 * ldr] + d0,
-                            kp * a9[6 * ldr] + d1, kp * a9[7 * ldr] - d0, kp * a9[8 * ldr]};
-#pragma unroll
-      for (int k = 0; k < 9; ++k) DJ[k * ldo + o] = -w * jd[k];
-    }
+    for (int k = 0; k < 9; ++k) pot[(3 + k) * ldp + i] = jf[k];
   }
 }
 
-// L2P: the group's local expansion at each of its targets, added to U and J
-// (after far_kernel wrote them) at the target's original index.  A kernel of
-// its own: inside far_kernel its registers would cut the M2P loop's occupancy.
-template <int Q>
-__global__ void __launch_bounds__(kTreeBlock) l2p_kernel(int64_t n, const float4* __restrict__ ggeom,
-                                                        const float* __restrict__ loc,
-                                                        const double* __restrict__ sorted,
-                                                        int64_t ldw, const int* __restrict__ perm,
-                                                        double* U, double* J, int64_t ldo) {
+// Final values of a group's targets, at their original indices: the near items'
+// raw sums, the far field of far_kernel and, with Q > 0, the group's local expansion
+// (L2P).  One CTA per group, thread = target.
+template <int KERNEL, typename R, bool D, int Q>
+__global__ void __launch_bounds__(kTreeBlock) finish_kernel(
+    int64_t n, int ngroups, const int* __restrict__ gbase, const long long* __restrict__ totals,
+    const double* __restrict__ raw, const R* __restrict__ pot, int64_t ldp,
+    const float4* __restrict__ ggeom, const float* __restrict__ loc,
+    const double* __restrict__ sorted, int64_t ldw, const int* __restrict__ perm, double* U,
+    double* J, double* DJ, int64_t ldo) {
+  constexpr int NV = D ? 27 : 15;
   const int64_t i = int64_t(blockIdx.x) * kTreeBlock + threadIdx.x;
   if (i >= n) return;
-  const float4 tg = ggeom[blockIdx.x];
-  const double ih = 1.0 / double(tg.w);
-  float dp[9], dd[18];
+  int item0, item1;
+  group_items(gbase, totals, ngroups, int(blockIdx.x), item0, item1);
+  float lu[3], lj[9];
+  if constexpr (Q > 0) {
+    const float4 tg = ggeom[blockIdx.x];
+    const double ih = 1.0 / double(tg.w);
+    float dp[9], dd[18];
 #pragma unroll
-  for (int k = 0; k < 9; ++k) dp[k] = 0.f;
+    for (int k = 0; k < 9; ++k) dp[k] = 0.f;
 #pragma unroll
-  for (int k = 0; k < 18; ++k) dd[k] = 0.f;
-  l2p_accumulate<Q, float>(loc + int64_t(blockIdx.x) * 3 * ncoef(Q),
-                           float((sorted[i] - double(tg.x)) * ih),
-                           float((sorted[ldw + i] - double(tg.y)) * ih),
-                           float((sorted[2 * ldw + i] - double(tg.z)) * ih), float(ih), dp, dd);
-  float uf[3], jf[9];
-  curl_from_potential<float>(dp, dd, uf, jf);
+    for (int k = 0; k < 18; ++k) dd[k] = 0.f;
+    l2p_accumulate<Q, float>(loc + int64_t(blockIdx.x) * 3 * ncoef(Q),
+                             float((sorted[i] - double(tg.x)) * ih),
+                             float((sorted[ldw + i] - double(tg.y)) * ih),
+                             float((sorted[2 * ldw + i] - double(tg.z)) * ih), float(ih), dp, dd);
+    curl_from_potential<float>(dp, dd, lu, lj);
+  }
+  const double w = kInv4Pi, kp = kp_to_qr<KERNEL>();
   const int64_t o = perm[i];
+  auto sum = [&](int k) { return near_sum<NV>(raw, item0, item1, k, threadIdx.x); };
 #pragma unroll
-  for (int k = 0; k < 3; ++k) U[k * ldo + o] += kInv4Pi * double(uf[k]);
+  for (int k = 0; k < 3; ++k) {
+    double u = -w * sum(k) + w * double(pot[k * ldp + i]);
+    if constexpr (Q > 0) u += w * double(lu[k]);
+    U[k * ldo + o] = u;
+  }
+  // J_ab = -(kp A_ab + ε_abc W_c)/(4π)
+  const double w3[3] = {sum(12), sum(13), sum(14)};
 #pragma unroll
-  for (int k = 0; k < 9; ++k) J[k * ldo + o] += kInv4Pi * double(jf[k]);
+  for (int k = 0; k < 9; ++k) {
+    const int a = k / 3, b = k % 3;
+    double v = kp * sum(3 + k);
+    if (a != b) v = (b - a + 3) % 3 == 1 ? v + w3[3 - a - b] : v - w3[3 - a - b];
+    double j = -w * v + w * double(pot[(3 + k) * ldp + i]);
+    if constexpr (Q > 0) j += w * double(lj[k]);
+    J[k * ldo + o] = j;
+  }
+  if constexpr (D) {   // α-derivative: near field only (see near_tile_kernel)
+    const double d3[3] = {sum(24), sum(25), sum(26)};
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+      const int a = k / 3, b = k % 3;
+      double v = kp * sum(15 + k);
+      if (a != b) v = (b - a + 3) % 3 == 1 ? v + d3[3 - a - b] : v - d3[3 - a - b];
+      DJ[k * ldo + o] = -w * v;
+    }
+  }
 }
 
 // ------------------------------------------------------------------- host --
 namespace {
 
-template <typename T>
-cudaError_t grow(T*& p, size_t& have, size_t need) {
-  if (need <= have) return cudaSuccess;
-  cudaFree(p);
-  p = nullptr;
-  have = 0;
-  cudaError_t e = cudaMalloc(&p, need * sizeof(T));
-  if (e == cudaSuccess) have = need;
-  return e;
-}
-
 cudaError_t reserve_particles(FmmWork* w, int64_t n) {
   if (n <= w->cap) return cudaSuccess;
   const int64_t cap = std::max<int64_t>(n, 1024);
   const int64_t cells = 2 * cap + 8;
-  void* ptrs[] = {w->codes, w->codes_alt, w->idx, w->perm, w->sorted, w->rec, w->near_raw,
-                  w->vw, w->lo, w->hi, w->child, w->nchild, w->geom, w->leaves, w->ggeom, w->cgeom,
-                  w->front, w->pairs, w->counters, w->box, w->box_part, w->nfar, w->nnear,
-                  w->ofar, w->onear, w->nloc, w->oloc, w->cub_tmp};
+  void* ptrs[] = {w->codes, w->codes_alt, w->idx, w->perm, w->sorted, w->rec, w->pot, w->vw,
+                  w->lo, w->hi, w->child, w->nchild, w->skip, w->geom, w->leaves, w->ggeom,
+                  w->cgeom, w->front, w->pairs, w->counters, w->box, w->box_part, w->wcnt,
+                  w->gtot, w->gbase, w->gorder, w->totals, w->cub_tmp};
   for (void* p : ptrs) cudaFree(p);
   cudaError_t e = cudaSuccess;
   auto al = [&](auto*& p, size_t count) {
     if (e == cudaSuccess) e = cudaMalloc(&p, count * sizeof(*p));
   };
   al(w->codes, cap); al(w->codes_alt, cap); al(w->idx, cap); al(w->perm, cap);
-  al(w->sorted, 7 * size_t(cap)); al(w->rec, 3 * size_t(cap)); al(w->near_raw, 27 * size_t(cap));
+  al(w->sorted, 7 * size_t(cap)); al(w->rec, 3 * size_t(cap)); al(w->pot, 12 * size_t(cap));
   al(w->vw, 6 * size_t(cap));
   al(w->lo, cells); al(w->hi, cells); al(w->child, cells); al(w->nchild, cells);
-  const int64_t meta = (cap / kTreeBlock + 2) * kMaxFront;
+  al(w->skip, cells);
+  const int64_t groups = cap / kTreeBlock + 2, meta = groups * kMaxFront;
   al(w->geom, size_t(cells) * kGeom); al(w->leaves, cells);
   al(w->ggeom, cap / kTreeBlock + 2); al(w->cgeom, 2 * size_t(cells));
   al(w->front, kMaxFront); al(w->pairs, 3);
   al(w->counters, kNumCounters); al(w->box, 4); al(w->box_part, kBoxBlocks * 6);
-  al(w->nfar, meta); al(w->nnear, meta); al(w->ofar, meta); al(w->onear, meta);
-  al(w->nloc, meta); al(w->oloc, meta);
+  al(w->wcnt, (kListKinds + 1) * size_t(meta)); al(w->gtot, (kListKinds + 1) * size_t(groups));
+  al(w->gbase, (kListKinds + 1) * size_t(groups)); al(w->gorder, groups); al(w->totals, 6);
   if (e != cudaSuccess) {
     w->cap = 0;
     return e;
   }
-  size_t sort_bytes = 0, scan_bytes = 0;
-  e = cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, w->codes, w->codes_alt, w->idx, w->perm,
-                                      int(cap), 0, 63);
-  if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, w->nfar, w->ofar, int(meta));
-  if (e == cudaSuccess) {
-    w->cub_bytes = std::max(sort_bytes, scan_bytes);
-    e = cudaMalloc(&w->cub_tmp, w->cub_bytes);
+  if (!w->aux) e = cudaStreamCreateWithFlags(&w->aux, cudaStreamNonBlocking);
+  if (e == cudaSuccess && !w->fork) e = cudaEventCreateWithFlags(&w->fork, cudaEventDisableTiming);
+  if (e == cudaSuccess && !w->join) e = cudaEventCreateWithFlags(&w->join, cudaEventDisableTiming);
+  if (e != cudaSuccess) {
+    w->cap = 0;
+    return e;
   }
+  e = cub::DeviceRadixSort::SortPairs(nullptr, w->cub_bytes, w->codes, w->codes_alt, w->idx, w->perm,
+                                      int(cap), 0, 63);
+  if (e == cudaSuccess) e = cudaMalloc(&w->cub_tmp, w->cub_bytes);
   if (e != cudaSuccess) {
     w->cap = 0;
     return e;
@@ -1433,20 +1648,20 @@ cudaError_t reserve_particles(FmmWork* w, int64_t n) {
 // the launches.
 template <int P>
 int launch_upward(FmmWork* w, int nleaves, int last_gen, bool f64, int64_t ldw, cudaStream_t st) {
-  const CellOut out = {w->geom, w->mom, f64 ? nullptr : w->momf, w->cgeom};
+  const CellOut out = {w->geom, w->mom, f64 ? nullptr : w->momf, w->cgeom, w->skip};
   tree_leaf_kernel<P><<<(nleaves + kLeafWarps - 1) / kLeafWarps, 32 * kLeafWarps, 0, st>>>(
       nleaves, w->leaves, w->lo, w->hi, w->sorted, ldw, out);
   int launches = 1;
   for (int g = last_gen - 1; g >= 0; --g, ++launches) {
     const int ncells_in_gen = w->h_counters[kGenBase + g + 1] - w->h_counters[kGenBase + g];
     tree_upward_kernel<P><<<std::min(ncells_in_gen, 4096), kUpThreads * kUpSlots, 0, st>>>(
-        g, w->counters, w->hi, w->child, w->nchild, out);
+        g, w->counters, w->child, w->nchild, out);
   }
   return launches;
 }
 
 template <int P, int Q>
-void launch_m2l(FmmWork* w, int ngroups, int nfront, int ncells, cudaStream_t st) {
+void launch_m2l(FmmWork* w, int ngroups, int ncells, cudaStream_t st) {
   static const bool once = [] {
     cudaFuncSetAttribute(m2l_kernel<P, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          int(M2lShape<P, Q>::kSmem));
@@ -1454,38 +1669,67 @@ void launch_m2l(FmmWork* w, int ngroups, int nfront, int ncells, cudaStream_t st
   }();
   (void)once;
   m2l_kernel<P, Q><<<ngroups, 32, M2lShape<P, Q>::kSmem, st>>>(
-      nfront, w->oloc, w->nloc, w->loc_list, w->geom, w->momf, w->ggeom, ncells, w->loc,
+      ngroups, w->gbase, w->gtot, w->loc_list, w->geom, w->momf, w->ggeom, ncells, w->loc,
       w->counters);
 }
 
-// The far field with local expansions where `local` (FP32, p = 4; see
-// fmm_eval), else M2P at every target.
 template <int P>
-cudaError_t launch_far(FmmWork* w, int kernel, bool f64, bool local, int64_t n, int ngroups,
-                       int nfront, int ncells, int64_t ldw, double* U, double* J, double* DJ,
-                       int64_t ldo, cudaStream_t st) {
-  const dim3 grid(ngroups), block(kTreeBlock);
-#define VPM_FAR(K, R, M, DD, mp)                                                                   \
-  far_kernel<P, K, R, M, DD><<<grid, block, 0, st>>>(n, nfront, w->ofar, w->nfar, w->far_list,    \
-                                                     w->geom, mp, w->sorted, ldw, w->near_raw, ldw, \
-                                                     w->perm, U, J, DJ, ldo, ncells, w->counters,   \
-                                                     w->pairs)
-  if (DJ) {   // FP32 Gaussian-erf only (checked by the caller)
-    VPM_FAR(VPM_KERNEL_GAUSSIANERF, float, float, true, w->momf);
-  } else if (kernel == VPM_KERNEL_WINCKELMANS) {
-    if (f64) VPM_FAR(VPM_KERNEL_WINCKELMANS, double, double, false, w->mom);
-    else VPM_FAR(VPM_KERNEL_WINCKELMANS, float, float, false, w->momf);
-  } else {
-    if (f64) VPM_FAR(VPM_KERNEL_GAUSSIANERF, double, double, false, w->mom);
-    else VPM_FAR(VPM_KERNEL_GAUSSIANERF, float, float, false, w->momf);
-  }
-#undef VPM_FAR
-  if constexpr (P == 4) {
-    if (local)
-      l2p_kernel<kLocalOrder><<<grid, block, 0, st>>>(n, w->ggeom, w->loc, w->sorted, ldw, w->perm,
-                                                      U, J, ldo);
-  }
-  return cudaGetLastError();
+void launch_far(FmmWork* w, bool f64, int64_t n, int ngroups, int ncells, int64_t ldw,
+                cudaStream_t st) {
+  if (f64)
+    far_kernel<P, double, double><<<ngroups, kTreeBlock, 0, st>>>(
+        n, ngroups, w->gorder, w->gbase, w->gtot, w->far_list, w->geom, w->mom, w->sorted, ldw,
+        w->pot, ldw, ncells, w->counters, w->pairs);
+  else
+    far_kernel<P, float, float><<<ngroups, kTreeBlock, 0, st>>>(
+        n, ngroups, w->gorder, w->gbase, w->gtot, w->far_list, w->geom, w->momf, w->sorted, ldw,
+        reinterpret_cast<float*>(w->pot), ldw, ncells, w->counters, w->pairs);
+}
+
+template <int KERNEL, typename R, bool D, int Q>
+void launch_finish(FmmWork* w, int64_t n, int ngroups, int64_t ldw, double* U, double* J, double* DJ,
+                   int64_t ldo, cudaStream_t st) {
+  finish_kernel<KERNEL, R, D, Q><<<ngroups, kTreeBlock, 0, st>>>(
+      n, ngroups, w->gbase, w->totals, w->near_raw, reinterpret_cast<const R*>(w->pot), ldw, w->ggeom,
+      w->loc, w->sorted, ldw, w->perm, U, J, DJ, ldo);
+}
+
+// FP64, or FP32 without and with local expansions; the α-derivative is FP32
+// Gaussian-erf only (checked by the caller).
+template <int KERNEL>
+void finish(FmmWork* w, bool f64, bool local, int64_t n, int ngroups, int64_t ldw, double* U, double* J,
+            double* DJ, int64_t ldo, cudaStream_t st) {
+  constexpr int Q = kLocalOrder, G = VPM_KERNEL_GAUSSIANERF;
+  if (DJ && local) launch_finish<G, float, true, Q>(w, n, ngroups, ldw, U, J, DJ, ldo, st);
+  else if (DJ) launch_finish<G, float, true, 0>(w, n, ngroups, ldw, U, J, DJ, ldo, st);
+  else if (f64) launch_finish<KERNEL, double, false, 0>(w, n, ngroups, ldw, U, J, nullptr, ldo, st);
+  else if (local) launch_finish<KERNEL, float, false, Q>(w, n, ngroups, ldw, U, J, nullptr, ldo, st);
+  else launch_finish<KERNEL, float, false, 0>(w, n, ngroups, ldw, U, J, nullptr, ldo, st);
+}
+
+// Room for the raw sums of the near items of a pass.
+cudaError_t reserve_raw(FmmWork* w, int64_t items, int nv) {
+  const size_t need = size_t(items) * nv * kTreeBlock;
+  if (need <= w->near_raw_cap) return cudaSuccess;
+  cudaFree(w->near_raw);
+  w->near_raw = nullptr;
+  w->near_raw_cap = 0;
+  const cudaError_t e = cudaMalloc(&w->near_raw, need * sizeof(double));
+  if (e == cudaSuccess) w->near_raw_cap = need;
+  return e;
+}
+
+// Room for `need` entries of a list.
+template <typename T>
+cudaError_t reserve_list(T*& p, int64_t& have, int64_t need) {
+  need = std::max<int64_t>(need, 1);
+  if (need <= have) return cudaSuccess;
+  cudaFree(p);
+  p = nullptr;
+  have = 0;
+  const cudaError_t e = cudaMalloc(&p, need * sizeof(T));
+  if (e == cudaSuccess) have = need;
+  return e;
 }
 
 }  // namespace
@@ -1557,11 +1801,11 @@ cudaError_t fmm_eval(vpm_ctx* c, int kernel, int prec, int p, int ncrit, double 
 
   // 2. tree, generation by generation
   stage = "tree build";
-  tree_init_kernel<<<1, 1, 0, st>>>(n, w->lo, w->hi, w->counters);
+  tree_init_kernel<<<1, 1, 0, st>>>(n, w->lo, w->hi, w->skip, w->counters);
   const int split_grid = int(std::min<int64_t>((w->cell_cap + 255) / 256, 4 * 152));
   for (int g = 0; g < kMaxGen - 1; ++g) {
     tree_split_kernel<<<split_grid, 256, 0, st>>>(g, ncrit, w->cell_cap, codes, w->lo, w->hi,
-                                                  w->child, w->nchild, w->leaves, w->counters);
+                                                  w->child, w->nchild, w->skip, w->leaves, w->counters);
   }
   if ((e = launched(1 + (kMaxGen - 1))) != cudaSuccess) return e;
   int* hc = w->h_counters;
@@ -1636,135 +1880,91 @@ cudaError_t fmm_eval(vpm_ctx* c, int kernel, int prec, int p, int ncrit, double 
   // 4. interaction lists: count, scan, fill
   stage = "traversal";
   const int tgrid = int((nwalk + 127) / 128);
-  traverse_kernel<false><<<tgrid, 128, 0, st>>>(nwalk, nfront, w->front, w->ggeom, w->cgeom,
-                                                float(theta), float(sfac), local, w->nfar,
-                                                w->nnear, w->nloc, nullptr, nullptr, nullptr,
-                                                nullptr, nullptr, nullptr, w->counters, ncells);
-  if ((e = launched(1)) != cudaSuccess) return e;
-  bytes = w->cub_bytes;
-  e = cub::DeviceScan::ExclusiveSum(w->cub_tmp, bytes, w->nfar, w->ofar, int(nwalk), st);
-  if (e == cudaSuccess) {
-    bytes = w->cub_bytes;
-    e = cub::DeviceScan::ExclusiveSum(w->cub_tmp, bytes, w->nnear, w->onear, int(nwalk), st);
-  }
-  if (e == cudaSuccess && local) {
-    bytes = w->cub_bytes;
-    e = cub::DeviceScan::ExclusiveSum(w->cub_tmp, bytes, w->nloc, w->oloc, int(nwalk), st);
-  }
-  if (e != cudaSuccess) return e;
-  c->launches += local ? 3 : 2;
-  int tail[6] = {0, 0, 0, 0, 0, 0};
-  e = cudaMemcpyAsync(&tail[0], w->ofar + nwalk - 1, sizeof(int), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&tail[1], w->nfar + nwalk - 1, sizeof(int), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&tail[2], w->onear + nwalk - 1, sizeof(int), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess)
-    e = cudaMemcpyAsync(&tail[3], w->nnear + nwalk - 1, sizeof(int), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess && local)
-    e = cudaMemcpyAsync(&tail[4], w->oloc + nwalk - 1, sizeof(int), cudaMemcpyDeviceToHost, st);
-  if (e == cudaSuccess && local)
-    e = cudaMemcpyAsync(&tail[5], w->nloc + nwalk - 1, sizeof(int), cudaMemcpyDeviceToHost, st);
+  int* nsrc = w->wcnt + kListKinds * nwalk;
+  traverse_kernel<false><<<tgrid, 128, 0, st>>>(ngroups, nfront, w->front, w->ggeom, w->cgeom,
+                                                float(theta), float(sfac), local, w->wcnt, nsrc,
+                                                nullptr, nullptr, nullptr, nullptr, w->counters,
+                                                ncells);
+  group_lists_kernel<<<(ngroups + 3) / 4, 128, 0, st>>>(ngroups, nfront, w->wcnt, nsrc, w->gtot);
+  group_scan_kernel<<<1, kScanThreads, 0, st>>>(ngroups, w->gtot, w->gbase, w->gorder, f64, w->totals);
+  if ((e = launched(3)) != cudaSuccess) return e;
+  long long totals[6];
+  e = cudaMemcpyAsync(totals, w->totals, sizeof(totals), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return e;
-  const int64_t nf = int64_t(tail[0]) + tail[1], nn = int64_t(tail[2]) + tail[3];
-  const int64_t nl = int64_t(tail[4]) + tail[5];
+  const int64_t nf = totals[LIST_FAR], nn = totals[LIST_NEAR], nl = totals[LIST_LOC], items = totals[3];
   if (nf > INT32_MAX || nn > INT32_MAX || nl > INT32_MAX) {
     *why = "treecode interaction lists exceed 2^31 entries";
     return cudaErrorInvalidValue;
   }
-  const int64_t need = std::max<int64_t>(std::max(nf, nn), 1);
-  if (need > w->list_cap) {
-    cudaFree(w->far_list);
-    cudaFree(w->near_list);
-    w->far_list = nullptr;
-    w->near_list = nullptr;
-    w->list_cap = 0;
-    e = cudaMalloc(&w->far_list, need * sizeof(int));
-    if (e == cudaSuccess) e = cudaMalloc(&w->near_list, need * sizeof(int2));
-    if (e != cudaSuccess) return e;
-    w->list_cap = need;
-  }
-  if (local && std::max<int64_t>(nl, 1) > w->loc_list_cap) {
-    cudaFree(w->loc_list);
-    w->loc_list = nullptr;
-    w->loc_list_cap = 0;
-    e = cudaMalloc(&w->loc_list, std::max<int64_t>(nl, 1) * sizeof(int));
-    if (e != cudaSuccess) return e;
-    w->loc_list_cap = std::max<int64_t>(nl, 1);
-  }
+  e = reserve_list(w->far_list, w->far_cap, nf);
+  if (e == cudaSuccess) e = reserve_list(w->near_list, w->near_cap, nn);
+  if (e == cudaSuccess && local) e = reserve_list(w->loc_list, w->loc_cap_list, nl);
+  if (e == cudaSuccess) e = reserve_raw(w, items, dj ? 27 : 15);
+  if (e == cudaSuccess && local)
+    e = reserve_list(w->loc, w->loc_cap, int64_t(ngroups) * 3 * ncoef(kLocalOrder));
+  if (e != cudaSuccess) return e;
   e = cudaMemsetAsync(w->pairs, 0, 2 * sizeof(unsigned long long), st);
   if (e != cudaSuccess) return e;
-  traverse_kernel<true><<<tgrid, 128, 0, st>>>(nwalk, nfront, w->front, w->ggeom, w->cgeom,
-                                               float(theta), float(sfac), local, w->nfar,
-                                               w->nnear, w->nloc, w->ofar, w->onear, w->oloc,
-                                               w->far_list, w->near_list, w->loc_list,
+  traverse_kernel<true><<<tgrid, 128, 0, st>>>(ngroups, nfront, w->front, w->ggeom, w->cgeom,
+                                               float(theta), float(sfac), local, w->wcnt, nsrc,
+                                               w->gbase, w->far_list, w->near_list, w->loc_list,
                                                w->counters, ncells);
   if ((e = launched(1)) != cudaSuccess) return e;
 
-  // 5. local expansions of the groups (M2L)
-  if (local) {
-    stage = "local expansions";
-    constexpr int NQ = ncoef(kLocalOrder);
-    if (int64_t(ngroups) * 3 * NQ > w->loc_cap) {
-      cudaFree(w->loc);
-      w->loc = nullptr;
-      w->loc_cap = 0;
-      e = cudaMalloc(&w->loc, size_t(ngroups) * 3 * NQ * sizeof(float));
-      if (e != cudaSuccess) return e;
-      w->loc_cap = int64_t(ngroups) * 3 * NQ;
-    }
-    launch_m2l<4, kLocalOrder>(w, ngroups, nfront, ncells, st);
-    if ((e = launched(1)) != cudaSuccess) return e;
-  }
-
-  // 6. near field, 7. far field + output
-  stage = "near field";
+  // 5.-7. far field (M2P) and local expansions (M2L) on the second stream, the near
+  // field on the context's: they share nothing that is written, each leaves parts of
+  // the chip idle at its end, and the M2L kernel (a warp per group) all along.
+  e = cudaEventRecord(w->fork, st);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(w->aux, w->fork, 0);
+  if (e != cudaSuccess) return e;
+  stage = "far field";
+  if (p == 2) launch_far<2>(w, f64, n, ngroups, ncells, ldw, w->aux);
+  else if (p == 4) launch_far<4>(w, f64, n, ngroups, ncells, ldw, w->aux);
+  else launch_far<6>(w, f64, n, ngroups, ncells, ldw, w->aux);
+  if (local) launch_m2l<4, kLocalOrder>(w, ngroups, ncells, w->aux);
   if (f64) {
     if (kernel == VPM_KERNEL_WINCKELMANS)
       near_f64_kernel<VPM_KERNEL_WINCKELMANS><<<ngroups, kTreeBlock, 0, st>>>(
-          nfront, w->onear, w->nnear, w->near_list, w->sorted, ldw, w->near_raw, ldw, n,
-          w->counters);
+          ngroups, w->gbase, w->gtot, w->near_list, w->sorted, ldw, w->near_raw, n, w->counters);
     else
       near_f64_kernel<VPM_KERNEL_GAUSSIANERF><<<ngroups, kTreeBlock, 0, st>>>(
-          nfront, w->onear, w->nnear, w->near_list, w->sorted, ldw, w->near_raw, ldw, n,
-          w->counters);
+          ngroups, w->gbase, w->gtot, w->near_list, w->sorted, ldw, w->near_raw, n, w->counters);
+  } else if (dj) {
+    launch_near<VPM_KERNEL_GAUSSIANERF, PASS_UJD>(ngroups, items, w, nullptr, 0, n, w->pairs, st);
+  } else if (kernel == VPM_KERNEL_WINCKELMANS) {
+    launch_near<VPM_KERNEL_WINCKELMANS, PASS_UJ>(ngroups, items, w, nullptr, 0, n, w->pairs, st);
   } else {
-    if (dj)
-      launch_near<VPM_KERNEL_GAUSSIANERF, PASS_UJD>(ngroups, nfront, w, nullptr, 0, ldw, n,
-                                                    w->pairs, st);
-    else if (kernel == VPM_KERNEL_WINCKELMANS)
-      launch_near<VPM_KERNEL_WINCKELMANS, PASS_UJ>(ngroups, nfront, w, nullptr, 0, ldw, n,
-                                                   w->pairs, st);
-    else
-      launch_near<VPM_KERNEL_GAUSSIANERF, PASS_UJ>(ngroups, nfront, w, nullptr, 0, ldw, n,
-                                                   w->pairs, st);
+    launch_near<VPM_KERNEL_GAUSSIANERF, PASS_UJ>(ngroups, items, w, nullptr, 0, n, w->pairs, st);
   }
-  if ((e = launched(1)) != cudaSuccess) return e;
-  if (p == 2)
-    e = launch_far<2>(w, kernel, f64, local, n, ngroups, nfront, ncells, ldw, c->U, c->J, dj,
-                      c->ld, st);
-  else if (p == 4)
-    e = launch_far<4>(w, kernel, f64, local, n, ngroups, nfront, ncells, ldw, c->U, c->J, dj,
-                      c->ld, st);
+  const cudaError_t le = launched(2 + local);
+  // The second stream always rejoins, whatever failed.
+  e = cudaEventRecord(w->join, w->aux);
+  if (e == cudaSuccess) e = cudaStreamWaitEvent(st, w->join, 0);
+  if (e != cudaSuccess) cudaStreamSynchronize(w->aux);
+  if (le != cudaSuccess) return le;
+  if (e != cudaSuccess) return e;
+
+  // 8. final values
+  stage = "output";
+  if (kernel == VPM_KERNEL_WINCKELMANS)
+    finish<VPM_KERNEL_WINCKELMANS>(w, f64, local, n, ngroups, ldw, c->U, c->J, dj, c->ld, st);
   else
-    e = launch_far<6>(w, kernel, f64, local, n, ngroups, nfront, ncells, ldw, c->U, c->J, dj,
-                      c->ld, st);
-  stage = "far field";
-  if ((e = e == cudaSuccess ? launched(local ? 2 : 1) : e) != cudaSuccess) return e;
+    finish<VPM_KERNEL_GAUSSIANERF>(w, f64, local, n, ngroups, ldw, c->U, c->J, dj, c->ld, st);
+  if ((e = launched(1)) != cudaSuccess) return e;
   e = cudaMemcpyAsync(hc, w->counters, sizeof(int) * kGenBase, cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess)
     e = cudaMemcpyAsync(w->h_pairs, w->pairs, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return e;
   if (hc[kCntFlags] != 0) {
-    *why = (hc[2] & 2) ? "tree traversal stack overflow" : "treecode index out of range (checked, skipped)";
+    *why = "treecode index out of range (checked, skipped)";
     return cudaErrorInvalidValue;
   }
   w->last_cells = ncells;
   w->last_leaves = nleaves;
   w->last_groups = ngroups;
-  w->last_nfront = nfront;
+  w->last_items = items;
   w->last_far = nf + nl;
   w->h_pairs[2] = (unsigned long long)nl;
   w->last_near = nn;
@@ -1787,18 +1987,23 @@ cudaError_t fmm_zeta(vpm_ctx* c, bool d, const double* vs, const double* ws, dou
   }
   cudaStream_t st = c->st;
   const int64_t ldw = w->cap;
-  const int ngroups = int(w->last_groups), nfront = int(w->last_nfront);
+  const int ngroups = int(w->last_groups);
+  const int64_t items = w->last_items;
   const int grid = int((n + 255) / 256);
+  const cudaError_t re = reserve_raw(w, items, d ? 12 : 6);
+  if (re != cudaSuccess) return re;
   gather_rows_f32_kernel<<<grid, 256, 0, st>>>(n, 3, w->perm, vs, c->ld, w->vw, ldw);
   if (d)
     gather_rows_f32_kernel<<<grid, 256, 0, st>>>(n, 3, w->perm, ws, c->ld, w->vw + 3 * ldw, ldw);
-  if (d)
-    launch_near<VPM_KERNEL_GAUSSIANERF, PASS_ZETAD>(ngroups, nfront, w, w->vw, ldw, ldw, n,
-                                                    nullptr, st);
-  else
-    launch_near<VPM_KERNEL_GAUSSIANERF, PASS_ZETA>(ngroups, nfront, w, w->vw, ldw, ldw, n,
-                                                   nullptr, st);
-  scatter_rows_kernel<<<grid, 256, 0, st>>>(n, d ? 12 : 6, w->perm, w->near_raw, ldw, out, c->ld);
+  if (d) {
+    launch_near<VPM_KERNEL_GAUSSIANERF, PASS_ZETAD>(ngroups, items, w, w->vw, ldw, n, nullptr, st);
+    zeta_scatter_kernel<12><<<ngroups, kTreeBlock, 0, st>>>(n, ngroups, w->gbase, w->totals,
+                                                            w->near_raw, w->perm, out, c->ld);
+  } else {
+    launch_near<VPM_KERNEL_GAUSSIANERF, PASS_ZETA>(ngroups, items, w, w->vw, ldw, n, nullptr, st);
+    zeta_scatter_kernel<6><<<ngroups, kTreeBlock, 0, st>>>(n, ngroups, w->gbase, w->totals,
+                                                           w->near_raw, w->perm, out, c->ld);
+  }
   c->launches += d ? 4 : 3;
   return cudaGetLastError();
 }

@@ -229,3 +229,22 @@ def test_upward_pass_at_the_edges_of_its_warps_and_slots(oracle, n, ncrit, p):
     assert np.array_equal(U, U2) and np.array_equal(J, J2)
     if n > 1:
         assert rel_l2(U, U0) <= bound and rel_l2(J, J0) <= bound
+
+
+@pytest.mark.parametrize("k", [L.KERNEL_WINCKELMANS, L.KERNEL_GAUSSIANERF])
+@pytest.mark.parametrize("n,ncrit", [(63, 50), (64, 1), (2114, 1), (20000, 300)])
+def test_near_items_cover_every_range_once(oracle, k, n, ncrit):
+    # With every cell near, a group's near field is the whole field, dealt to several
+    # near items: ranges that end inside tiles (ncrit 1: far more than 128 ranges a
+    # group), a last short group, items that end inside a chunk of ranges.  A range
+    # left out or summed twice shows at 1/n of the field or more; 1e-5 is what FP32C
+    # sums are held to against the oracle everywhere.
+    X, G, S = uniform_box(n, seed_index=143)
+    idx = np.sort(np.random.default_rng(5).choice(n, min(n, 500), replace=False))
+    U0, J0 = oracle.uj_direct(k, X, G, S, Xt=X[idx])
+    with Ctx(n) as c:
+        c.set(X, G, S)
+        U, J = eval_fmm(c, k, L.PREC_FP32C, fmm(theta=0.001, ncrit=ncrit))
+        st = all_stats(c)
+    assert st["far_entries"] == 0 and st["near_pairs"] == n * n
+    assert rel_l2(U[idx], U0) <= 1e-5 and rel_l2(J[idx], J0) <= 1e-5
