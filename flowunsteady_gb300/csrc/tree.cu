@@ -1095,13 +1095,18 @@ void launch_near(int ngroups, int64_t items, const FmmWork* w, const float* vw, 
       w->counters, pairs);
 }
 
-// Raw sum k of target t of a group: its near items in order.
-template <int NV>
-__device__ __forceinline__ double near_sum(const double* __restrict__ raw, int item0, int item1, int k,
-                                           int t) {
-  double v = 0.0;
-  for (int i = item0; i < item1; ++i) v += raw[(int64_t(i) * NV + k) * kTreeBlock + t];
-  return v;
+// Raw sums [K0, K0 + K) of target t of a group: its near items in order, all K loads
+// of an item in flight together (a group has up to 30 items).
+template <int NV, int K0, int K>
+__device__ __forceinline__ void near_sums(const double* __restrict__ raw, int item0, int item1, int t,
+                                          double (&v)[K]) {
+#pragma unroll
+  for (int k = 0; k < K; ++k) v[k] = 0.0;
+  for (int i = item0; i < item1; ++i) {
+    const double* r = raw + (int64_t(i) * NV + K0) * kTreeBlock + t;
+#pragma unroll
+    for (int k = 0; k < K; ++k) v[k] += r[k * kTreeBlock];
+  }
 }
 __device__ __forceinline__ void group_items(const int* __restrict__ gbase,
                                             const long long* __restrict__ totals, int ngroups, int g,
@@ -1121,9 +1126,10 @@ __global__ void __launch_bounds__(kTreeBlock) zeta_scatter_kernel(
   int item0, item1;
   group_items(gbase, totals, ngroups, int(blockIdx.x), item0, item1);
   const int64_t o = perm[i];
-#pragma unroll 1
-  for (int k = 0; k < NV; ++k)
-    dst[k * ldd + o] = near_sum<NV>(raw, item0, item1, k, threadIdx.x);
+  double v[NV];
+  near_sums<NV, 0, NV>(raw, item0, item1, threadIdx.x, v);
+#pragma unroll
+  for (int k = 0; k < NV; ++k) dst[k * ldd + o] = v[k];
 }
 
 // Rows of a Morton-ordered array back to the original order.
@@ -1238,25 +1244,29 @@ __global__ void __launch_bounds__(kTreeBlock) near_f64_kernel(
 // target (L2P) and skips them in its M2P loop.
 constexpr int kLocalOrder = 7;   // Q for P = 4: L2P within a few per cent of M2P in J (tree.cuh)
 
-// One warp per target group.  The group's local-expansion cells are taken
+// Two warps per target group.  The group's local-expansion cells are taken
 // kM2lChunk at a time; then
-//   1. each of the first kM2lChunk lanes forms its cell's ρ, s and powers, and
-//      B̃_j for |j| <= P + Q (one shared-memory row per cell);
-//   2. the warp loads the chunk's moments coalesced and scales them by
-//      ρ^{|k|}/k!;
-//   3. lane l accumulates the local coefficients n = l + 32·q over the chunk's
-//      cells, Σ_k M̃_k B̃_{k+n} times ρ(-s)^{|n|}/n!, two coefficients per
-//      packed FP32 instruction.
-// The group's coefficients go to loc[g·3·NQ + m·NQ + n].  Chunks of 16 cells
-// keep the shared memory of a warp near 33 KB (six warps per SM).
-constexpr int kM2lChunk = 16;
+//   1. one lane per cell forms its ρ, s and powers;
+//   2. four lanes per cell form B̃_j for |j| <= P + Q, order by order (one
+//      shared-memory row per cell);
+//   3. the moments are loaded coalesced and scaled by ρ^{|k|}/k!;
+//   4. lane l of warp v accumulates the local coefficients n = l + 32·(2q + v),
+//      q = 0, 1, over the chunk's cells, Σ_k M̃_k B̃_{k+n} times ρ(-s)^{|n|}/n!, two
+//      coefficients per packed FP32 instruction.
+// The group's coefficients go to loc[g·3·NQ + m·NQ + n].  Bound by shared-memory
+// loads: 35 moments (one broadcast each) and 35·4 gathers of B̃ (2.1 wavefronts on
+// average) a cell, beside the 120·35·3 FMAs, which take a quarter of that.  The
+// chunk's 33 KB leave six groups on an SM.  With one warp a group and one lane a
+// cell in step 2 those were six warps with half their lanes idle a third of the
+// time: 11.1 ms at N = 500,000, now 8.4 ms.
+constexpr int kM2lChunk = 16, kM2lThreads = 64;
 
 template <int P, int Q>
 struct M2lShape {
   static constexpr int NC = ncoef(P), NQ = ncoef(Q), NB = ncoef(P + Q);
   static constexpr int ROW = NB % 2 ? NB : NB + 1;        // odd stride: lanes' rows hit distinct banks
   static constexpr int NPOW = (P + 1) + (Q + 1);          // ρ^0..ρ^P, then ρ(-s)^0..ρ(-s)^Q
-  static constexpr int SLOTS = (NQ + 31) / 32;            // coefficients per lane
+  static constexpr int SLOTS = (NQ + 63) / 64;            // coefficients per lane
   static constexpr size_t kSmem = size_t(kM2lChunk) * ROW * sizeof(float) +
                                   size_t(kM2lChunk) * NC * sizeof(float4) +
                                   size_t(kM2lChunk) * NPOW * sizeof(float);
@@ -1285,7 +1295,7 @@ __device__ __forceinline__ float inv_fact3(int a, int b, int c) {
 }
 
 template <int P, int Q>
-__global__ void __launch_bounds__(32) m2l_kernel(int ngroups, const int* __restrict__ gbase,
+__global__ void __launch_bounds__(kM2lThreads) m2l_kernel(int ngroups, const int* __restrict__ gbase,
                                                  const int* __restrict__ gtot,
                                                  const int* __restrict__ loc_list,
                                                  const double* __restrict__ geom,
@@ -1300,18 +1310,19 @@ __global__ void __launch_bounds__(32) m2l_kernel(int ngroups, const int* __restr
   float* sB = reinterpret_cast<float*>(m2l_smem + size_t(CH) * NC * sizeof(float4));   // [cell][j]
   float* sP = sB + CH * ROW;                                                     // [cell][NPOW]
   __shared__ int ids[CH];
-  const int lane = threadIdx.x;
+  __shared__ float4 dir[CH];
+  const int tid = threadIdx.x, lane = tid & 31, wv = tid >> 5;
   const int g = blockIdx.x;
   const float4 tg = ggeom[g];
   const double zx = tg.x, zy = tg.y, zz = tg.z;
   const double h = tg.w;
 
-  // This lane's local coefficients n = lane + 32·q: index tables of k + n.
+  // This lane's local coefficients n = lane + 32·(2q + warp): index tables of k + n.
   int t3[SLOTS][P + 1], t2[SLOTS][P + 1], ncs[SLOTS], nord[SLOTS];
   float invf[SLOTS];
 #pragma unroll
   for (int q = 0; q < SLOTS; ++q) {
-    const int n = lane + 32 * q;
+    const int n = lane + 32 * (2 * q + wv);
     int na = 0, nb = 0, nc = 0;
     if (n < NQ) decode_midx(n, na, nb, nc);
     const int nn = na + nb + nc;
@@ -1326,13 +1337,13 @@ __global__ void __launch_bounds__(32) m2l_kernel(int ngroups, const int* __restr
       t2[q][K] = M * (M + 1) / 2;
     }
   }
-  // The moment elements e = lane + 32·i of a cell row this lane scales.
-  constexpr int NE = (3 * NC + 31) / 32;
+  // The moment elements e = tid + 64·i of a cell row this thread scales.
+  constexpr int NE = (3 * NC + kM2lThreads - 1) / kM2lThreads;
   int eord[NE];
   float efac[NE];
 #pragma unroll
   for (int i = 0; i < NE; ++i) {
-    const int e = lane + 32 * i;
+    const int e = tid + kM2lThreads * i;
     int a = 0, b = 0, c = 0;
     if (e < 3 * NC) decode_midx(e % NC, a, b, c);
     eord[i] = a + b + c;
@@ -1346,18 +1357,17 @@ __global__ void __launch_bounds__(32) m2l_kernel(int ngroups, const int* __restr
   const int f0 = gbase[int64_t(LIST_LOC) * ngroups + g], fn = gtot[int64_t(LIST_LOC) * ngroups + g];
   for (int base = 0; base < fn; base += CH) {
     const int cnt = min(CH, fn - base);
-    if (lane < cnt) {
-      int cell = loc_list[f0 + base + lane];
-      if (cell < 0 || cell >= ncells) {   // a list entry outside the tree: record, skip
-        atomicOr(&counters[kCntFlags], 4);
-        cell = -1;
+    // 1. scale factors of cell tid, and its direction for the lanes of step 2.
+    if (tid < CH) {
+      int cell = -1;
+      if (tid < cnt) {
+        cell = loc_list[f0 + base + tid];
+        if (cell < 0 || cell >= ncells) {   // a list entry outside the tree: record, skip
+          atomicOr(&counters[kCntFlags], 4);
+          cell = -1;
+        }
       }
-      ids[lane] = cell;
-    }
-    __syncwarp();
-    // 1. this lane's cell: scale factors and B̃ row.
-    if (lane < CH) {
-      const int cell = lane < cnt ? ids[lane] : -1;
+      ids[tid] = cell;
       double rho = 0.0;
       float rx = 1.f, ry = 0.f, rz = 0.f;
       if (cell >= 0) {
@@ -1367,7 +1377,8 @@ __global__ void __launch_bounds__(32) m2l_kernel(int ngroups, const int* __restr
         rho = 1.0 / sqrt(dx * dx + dy * dy + dz * dz);
         rx = float(dx * rho); ry = float(dy * rho); rz = float(dz * rho);
       }
-      float* pw = sP + lane * NPOW;
+      dir[tid] = make_float4(rx, ry, rz, 0.f);
+      float* pw = sP + tid * NPOW;
       float v = 1.f;
 #pragma unroll
       for (int j = 0; j <= P; ++j) {
@@ -1381,17 +1392,21 @@ __global__ void __launch_bounds__(32) m2l_kernel(int ngroups, const int* __restr
         pw[P + 1 + j] = v;
         v *= ns;
       }
-      scaled_taylor_unit<P + Q>(rx, ry, rz, sB + lane * ROW);
     }
-    __syncwarp();
-    // 2. moments of the chunk's cells, coalesced, scaled by ρ^{|k|}/k!.
+    __syncthreads();
+    // 2. B̃ rows: lanes 4c .. 4c + 3 of the block for cell c.
+    {
+      const float4 r = dir[tid >> 2];
+      scaled_taylor_unit4<P + Q>(r.x, r.y, r.z, tid & 3, sB + (tid >> 2) * ROW);
+    }
+    // 3. moments of the chunk's cells, coalesced, scaled by ρ^{|k|}/k!.
     for (int c = 0; c < cnt; ++c) {
       const int cell = ids[c];
       const float* row = momf + int64_t(cell < 0 ? 0 : cell) * 3 * NC;
       const float* pw = sP + c * NPOW;
 #pragma unroll
       for (int i = 0; i < NE; ++i) {
-        const int e = lane + 32 * i;
+        const int e = tid + kM2lThreads * i;
         if (e < 3 * NC) {
           const int m = e / NC, k = e % NC;
           reinterpret_cast<float*>(&sM[c * NC + k])[m] =
@@ -1399,8 +1414,8 @@ __global__ void __launch_bounds__(32) m2l_kernel(int ngroups, const int* __restr
         }
       }
     }
-    __syncwarp();
-    // 3. local coefficients, slots (2h, 2h + 1) packed.
+    __syncthreads();
+    // 4. local coefficients, slots (2h, 2h + 1) packed.
     for (int c = 0; c < cnt; ++c) {
       const float* brow = sB + c * ROW;
       const float4* mrow = sM + c * NC;
@@ -1437,12 +1452,12 @@ __global__ void __launch_bounds__(32) m2l_kernel(int ngroups, const int* __restr
         }
       }
     }
-    __syncwarp();
+    __syncthreads();
   }
   float* out = loc + int64_t(g) * 3 * NQ;
 #pragma unroll
   for (int q = 0; q < SLOTS; ++q) {
-    const int n = lane + 32 * q;
+    const int n = lane + 32 * (2 * q + wv);
     if (n < NQ) {
       out[n] = Lacc[q][0];
       out[NQ + n] = Lacc[q][1];
@@ -1462,7 +1477,7 @@ __global__ void __launch_bounds__(32) m2l_kernel(int ngroups, const int* __restr
 // reads them from there (broadcast) for its target.
 template <int P, typename M>
 __host__ __device__ constexpr int far_chunk() {
-  return 12288 / int(3 * ncoef(P) * sizeof(M)) > 0 ? 12288 / int(3 * ncoef(P) * sizeof(M)) : 1;
+  return 12288 / int(ncoef(P) * sizeof(M4<M>)) > 0 ? 12288 / int(ncoef(P) * sizeof(M4<M>)) : 1;
 }
 
 template <int P, typename R, typename M>
@@ -1473,7 +1488,9 @@ __global__ void __launch_bounds__(kTreeBlock) far_kernel(
     int64_t ldw, R* __restrict__ pot, int64_t ldp, int ncells, int* counters,
     unsigned long long* pairs) {
   constexpr int NC = ncoef(P), ROWM = 3 * NC, FCH = far_chunk<P, M>();
-  __shared__ M smom[FCH * ROWM];
+  // The three components of a moment together: one broadcast load, where a row of
+  // each took three (a third of the kernel's shared-memory instructions remain).
+  __shared__ M4<M> smom[FCH * NC];
   __shared__ R sctr[FCH][3];
   const int g = gorder[blockIdx.x];
   const int a = g * kTreeBlock, b = int(min(int64_t(a) + kTreeBlock, n));
@@ -1501,7 +1518,9 @@ __global__ void __launch_bounds__(kTreeBlock) far_kernel(
       for (int e = int(threadIdx.x); e < cnt * ROWM; e += kTreeBlock) {
         const int c = e / ROWM, k = e - c * ROWM;
         const int s = far_list[f0 + c0 + c];
-        smom[e] = (s < 0 || s >= ncells) ? M(0) : mom[int64_t(s) * ROWM + k];
+        const int m = k / NC;
+        reinterpret_cast<M*>(&smom[c * NC + (k - m * NC)])[m] =
+            (s < 0 || s >= ncells) ? M(0) : mom[int64_t(s) * ROWM + k];
       }
       for (int c = int(threadIdx.x); c < cnt; c += kTreeBlock) {
         const int s = far_list[f0 + c0 + c];
@@ -1517,7 +1536,7 @@ __global__ void __launch_bounds__(kTreeBlock) far_kernel(
       for (int c = 0; c < cnt; ++c) {
         R bk[ncoef(P + 2)];
         taylor_coefficients<P + 2, R>(x - sctr[c][0], y - sctr[c][1], z - sctr[c][2], bk);
-        m2p_accumulate<P, R, M>(bk, smom + c * ROWM, dp, dd);
+        m2p_accumulate<P, R, M>(bk, smom + c * NC, dp, dd);
       }
     }
     if (!active) return;
@@ -1562,31 +1581,32 @@ __global__ void __launch_bounds__(kTreeBlock) finish_kernel(
   }
   const double w = kInv4Pi, kp = kp_to_qr<KERNEL>();
   const int64_t o = perm[i];
-  auto sum = [&](int k) { return near_sum<NV>(raw, item0, item1, k, threadIdx.x); };
+  double v15[15];
+  near_sums<NV, 0, 15>(raw, item0, item1, threadIdx.x, v15);
 #pragma unroll
   for (int k = 0; k < 3; ++k) {
-    double u = -w * sum(k) + w * double(pot[k * ldp + i]);
+    double u = -w * v15[k] + w * double(pot[k * ldp + i]);
     if constexpr (Q > 0) u += w * double(lu[k]);
     U[k * ldo + o] = u;
   }
   // J_ab = -(kp A_ab + ε_abc W_c)/(4π)
-  const double w3[3] = {sum(12), sum(13), sum(14)};
 #pragma unroll
   for (int k = 0; k < 9; ++k) {
     const int a = k / 3, b = k % 3;
-    double v = kp * sum(3 + k);
-    if (a != b) v = (b - a + 3) % 3 == 1 ? v + w3[3 - a - b] : v - w3[3 - a - b];
+    double v = kp * v15[3 + k];
+    if (a != b) v = (b - a + 3) % 3 == 1 ? v + v15[15 - a - b] : v - v15[15 - a - b];
     double j = -w * v + w * double(pot[(3 + k) * ldp + i]);
     if constexpr (Q > 0) j += w * double(lj[k]);
     J[k * ldo + o] = j;
   }
   if constexpr (D) {   // α-derivative: near field only (see near_tile_kernel)
-    const double d3[3] = {sum(24), sum(25), sum(26)};
+    double d12[12];
+    near_sums<NV, 15, 12>(raw, item0, item1, threadIdx.x, d12);
 #pragma unroll
     for (int k = 0; k < 9; ++k) {
       const int a = k / 3, b = k % 3;
-      double v = kp * sum(15 + k);
-      if (a != b) v = (b - a + 3) % 3 == 1 ? v + d3[3 - a - b] : v - d3[3 - a - b];
+      double v = kp * d12[k];
+      if (a != b) v = (b - a + 3) % 3 == 1 ? v + d12[12 - a - b] : v - d12[12 - a - b];
       DJ[k * ldo + o] = -w * v;
     }
   }
@@ -1668,7 +1688,7 @@ void launch_m2l(FmmWork* w, int ngroups, int ncells, cudaStream_t st) {
     return true;
   }();
   (void)once;
-  m2l_kernel<P, Q><<<ngroups, 32, M2lShape<P, Q>::kSmem, st>>>(
+  m2l_kernel<P, Q><<<ngroups, kM2lThreads, M2lShape<P, Q>::kSmem, st>>>(
       ngroups, w->gbase, w->gtot, w->loc_list, w->geom, w->momf, w->ggeom, ncells, w->loc,
       w->counters);
 }

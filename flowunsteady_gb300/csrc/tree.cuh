@@ -77,14 +77,19 @@ __device__ __forceinline__ void taylor_coefficients(R rx, R ry, R rz, R (&bk)[nc
   }
 }
 
-// Contract the moments of one cell (mom[m·NC + k], NC = ncoef(P)) with the
+// The three components of one moment.
+template <typename M>
+struct alignas(4 * sizeof(M)) M4 {
+  M x, y, z, w;
+};
+
+// Contract the moments of one cell (mom[k], components x, y, z) with the
 // coefficients at R = x - c: dpsi[3i + m] += Σ_k -(k_i+1) M_k^m b_{k+e_i} and
 // ddpsi[3·s + m] += Σ_k (k_i+1)(k_j+δ_ij+1) M_k^m b_{k+e_i+e_j} for the six
 // pairs s = (00, 01, 02, 11, 12, 22), both without the 1/(4π).
 template <int P, typename R, typename M>
-__device__ __forceinline__ void m2p_accumulate(const R (&bk)[ncoef(P + 2)], const M* mom,
+__device__ __forceinline__ void m2p_accumulate(const R (&bk)[ncoef(P + 2)], const M4<M>* mom,
                                                R (&dpsi)[9], R (&ddpsi)[18]) {
-  constexpr int NC = ncoef(P);
 #pragma unroll
   for (int n = 0; n <= P; ++n)
 #pragma unroll
@@ -92,8 +97,8 @@ __device__ __forceinline__ void m2p_accumulate(const R (&bk)[ncoef(P + 2)], cons
 #pragma unroll
       for (int b = n - a; b >= 0; --b) {
         const int c = n - a - b;
-        const int k = midx(a, b, c);
-        const R m0 = R(mom[k]), m1 = R(mom[NC + k]), m2 = R(mom[2 * NC + k]);
+        const M4<M> mk = mom[midx(a, b, c)];
+        const R m0 = R(mk.x), m1 = R(mk.y), m2 = R(mk.z);
         const R g0 = R(-(a + 1)) * bk[midx(a + 1, b, c)];
         const R g1 = R(-(b + 1)) * bk[midx(a, b + 1, c)];
         const R g2 = R(-(c + 1)) * bk[midx(a, b, c + 1)];
@@ -154,30 +159,39 @@ __device__ __forceinline__ void curl_from_potential(const R (&dp)[9], const R (&
 //   ∂_i ψ_m     = (1/h)  Σ_n n_i L_n^m u^{n-e_i},
 //   ∂_i ∂_j ψ_m = (1/h²) Σ_n n_i (n_j - δ_ij) L_n^m u^{n-e_i-e_j}.
 
-// B̃_j (j! b_j at a unit vector) for |j| <= O into out[j] (shared memory), by
-// the recurrence above (unrolled); each order reads the two before it back
-// from out, which holds O(O³) values, more than the registers of a thread.
+// B̃_j (j! b_j at a unit vector) for |j| <= O into out[j] (shared memory), by the
+// recurrence above, by four neighbouring lanes of a warp (the whole warp calls it):
+// lane part of 0..3 takes every fourth coefficient of an order, which needs only the
+// two orders before it.
 template <int O>
-__device__ __forceinline__ void scaled_taylor_unit(float rx, float ry, float rz, float* out) {
-  out[0] = 1.f;
-#pragma unroll
+__device__ __forceinline__ void scaled_taylor_unit4(float rx, float ry, float rz, int part,
+                                                    float* out) {
+  if (part == 0) out[0] = 1.f;
+  __syncwarp();
+#pragma unroll 1
   for (int n = 1; n <= O; ++n) {
     const float f1 = float(2 * n - 1) / float(n);
     const float f2 = float(n - 1) / float(n);
-#pragma unroll
-    for (int a = n; a >= 0; --a)
-#pragma unroll
-      for (int b = n - a; b >= 0; --b) {
-        const int c = n - a - b;
-        float s1 = 0.f, s2 = 0.f;
-        if (a > 0) s1 += float(a) * rx * out[midx(a - 1, b, c)];
-        if (b > 0) s1 += float(b) * ry * out[midx(a, b - 1, c)];
-        if (c > 0) s1 += float(c) * rz * out[midx(a, b, c - 1)];
-        if (a > 1) s2 += float(a * (a - 1)) * out[midx(a - 2, b, c)];
-        if (b > 1) s2 += float(b * (b - 1)) * out[midx(a, b - 2, c)];
-        if (c > 1) s2 += float(c * (c - 1)) * out[midx(a, b, c - 2)];
-        out[midx(a, b, c)] = f1 * s1 - f2 * s2;
-      }
+    const int t0 = n * (n + 1) * (n + 2) / 6;          // midx of the order's first
+    const int t1 = t0 - n * (n + 1) / 2;                // of the order before
+    const int t2 = t1 - (n - 1) * n / 2;                // of the one before that
+    int m = 0, c = part;                                // i-th: m = b + c, c
+    while (c > m) c -= ++m;
+    for (int i = part; i < (n + 1) * (n + 2) / 2; i += 4) {
+      const int a = n - m, b = m - c;
+      const int tm = m * (m + 1) / 2 + c;               // place of (b, c) within an order
+      float s1 = 0.f, s2 = 0.f;
+      if (a > 0) s1 += float(a) * rx * out[t1 + tm];
+      if (b > 0) s1 += float(b) * ry * out[t1 + tm - m];
+      if (c > 0) s1 += float(c) * rz * out[t1 + tm - m - 1];
+      if (a > 1) s2 += float(a * (a - 1)) * out[t2 + tm];
+      if (b > 1) s2 += float(b * (b - 1)) * out[t2 + tm - 2 * m + 1];
+      if (c > 1) s2 += float(c * (c - 1)) * out[t2 + tm - 2 * m - 1];
+      out[t0 + tm] = f1 * s1 - f2 * s2;
+      c += 4;
+      while (c > m) c -= ++m;
+    }
+    __syncwarp();
   }
 }
 
