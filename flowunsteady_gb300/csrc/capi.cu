@@ -289,8 +289,6 @@ cudaError_t run_pair(const PairCall& pc, int device, int num_sms, const Shape* p
   a.rec = pc.rec;
   a.tma = (pc.rec && !tma_disabled()) ? 1 : 0;
   a.far = farfield_enabled() ? 1 : 0;
-  a.coh = pc.coh;
-  a.coh_blocks = ceil_div(pc.ns, 32);
   a.cluster = cluster;
   a.tile_done = nullptr;
   cudaError_t e = cudaSuccess;
@@ -307,11 +305,6 @@ cudaError_t run_pair(const PairCall& pc, int device, int num_sms, const Shape* p
   }
   return e;
 }
-
-// Below this size the far-field classification neither pays nor costs
-// measurably, and the coherence count (a memset and atomics per pass) is
-// left out: the classification then stays on.
-bool coherence_counted(int64_t n) { return n >= 65536; }
 
 bool tma_disabled() {
   static const bool off = [] {
@@ -621,7 +614,7 @@ static cudaError_t ctx_pair_sorted(vpm_ctx* c, int pass, int kernel, int prec, d
     if (e == cudaSuccess) e = gather_inputs(c, perm, vs, ws);
     if (e == cudaSuccess && recs && uj)
       e = launch_pack_sources(kernel, n, c->srt, c->srt + 3 * ld, c->srt + 6 * ld, ld, scale,
-                              c->rec, nullptr, c->st);
+                              c->rec, c->st);
     else if (e == cudaSuccess && recs)
       e = launch_pack_zeta_sources(kernel, pass == PASS_ZETAD, n, c->srt, c->srt + 3 * ld,
                                    c->srt + 6 * ld, vs ? c->srt + 7 * ld : nullptr,
@@ -640,7 +633,6 @@ static cudaError_t ctx_pair_sorted(vpm_ctx* c, int pass, int kernel, int prec, d
   pc.u = c->sout; pc.j = uj ? c->sout + 3 * ld : nullptr; pc.dj = dj ? c->sout + 12 * ld : nullptr;
   pc.ldo = ld;
   pc.status = c->status;
-  pc.coh = nullptr;
   if (recs) pc.rec = c->rec;
   const Shape* pinned = &c->pinned[pass & 1][kernel][prec];
   pc.chunk = c->pinned_chunk[pass & 1][kernel][prec];
@@ -688,7 +680,6 @@ cudaError_t ctx_pair(vpm_ctx* c, int pass, int kernel, int prec, int64_t t0, int
       wq = ws ? c->srt + 10 * ld : nullptr;
       uo = c->sout; jo = j ? c->sout + 3 * ld : nullptr; djo = dj ? c->sout + 12 * ld : nullptr;
     }
-    unsigned int* coh = !srt && coherence_counted(c->n) ? c->coh : nullptr;
     e = cudaMemsetAsync(bp->d_counter, 0, kMaxBatchGroups * sizeof(unsigned int), c->st);
     if (e != cudaSuccess) return e;
     PairArgs a;
@@ -701,10 +692,8 @@ cudaError_t ctx_pair(vpm_ctx* c, int pass, int kernel, int prec, int64_t t0, int
     a.u = uo; a.j = jo; a.ldo = ld;
     a.part = c->part; a.ldp = ld;
     a.far = farfield_enabled() ? 1 : 0;
-    a.coh = coh;
-    a.coh_blocks = ceil_div(c->n, 32);
     if (prec != VPM_PREC_FP64 && (pass == PASS_UJ || pass == PASS_UJD)) {
-      e = launch_pack_sources(kernel, c->n, xs, gs, ss, ld, scale, c->rec, coh, c->st);
+      e = launch_pack_sources(kernel, c->n, xs, gs, ss, ld, scale, c->rec, c->st);
       if (e != cudaSuccess) return e;
       c->launches += 1;
       a.rec = c->rec;
@@ -747,11 +736,10 @@ cudaError_t ctx_pair(vpm_ctx* c, int pass, int kernel, int prec, int64_t t0, int
   pc.u = u; pc.j = j; pc.ldo = c->ld;
   pc.ws = ws; pc.dj = dj;
   pc.status = c->status;
-  pc.coh = coherence_counted(c->n) ? c->coh : nullptr;
   if (prec != VPM_PREC_FP64 && (pass == PASS_UJ || pass == PASS_UJD)) {
     if (!c->dry) {
       cudaError_t e = launch_pack_sources(kernel, c->n, c->X, c->G, c->S, c->ld, scale, c->rec,
-                                          pc.coh ? c->coh : nullptr, c->st);
+                                          c->st);
       if (e != cudaSuccess) return e;
       c->launches += 1;
     }
@@ -1061,8 +1049,6 @@ int vpm_ctx_create(int device, int64_t capacity, vpm_ctx** out) {
   // Packed source records: 3 float4 per particle for the U/J passes, up to 5 for ζ.
   if (e == cudaSuccess) e = cudaMalloc(&c->rec, 5 * ld * sizeof(float4));
   // Until the first packing the particle order counts as coherent.
-  if (e == cudaSuccess) e = cudaMalloc(&c->coh, sizeof(unsigned int));
-  if (e == cudaSuccess) e = cudaMemset(c->coh, 0xff, sizeof(unsigned int));
   if (e == cudaSuccess) e = cudaMalloc(&c->status, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(c->status, 0, sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&c->red, (size_t(kRedBlocks) + 1) * kDiagSlots * sizeof(double));
@@ -1087,7 +1073,6 @@ int vpm_ctx_destroy(vpm_ctx* c) {
   cudaFree(c->part);
   cudaFree(c->ffv);
   cudaFree(c->rec);
-  cudaFree(c->coh);
   vpm::fmm_free(c->fmm);
   vpm::sort_free(c->sortw);
   cudaFree(c->srt);

@@ -36,7 +36,6 @@ struct PairCall {
   // U/J, launch_pack_zeta_sources for ζ), or null to read the FP64 rows in the
   // kernel.  Bulk copies stage the U/J records.
   const float4* rec = nullptr;
-  const unsigned int* coh = nullptr;   // compact-block count (see PairArgs::coh)
   int* status = nullptr;
 };
 
@@ -189,7 +188,6 @@ struct vpm_ctx {
   double* srt = nullptr;          // Morton-ordered inputs: X3 Γ3 σ1 v3 w3 (13 rows of ld)
   double* sout = nullptr;         // Morton-ordered outputs: U3 J9 DJ9 or ζ sums (21 rows of ld)
   float4* rec = nullptr;          // packed source records, 3 per particle (FP32 U/J passes)
-  unsigned int* coh = nullptr;    // compact 32-particle blocks at the last packing
   double* ffv = nullptr;          // bound particles (X3 Γ3 σ1) and M (6) rows, ffv_cap apart
   int64_t ffv_cap = 0;
   int64_t launches = 0;           // kernels enqueued (graph replays add their kernel count)

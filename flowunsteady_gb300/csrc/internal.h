@@ -68,14 +68,9 @@ struct PairArgs {
   const float4* rec;
   // Stage the records with bulk asynchronous copies (PASS_UJ; needs rec).
   int32_t tma;
-  // Gaussian-erf FP32 passes: classify (warp, 32-source) blocks by their
-  // bounding boxes and take the far-field forms (0 = always the general form).
+  // Gaussian-erf FP32 passes: classify (warp, source) by distance and take the
+  // far-field forms (0 = always the general form).
   int32_t far;
-  // When non-null: the number of compact 32-particle source blocks (counted
-  // by the pack kernel); the classification runs only when at least a quarter
-  // of the coh_blocks blocks are compact (coherent particle order).
-  const unsigned int* coh;
-  int64_t coh_blocks;
   int* status;   // STATUS_TIMEOUT is OR-ed here if a copy wait gives up (may be null)
   // FP32C single-field form only: > 1 when the n_chunk source chunks of a
   // target tile run as one thread-block cluster of `cluster` CTAs (grid =
@@ -97,9 +92,6 @@ bool farfield_enabled();
 // Bulk-copy staging of the packed records is on unless VPM_NO_TMA is set (to
 // non-zero); the kernels then read the records with plain loads.
 bool tma_disabled();
-// Whether the pack kernel counts compact source blocks for a field of n particles.
-bool coherence_counted(int64_t n);
-
 struct Shape {
   int block;   // threads per CTA
   int tpt;     // targets per thread
@@ -125,11 +117,10 @@ bool pair_shape_supported(int precision, Shape shape);
 // when foff is null, else found from the device field table (foff[f] <= i,
 // fchunks[f]); targets whose count is 1 are skipped (already final).
 // Packed source records (3 float4 per source) of n particles for the FP32
-// U/J passes with kernel constants of σ·scale.  Gaussian-erf: *compact (may
-// be null) is reset and then counts the compact 32-particle blocks.
+// U/J passes with kernel constants of σ·scale.
 cudaError_t launch_pack_sources(int kernel, int64_t n, const double* X, const double* G,
                                 const double* S, int64_t ld, double scale, float4* rec,
-                                unsigned int* compact, cudaStream_t st);
+                                cudaStream_t st);
 // Packed source records of the FP32 ζ passes (4 float4 per source, 5 with d
 // for PASS_ZETAD): split positions and ζ constants of σ·scale, Γ, v_q (V rows,
 // zero when null) and w_q (W rows).

@@ -62,6 +62,12 @@ struct PairTraits {
   // copies.
   static constexpr bool kRec = PREC != VPM_PREC_FP64;
   static constexpr bool kTma = PASS == PASS_UJ && PREC != VPM_PREC_FP64;
+  // Targets of a warp: consecutive (32·T of them), so that its box is as small as
+  // the particles' order allows.  Only the FP32 Winckelmans U/J passes keep the T
+  // runs of 32 a block apart: which of their pairs take the masked form, rounded
+  // differently, follows from the boxes.
+  template <int KERNEL>
+  static constexpr bool kWarpRuns = !(kUJ && KERNEL == VPM_KERNEL_WINCKELMANS && PREC != VPM_PREC_FP64);
   // float4 per source record: U/J 3, ζ 4 (+ v_q), ζ + α-derivative 5 (+ w_q).
   static constexpr int kRecQuads = kUJ ? 3 : (PASS == PASS_ZETA ? 4 : 5);
   static constexpr int kRecBytes = 16 * kRecQuads;
@@ -106,6 +112,7 @@ __host__ __device__ constexpr size_t smem_bytes(int block, int tpt) {
 template <int PASS, int PREC, int BLOCK, int T>
 constexpr int min_blocks() {
   constexpr int regs = PASS == PASS_UJD ? (T >= 4 ? 255 : 168) : (T >= 4 ? 168 : 96);
+  if (PASS == PASS_ZETA && PREC == VPM_PREC_FP32C && T >= 4) return 4;   // 128 registers
   return (PairTraits<PASS, PREC>::kUJ && PREC != VPM_PREC_FP64)
              ? (65536 / (BLOCK * regs) > 0 ? 65536 / (BLOCK * regs) : 1)
              : 1;
@@ -197,6 +204,12 @@ __device__ __forceinline__ void finish_f64_sums(double* v) {
   }
 }
 
+// Place within a tile of the k-th target of thread tid.
+template <int T, int BLOCK, bool RUNS>
+__device__ __forceinline__ int tile_target(int k, int tid) {
+  return RUNS ? (tid & ~31) * T + k * 32 + (tid & 31) : k * BLOCK + tid;
+}
+
 // Cluster form of the epilogue (FP32C): after every rank's (hi, lo) pairs are
 // final, rank r forms the values of the targets [r·per, (r+1)·per) of the
 // tile from every rank's pairs, in rank order, as FP64 sums of each rank's
@@ -214,7 +227,9 @@ __device__ __forceinline__ void cluster_epilogue(const PairArgs& a, const float*
   for (int t = int(rank) * per + tid; t < tend; t += BLOCK) {
     const int64_t i = t0 + t;
     if (i >= t1) break;
-    const int k = t / BLOCK, j = t % BLOCK;
+    constexpr bool RUNS = Tr::template kWarpRuns<KERNEL>;
+    const int k = RUNS ? t / 32 % T : t / BLOCK;
+    const int j = RUNS ? t / (32 * T) * 32 + t % 32 : t % BLOCK;
     // Rank q's value w, as the partial-slot epilogue forms it.
     auto rank_value = [&](int w, uint32_t q) {
       const int o = (w * T + k) * BLOCK + j;
@@ -370,11 +385,13 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
   const bool use_tma = Tr::kTma && use_rec && a.tma != 0;
   // The targets are the sources (same rows): their records hold their split.
   const bool tgt_rec = use_rec && a.xt == a.xs && a.ldt == a.lds;
-  // Gaussian-erf FP32 passes classify (warp, 32 sources) blocks by distance.
+  // Gaussian-erf FP32 passes classify every (warp, source) by distance.
   constexpr bool kFarKernel = F32 && KERNEL == VPM_KERNEL_GAUSSIANERF;
-  const bool use_far =
-      kFarKernel && a.far != 0 && (!a.coh || 4 * uint64_t(*a.coh) >= uint64_t(a.coh_blocks));
+  const bool use_far = kFarKernel && a.far != 0;
   const int warp = tid >> 5;
+  constexpr bool RUNS = Tr::template kWarpRuns<KERNEL>;
+  // Source boxes serve the block-wise masks of the passes without RUNS only.
+  constexpr bool kBoxes = F32 && !RUNS;
   uint32_t phase = 0;
   if (use_tma) {
     if (tid == 0) mbar_init(bar, 1);
@@ -458,10 +475,15 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
       }
     }
 
+    // A warp past the last target only stages; a lane past it stands in for the warp's
+    // first target, so that it does not widen the box (its sums are dropped).
+    const int64_t w0 = t0 + (RUNS ? (tid & ~31) * T : 0);
+    const bool live = w0 < t1;
     R tx[T], ty[T], tz[T];
 #pragma unroll
     for (int k = 0; k < T; ++k) {
-      const int64_t i = t0 + k * BLOCK + tid;
+      int64_t i = t0 + tile_target<T, BLOCK, RUNS>(k, tid);
+      if (RUNS && live && i >= t1) i = w0;
       if (i < t1 && tgt_rec) {
         const float4 r0 = a.rec[Tr::kRecQuads * i], r1 = a.rec[Tr::kRecQuads * i + 1];
         tx[k] = R(rel_f32(r0.x, r1.x, chx, clx));
@@ -543,7 +565,7 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
           }
           tileA[tid] = qa;
           tileB[tid] = qb;
-          warp_source_box(qa.x, qa.y, qa.z, qa.w, jj < s1, sbox + 2 * warp);
+          if constexpr (kBoxes) warp_source_box(qa.x, qa.y, qa.z, qa.w, jj < s1, sbox + 2 * warp);
           __syncthreads();  // quads ready, staging records consumed
           if (tid == 0 && tile0 + BLOCK < s1) issue(tile0 + BLOCK, s1);
         }
@@ -612,21 +634,23 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
         tileB[tid] = qb;
         if (Tr::kQuads > 2) tileC[tid] = qc;
         if (PASS == PASS_ZETAD) tileD[tid] = qd;
-        if constexpr (F32) warp_source_box(qa.x, qa.y, qa.z, qa.w, jj < s1, sbox + 2 * warp);
+        if constexpr (kBoxes) warp_source_box(qa.x, qa.y, qa.z, qa.w, jj < s1, sbox + 2 * warp);
         __syncthreads();
       }
 
       // ---- all pairs of the tile ------------------------------------------
       const int cnt = int(min(int64_t(BLOCK), s1 - tile0));
       // FP32: coincident pairs (r² = 0, skipped as the reference's direct sums
-      // skip them) can only occur in 32-source blocks whose box intersects the
-      // warp's target box; only those blocks run the masked pair forms.  The
-      // test is exact in the kernel's own coordinates (comparisons only), so
-      // a target's own particle and any other particle at the same position
-      // are masked wherever they sit.  (FP64 masks every pair.)
+      // skip them) can only occur for sources inside the warp's target box, or in
+      // 32-source blocks whose box intersects it; only those run the masked pair
+      // forms.  The tests are exact in the kernel's own coordinates (comparisons
+      // only), so a target's own particle and any other particle at the same
+      // position are masked wherever they sit.  (FP64 masks every pair.)
       uint32_t ovl = 0;
-      if constexpr (F32) ovl = overlap_blocks<BLOCK / 32>(tbox + 2 * warp, sbox, cnt);
-      if constexpr (Tr::kUJ && F32) {
+      if constexpr (kBoxes) ovl = overlap_blocks<BLOCK / 32>(tbox + 2 * warp, sbox, cnt);
+      if (RUNS && !live) {
+        // nothing to sum
+      } else if constexpr (Tr::kUJ && F32) {
         const float4* ta = reinterpret_cast<const float4*>(tileA);
         const float4* tb = reinterpret_cast<const float4*>(tileB);
         if constexpr (PASS == PASS_UJ) {
@@ -646,18 +670,17 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
           } else {
             // Gaussian-erf masks coincident pairs in its series branch, which
             // every warp holding a pair with ρ² < 3/2 takes.
-            // Gaussian-erf by runs of 32-source blocks of one class: far blocks
-            // skip erfcx/exp, vote blocks decide per source.
-            const uint32_t cls = classify_blocks<BLOCK / 32>(tbox + 2 * warp, sbox, cnt,
-                                                             kVoteSpan * kArgFar, use_far);
-            auto key = [](uint32_t c) { return c >= 2u ? 2u : c; };
+            // Gaussian-erf by runs of sources of one class: far sources skip
+            // erfcx/exp, vote sources decide by their true distances.
+            SourceMasks m;
             for (int js = 0; js < cnt;) {
-              const int je = block_run_end(cls, js, cnt, key);
-              const uint32_t c = key((cls >> (2 * (js >> 5))) & 3u);
-              if (c == 2u) {
+              const int b = js & 31;
+              if (b == 0) m = source_masks(tbox + 2 * warp, ta + js, kVoteSpan * kArgFar, use_far);
+              const int je = min(cnt, js - b + mask_run(m.far, b));
+              if ((m.far >> b) & 1u) {
 #pragma unroll 2
                 for (; js < je; ++js) uj_source_gauss_far<T>(ta[js], tb[js], tx, ty, tz, acc);
-              } else if (c == 1u) {
+              } else if (m.vote) {
 #pragma unroll 2
                 for (; js < je; ++js) uj_source_gauss<T, true>(ta[js], tb[js], tx, ty, tz, acc);
               } else {
@@ -679,18 +702,18 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
             }
           } else {
             // Gaussian-erf: where Dq and Dp vanish only the plain sums take the
-            // pair; far blocks skip erfcx.
-            const uint32_t cls = classify_blocks<BLOCK / 32>(tbox + 2 * warp, sbox, cnt,
-                                                             kVoteSpan * kArgFar, use_far);
-            auto key = [](uint32_t c) { return c; };
+            // pair; far sources skip erfcx.
+            SourceMasks m;
             for (int js = 0; js < cnt;) {
-              const int je = block_run_end(cls, js, cnt, key);
-              const uint32_t c = (cls >> (2 * (js >> 5))) & 3u;
-              if (c == 3u) {
+              const int b = js & 31;
+              if (b == 0) m = source_masks(tbox + 2 * warp, ta + js, kVoteSpan * kArgFar, use_far);
+              // (Zero sources are far too.)
+              const int je = min(cnt, js - b + min(mask_run(m.zero, b), mask_run(m.far, b)));
+              if ((m.zero >> b) & 1u) {
                 for (; js < je; ++js) uj_source_gauss_far<T>(ta[js], tb[js], tx, ty, tz, acc);
-              } else if (c == 2u) {
+              } else if ((m.far >> b) & 1u) {
                 for (; js < je; ++js) ujd_source_gauss_far<T>(ta[js], tb[js], tx, ty, tz, acc);
-              } else if (c == 1u) {
+              } else if (m.vote) {
                 for (; js < je; ++js) ujd_source_gauss<T, true>(ta[js], tb[js], tx, ty, tz, acc);
               } else {
                 for (; js < je; ++js) ujd_source_gauss<T, false>(ta[js], tb[js], tx, ty, tz, acc);
@@ -699,8 +722,8 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
           }
         }
       } else if constexpr (Tr::kUJ) {
-        // FP64 U/J (and DJ).  Warps without a target only stage.
-        if (t0 + (tid & ~31) < t1) {
+        // FP64 U/J (and DJ).
+        {
 #pragma unroll 2
           for (int js = 0; js < cnt; ++js) {
             const Quad<R> sa = tileA[js];
@@ -752,30 +775,22 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
         const float4* tc = reinterpret_cast<const float4*>(tileC);
         const float4* td = reinterpret_cast<const float4*>(PASS == PASS_ZETAD ? tileD : tileC);
         constexpr bool DD = PASS == PASS_ZETAD;
-        // Block codes: 3 skip (Gaussian-erf ζ is exactly zero at every target
-        // of the warp), 2 masked (boxes intersect), 1 per-source votes, 0 the
-        // general form.
-        uint32_t cls = overlap_codes<BLOCK / 32>(ovl, 2u);
-        if (kFarKernel && use_far) {
-          const uint32_t far = classify_blocks<BLOCK / 32>(tbox + 2 * warp, sbox, cnt,
-                                                           kVoteSpan * kArgZero, true);
-#pragma unroll
-          for (int b = 0; b < BLOCK / 32; ++b) {
-            const uint32_t f = (far >> (2 * b)) & 3u;
-            if (f == 3u) cls |= 3u << (2 * b);            // zero blocks cannot coincide
-            else if (f >= 1u && !((ovl >> b) & 1u)) cls |= 1u << (2 * b);
-          }
-        }
+        // Sources whose ζ is exactly zero at every target of the warp (Gaussian-erf)
+        // are skipped; a source inside the target box may coincide with a target
+        // (masked); the others take votes where the targets are compact.
+        SourceMasks m;
         for (int js = 0; js < cnt;) {
-          const int je = block_run_end(cls, js, cnt, [](uint32_t c) { return c; });
-          const uint32_t c = (cls >> (2 * (js >> 5))) & 3u;
-          if (c == 3u) {
+          const int b = js & 31;
+          if (b == 0) m = source_masks(tbox + 2 * warp, ta + js, kVoteSpan * kArgZero, use_far);
+          // (A zero source is never inside.)
+          const int je = min(cnt, js - b + min(mask_run(m.zero, b), mask_run(m.inside, b)));
+          if ((m.zero >> b) & 1u) {
             js = je;
-          } else if (c == 2u) {
+          } else if ((m.inside >> b) & 1u) {
 #pragma unroll 2
             for (; js < je; ++js)
               zeta_source<KERNEL, T, true, DD, false>(ta[js], tb[js], tc[js], td[js], tx, ty, tz, acc);
-          } else if (c == 1u) {
+          } else if (m.vote) {
 #pragma unroll 2
             for (; js < je; ++js)
               zeta_source<KERNEL, T, false, DD, true>(ta[js], tb[js], tc[js], td[js], tx, ty, tz, acc);
@@ -787,7 +802,7 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
         }
       } else {
         // ζ passes, FP64 (Gaussian-erf: the strengths carry ζ(0)/σ³).
-        if (t0 + (tid & ~31) < t1) {
+        {
 #pragma unroll 2
           for (int js = 0; js < cnt; ++js) {
             const Quad<R> sa = tileA[js];
@@ -853,7 +868,7 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
     // A slot is kept in L2 (evict_last) in the fused form until its tile is summed.
 #pragma unroll
     for (int k = 0; k < T; ++k) {
-      const int64_t i = t0 + k * BLOCK + tid;
+      const int64_t i = t0 + tile_target<T, BLOCK, RUNS>(k, tid);
       if (i >= t1) continue;
       if constexpr (F32) {
         if (slot >= 0) {   // the raw float pairs (PairSum)

@@ -1815,7 +1815,7 @@ cudaError_t fmm_eval(vpm_ctx* c, int kernel, int prec, int p, int ncrit, double 
   if ((e = launched(1)) != cudaSuccess) return e;
   if (!f64) {
     e = launch_pack_sources(kernel, n, w->sorted, w->sorted + 3 * ldw, w->sorted + 6 * ldw, ldw,
-                            1.0, w->rec, nullptr, st);
+                            1.0, w->rec, st);
     if ((e = e == cudaSuccess ? launched(1) : e) != cudaSuccess) return e;
   }
 

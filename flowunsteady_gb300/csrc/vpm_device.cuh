@@ -588,13 +588,13 @@ __device__ __forceinline__ void uj_source_gauss(const float4 sa, const float4 sb
 //    far routines compute, without erfcx, exp or the series test.
 //  - arg <= kArgZero: 2^arg is subnormal and ex2.approx.ftz returns +0, so
 //    ζ_σ, Dζ, Dq and Dp are exactly zero in FP32.
-// The classification is made per warp and per 32 staged sources from bounding
-// boxes (warp_target_box, warp_source_box): the box gap g² satisfies
-// g² <= r² for every pair of the two boxes in the same FP32 arithmetic
-// (rounding is monotone), so g²·max(a) >= arg for every pair.  Blocks that do
-// not pass as a whole are classified again per source by warp votes
-// (uj_source_gauss, ujd_source_gauss, zeta_source).  kArgFar and kArgZero are
-// defined above uj_source_gauss.
+// The classification is made per warp and staged source (source_masks): the gap g²
+// between the source and the box of the warp's targets satisfies g² <= r² for every
+// pair in the same FP32 arithmetic (rounding is monotone), so g²·a >= arg for every
+// pair.  Sources that do not pass are classified again by warp votes on the true
+// distances (uj_source_gauss, ujd_source_gauss, zeta_source).  Every form gives the
+// same bits where it applies.  kArgFar and kArgZero are defined above
+// uj_source_gauss.
 // q = 1/r³, p = -3/r⁵ for one source against T targets; acc holds the plain
 // sums first (U 0..2, A 3..10, W 12..14), so the α-derivative layout works too.
 template <int T, int NV>
@@ -674,45 +674,46 @@ __device__ __forceinline__ void warp_source_box(float x, float y, float z, float
   }
 }
 
-// Upper bound of the exponent argument over all pairs of a target box and a
-// source box (both read from shared memory; the result is warp-uniform), and
-// the exponent argument of the target box's own extent (its diagonal at the
-// block's widest core): per-source votes pay only when this is a few times
-// the vote's threshold at most.
-__device__ __forceinline__ float box_arg_bound(const float4* tbox, const float4* sbox,
-                                               float& span) {
-  const float4 tl = tbox[0], th = tbox[1], sl = sbox[0], sh = sbox[1];
-  const float gx = fmaxf(0.f, fmaxf(sl.x - th.x, tl.x - sh.x));
-  const float gy = fmaxf(0.f, fmaxf(sl.y - th.y, tl.y - sh.y));
-  const float gz = fmaxf(0.f, fmaxf(sl.z - th.z, tl.z - sh.z));
-  span = tl.w * sl.w;
-  return fmaf(gx, gx, fmaf(gy, gy, gz * gz)) * sl.w;
-}
-
 // Per-source votes are used where the target box's extent argument is above
 // kVoteSpan times the vote's threshold (both negative).
 constexpr float kVoteSpan = 4.f;
 
-// Classes of the 32-source blocks of a staged tile for one warp, 2 bits per
-// block (NB <= 16 blocks): 3 where every pair has arg <= kArgZero, 2 where
-// every pair has arg <= kArgFar, 1 where per-source votes pay (the target
-// box's extent argument is >= vote_span), 0 otherwise.  0 for every block
-// when the far field is off.
-template <int NB>
-__device__ __forceinline__ uint32_t classify_blocks(const float4* tbox, const float4* sbox,
-                                                    int cnt, float vote_span, bool on) {
-  uint32_t cls = 0;
-  if (!on) return cls;
-#pragma unroll
-  for (int b = 0; b < NB; ++b) {
-    if (b * 32 < cnt) {
-      float span;
-      const float bound = box_arg_bound(tbox, sbox + 2 * b, span);
-      const uint32_t c = bound <= kArgZero ? 3u : bound <= kArgFar ? 2u : (span >= vote_span ? 1u : 0u);
-      cls |= c << (2 * b);
-    }
-  }
-  return cls;
+// Classes of the 32 staged sources at ta[0..31] for one warp, a bit per source: lane j
+// tests source j against the box of the warp's targets (tbox[0..1]).
+//   zero    arg <= kArgZero at every target;     far    arg <= kArgFar at every target;
+//   inside  the source lies in the box, the only place where a target can have the
+//           same position (comparisons only: exact);
+//   vote    (for all of them) votes on the others pay: the exponent argument of the
+//           box's own diagonal is at most kVoteSpan times the vote's threshold
+//           (vote_span, negative) for one of the sources.
+// zero, far and vote are 0 when `on` is false.  About 25 instructions for 32 sources;
+// classifying whole blocks by their own boxes (60 shuffles and minima per warp and
+// staged tile) left most sources of a block that straddles the limit to votes of 8 to
+// 20 instructions each: ζ pass of 50,021 particles 785 -> 670 µs.
+struct SourceMasks {
+  uint32_t zero, far, inside;
+  bool vote;
+};
+__device__ __forceinline__ SourceMasks source_masks(const float4* tbox, const float4* ta,
+                                                    float vote_span, bool on) {
+  const float4 tl = tbox[0], th = tbox[1], q = ta[threadIdx.x & 31];
+  const float gx = fmaxf(0.f, fmaxf(q.x - th.x, tl.x - q.x));
+  const float gy = fmaxf(0.f, fmaxf(q.y - th.y, tl.y - q.y));
+  const float gz = fmaxf(0.f, fmaxf(q.z - th.z, tl.z - q.z));
+  const float g2 = fmaf(gx, gx, fmaf(gy, gy, gz * gz));
+  const float arg = g2 * q.w;
+  SourceMasks m;
+  m.zero = __ballot_sync(0xffffffffu, on && arg <= kArgZero);
+  m.far = __ballot_sync(0xffffffffu, on && arg <= kArgFar);
+  m.vote = __any_sync(0xffffffffu, on && tl.w * q.w >= vote_span);
+  m.inside = __ballot_sync(0xffffffffu, !(g2 > 0.f));
+  return m;
+}
+
+// End (exclusive, at most 32) of the run of equal bits of m that starts at bit js.
+__device__ __forceinline__ int mask_run(uint32_t m, int js) {
+  const uint32_t d = ((m >> js) & 1u) ? ~(m >> js) : m >> js;
+  return d ? js + __ffs(int(d)) - 1 : 32;
 }
 
 // Bit b set where the warp's target box (tbox[0..1]) and staged block b's
