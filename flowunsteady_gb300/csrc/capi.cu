@@ -571,20 +571,31 @@ static cudaError_t sort_scratch(vpm_ctx* c, int nfields) {
   return e;
 }
 
-static cudaError_t gather_inputs(vpm_ctx* c, const int* perm, const double* vs, const double* ws) {
+// The Morton order of a pass (of the fields of a batch, each within its range) and the
+// state and v, w rows gathered into it.  The passes of one stage see the same
+// particles: with share_sort the first one's order and state serve them all (a sort is
+// 12 launches; a dynamic-SFS step of 24 fields made six of them, 0.11 ms each, and now
+// makes three).
+static cudaError_t sorted_inputs(vpm_ctx* c, const BatchPlan* bp, const double* vs, const double* ws) {
   const int64_t n = c->n, ld = c->ld;
-  cudaError_t e = launch_gather_rows(n, 3, perm, c->X, ld, c->srt, ld, c->st);
-  if (e == cudaSuccess) e = launch_gather_rows(n, 3, perm, c->G, ld, c->srt + 3 * ld, ld, c->st);
-  if (e == cudaSuccess) e = launch_gather_rows(n, 1, perm, c->S, ld, c->srt + 6 * ld, ld, c->st);
+  cudaError_t e = cudaSuccess;
+  if (!c->sort_fresh) {
+    e = bp ? sort_order_fields(c->sortw, n, c->X, ld, bp->d_foff, bp->nfields, c->st, &c->sort_perm)
+           : sort_order(c->sortw, n, c->X, ld, c->st, &c->sort_perm);
+    if (e == cudaSuccess) e = launch_gather_rows(n, 7, c->sort_perm, c->X, ld, c->srt, ld, c->st);
+    c->launches += bp ? 3 : 4;   // X 3, Γ 3 and σ 1 are consecutive rows
+    c->sort_fresh = c->share_sort;
+  }
+  const int* perm = c->sort_perm;
   if (e == cudaSuccess && vs) e = launch_gather_rows(n, 3, perm, vs, ld, c->srt + 7 * ld, ld, c->st);
   if (e == cudaSuccess && ws) e = launch_gather_rows(n, 3, perm, ws, ld, c->srt + 10 * ld, ld, c->st);
-  c->launches += 3 + (vs ? 1 : 0) + (ws ? 1 : 0);
+  c->launches += (vs ? 1 : 0) + (ws ? 1 : 0);
   return e;
 }
 
-static cudaError_t scatter_outputs(vpm_ctx* c, int pass, const int* perm, double* u, double* j,
-                                   double* dj) {
+static cudaError_t scatter_outputs(vpm_ctx* c, int pass, double* u, double* j, double* dj) {
   const int64_t n = c->n, ld = c->ld;
+  const int* perm = c->sort_perm;
   if (pass == PASS_UJ || pass == PASS_UJD) {
     cudaError_t e = launch_scatter_rows(n, 3, perm, c->sout, ld, u, ld, c->st);
     if (e == cudaSuccess) e = launch_scatter_rows(n, 9, perm, c->sout + 3 * ld, ld, j, ld, c->st);
@@ -604,14 +615,12 @@ static cudaError_t ctx_pair_sorted(vpm_ctx* c, int pass, int kernel, int prec, d
   const bool uj = pass == PASS_UJ || pass == PASS_UJD;
   const bool recs = prec != VPM_PREC_FP64;   // FP32 passes read packed records
   cudaError_t e = cudaSuccess;
-  const int* perm = nullptr;
   if (c->dry) {
     e = sort_scratch(c, 1);
     if (e != cudaSuccess) return e;
   } else {
     if (!c->sortw || !c->srt || !c->sout) return cudaErrorInvalidValue;
-    e = sort_order(c->sortw, n, c->X, ld, c->st, &perm);
-    if (e == cudaSuccess) e = gather_inputs(c, perm, vs, ws);
+    e = sorted_inputs(c, nullptr, vs, ws);
     if (e == cudaSuccess && recs && uj)
       e = launch_pack_sources(kernel, n, c->srt, c->srt + 3 * ld, c->srt + 6 * ld, ld, scale,
                               c->rec, c->st);
@@ -620,7 +629,7 @@ static cudaError_t ctx_pair_sorted(vpm_ctx* c, int pass, int kernel, int prec, d
                                    c->srt + 6 * ld, vs ? c->srt + 7 * ld : nullptr,
                                    ws ? c->srt + 10 * ld : nullptr, ld, scale, c->rec, c->st);
     if (e != cudaSuccess) return e;
-    c->launches += 3 + (recs ? 1 : 0);
+    c->launches += recs ? 1 : 0;
   }
   PairCall pc;
   pc.pass = pass; pc.kernel = kernel; pc.prec = prec;
@@ -641,7 +650,7 @@ static cudaError_t ctx_pair_sorted(vpm_ctx* c, int pass, int kernel, int prec, d
                c->dry, c->st, &plan);
   if (c->dry || e != cudaSuccess) return e;
   c->launches += plan.launches();
-  return scatter_outputs(c, pass, perm, u, j, dj);
+  return scatter_outputs(c, pass, u, j, dj);
 }
 
 cudaError_t ctx_pair(vpm_ctx* c, int pass, int kernel, int prec, int64_t t0, int64_t t1,
@@ -667,14 +676,11 @@ cudaError_t ctx_pair(vpm_ctx* c, int pass, int kernel, int prec, int64_t t0, int
     const int64_t ld = c->ld;
     const double *xs = c->X, *gs = c->G, *ss = c->S, *vq = vs, *wq = ws;
     double *uo = u, *jo = j, *djo = dj;
-    const int* perm = nullptr;
     cudaError_t e = cudaSuccess;
     if (srt) {
       if (!c->sortw || !c->srt || !c->sout) return cudaErrorInvalidValue;
-      e = sort_order_fields(c->sortw, c->n, c->X, ld, bp->d_foff, bp->nfields, c->st, &perm);
-      if (e == cudaSuccess) e = gather_inputs(c, perm, vs, ws);
+      e = sorted_inputs(c, bp, vs, ws);
       if (e != cudaSuccess) return e;
-      c->launches += 2;
       xs = c->srt; gs = c->srt + 3 * ld; ss = c->srt + 6 * ld;
       vq = vs ? c->srt + 7 * ld : nullptr;
       wq = ws ? c->srt + 10 * ld : nullptr;
@@ -723,7 +729,7 @@ cudaError_t ctx_pair(vpm_ctx* c, int pass, int kernel, int prec, int64_t t0, int
       c->launches += 1;
       if (e != cudaSuccess) return e;
     }
-    return srt ? scatter_outputs(c, pass, perm, u, j, dj) : cudaSuccess;
+    return srt ? scatter_outputs(c, pass, u, j, dj) : cudaSuccess;
   }
   if (sorted_pass(c, t0, t1))
     return ctx_pair_sorted(c, pass, kernel, prec, scale, vs, u, j, ws, dj);
@@ -830,7 +836,7 @@ static cudaError_t zeta_pass(vpm_ctx* c, const vpm_scheme* s, bool d, const doub
 // U/J and the SFS pass of a stage (the first stage of a dynamic step also
 // computes C_d).  In the analytic form the first stage runs the α-derivative
 // passes (U/J + DJ, then ζ + Dζ) instead of separate passes at σ and ασ.
-static cudaError_t enqueue_uj_sfs(vpm_ctx* c, const vpm_scheme* s, int stage) {
+static cudaError_t enqueue_uj_sfs_passes(vpm_ctx* c, const vpm_scheme* s, int stage) {
   const int64_t n = c->n, ld = c->ld;
   int64_t nf = 0;
   const uint8_t* stat = nullptr;
@@ -876,6 +882,14 @@ static cudaError_t enqueue_uj_sfs(vpm_ctx* c, const vpm_scheme* s, int stage) {
                               c->st));
   }
   return cudaSuccess;
+}
+
+static cudaError_t enqueue_uj_sfs(vpm_ctx* c, const vpm_scheme* s, int stage) {
+  c->share_sort = true;
+  c->sort_fresh = false;
+  const cudaError_t e = enqueue_uj_sfs_passes(c, s, stage);
+  c->share_sort = c->sort_fresh = false;
+  return e;
 }
 
 // One stage of a step: U/J, SFS, fused update.

@@ -185,6 +185,10 @@ struct vpm_ctx {
   int order = VPM_ORDER_AUTO;     // vpm_set_particle_order
   vpm::FmmWork* fmm = nullptr;    // treecode workspace (allocated on first use)
   vpm::SortWork* sortw = nullptr; // Morton order of the direct pair passes (large fields)
+  // Sorted passes: within the passes of one stage (share_sort) the Morton order and
+  // the gathered state of the first serve the others (sort_fresh).
+  bool share_sort = false, sort_fresh = false;
+  const int* sort_perm = nullptr;
   double* srt = nullptr;          // Morton-ordered inputs: X3 Γ3 σ1 v3 w3 (13 rows of ld)
   double* sout = nullptr;         // Morton-ordered outputs: U3 J9 DJ9 or ζ sums (21 rows of ld)
   float4* rec = nullptr;          // packed source records, 3 per particle (FP32 U/J passes)

@@ -976,7 +976,13 @@ __global__ void __launch_bounds__(32 * reduce_rows(nval_of(PASS))) reduce_kernel
 #pragma unroll
           for (int l = 0; l < kReduceLoads; ++l) sum.add(a[l]);
         }
-        for (; c < nc; ++c) sum.add(p[int64_t(c) * step]);
+        float2 a[kReduceLoads];   // the rest in flight together too
+#pragma unroll
+        for (int l = 0; l < kReduceLoads; ++l)
+          if (c + l < nc) a[l] = p[int64_t(c + l) * step];
+#pragma unroll
+        for (int l = 0; l < kReduceLoads; ++l)
+          if (c + l < nc) sum.add(a[l]);
         sv[w][tx] = sum.value();
       } else {
         const double* p = part + int64_t(w) * ldp + i;
@@ -988,7 +994,13 @@ __global__ void __launch_bounds__(32 * reduce_rows(nval_of(PASS))) reduce_kernel
 #pragma unroll
           for (int l = 0; l < kReduceLoads; ++l) v += a[l];
         }
-        for (; c < nc; ++c) v += p[int64_t(c) * step];
+        double a[kReduceLoads];
+#pragma unroll
+        for (int l = 0; l < kReduceLoads; ++l)
+          if (c + l < nc) a[l] = p[int64_t(c + l) * step];
+#pragma unroll
+        for (int l = 0; l < kReduceLoads; ++l)
+          if (c + l < nc) v += a[l];
         sv[w][tx] = v;
       }
     }

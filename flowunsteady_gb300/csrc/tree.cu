@@ -2095,40 +2095,49 @@ cudaError_t sort_order(SortWork* s, int64_t n, const double* X, int64_t ld, cuda
 }
 
 // Bounding cube of field f (particles [foff[f], foff[f+1]) or [foff[f], n)),
-// one block per field.
-__global__ void field_box_kernel(int64_t n, const int64_t* __restrict__ foff, int nfields,
-                                 const double* __restrict__ X, int64_t ld, double* fbox) {
-  __shared__ double s[6][256];
+// one block per field.  Minima and maxima on the integer images (order_key): FP64
+// comparisons of 16,384 particles on one SM's FP64 pipe took 44 µs.
+constexpr int kFieldBoxThreads = 1024;
+__global__ void __launch_bounds__(kFieldBoxThreads) field_box_kernel(
+    int64_t n, const int64_t* __restrict__ foff, int nfields, const double* __restrict__ X,
+    int64_t ld, double* fbox) {
+  __shared__ long long s[6][32];
   const int f = blockIdx.x, t = threadIdx.x;
   const int64_t i0 = foff[f], i1 = f + 1 < nfields ? foff[f + 1] : n;
-  double v[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  long long v[6];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    v[d] = order_key(INFINITY);
+    v[3 + d] = order_key(-INFINITY);
+  }
   for (int64_t i = i0 + t; i < i1; i += blockDim.x)
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
       const double x = X[d * ld + i];
-      v[d] = fmin(v[d], x);
-      v[3 + d] = fmax(v[3 + d], x);
+      if (is_nan(x)) continue;
+      const long long k = order_key(x);
+      v[d] = min(v[d], k);
+      v[3 + d] = max(v[3 + d], k);
     }
 #pragma unroll
-  for (int d = 0; d < 6; ++d) s[d][t] = v[d];
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (t < o) {
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        s[d][t] = fmin(s[d][t], s[d][t + o]);
-        s[3 + d][t] = fmax(s[3 + d][t], s[3 + d][t + o]);
-      }
-    }
-    __syncthreads();
+  for (int d = 0; d < 6; ++d) {
+    v[d] = d < 3 ? warp_min_key(v[d]) : warp_max_key(v[d]);
+    if ((t & 31) == 0) s[d][t >> 5] = v[d];
   }
-  if (t == 0) {
-    const double size = fmax(fmax(s[3][0] - s[0][0], s[4][0] - s[1][0]), s[5][0] - s[2][0]);
-    const bool any = i1 > i0;
-    fbox[4 * f + 0] = any ? s[0][0] : 0.0;
-    fbox[4 * f + 1] = any ? s[1][0] : 0.0;
-    fbox[4 * f + 2] = any ? s[2][0] : 0.0;
-    fbox[4 * f + 3] = any && size > 0 ? size * (1.0 + 1e-9) : 1.0;
+  __syncthreads();
+  if (t < 32) {
+    double b[6];
+#pragma unroll
+    for (int d = 0; d < 6; ++d)
+      b[d] = order_value(d < 3 ? warp_min_key(s[d][t]) : warp_max_key(s[d][t]));
+    if (t == 0) {
+      const double size = fmax(fmax(b[3] - b[0], b[4] - b[1]), b[5] - b[2]);
+      const bool any = i1 > i0;
+      fbox[4 * f + 0] = any ? b[0] : 0.0;
+      fbox[4 * f + 1] = any ? b[1] : 0.0;
+      fbox[4 * f + 2] = any ? b[2] : 0.0;
+      fbox[4 * f + 3] = any && size > 0 ? size * (1.0 + 1e-9) : 1.0;
+    }
   }
 }
 
@@ -2162,7 +2171,7 @@ __global__ void morton_fields_kernel(int64_t n, const double* __restrict__ X, in
 cudaError_t sort_order_fields(SortWork* s, int64_t n, const double* X, int64_t ld,
                               const int64_t* foff, int nfields, cudaStream_t st, const int** perm) {
   if (nfields > s->fcap || n > s->cap) return cudaErrorInvalidValue;
-  field_box_kernel<<<nfields, 256, 0, st>>>(n, foff, nfields, X, ld, s->fbox);
+  field_box_kernel<<<nfields, kFieldBoxThreads, 0, st>>>(n, foff, nfields, X, ld, s->fbox);
   morton_fields_kernel<<<int((n + 255) / 256), 256, 0, st>>>(n, X, ld, foff, nfields, s->fbox,
                                                             s->codes, s->idx);
   cudaError_t e = cudaGetLastError();
