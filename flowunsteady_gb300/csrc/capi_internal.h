@@ -26,6 +26,7 @@ struct PairCall {
   int64_t lds;
   const double* xt;
   int64_t ldt;
+  double fd_alpha = 0.0;   // see PairArgs::fd_alpha
   double sigma_scale;
   double *u, *j;
   double* dj = nullptr;         // PASS_UJD: DJ rows
@@ -189,6 +190,7 @@ struct vpm_ctx {
   // the gathered state of the first serve the others (sort_fresh).
   bool share_sort = false, sort_fresh = false;
   const int* sort_perm = nullptr;
+  double fd_alpha = 0.0;          // of the pair passes being enqueued (PairArgs::fd_alpha)
   double* srt = nullptr;          // Morton-ordered inputs: X3 Γ3 σ1 v3 w3 (13 rows of ld)
   double* sout = nullptr;         // Morton-ordered outputs: U3 J9 DJ9 or ζ sums (21 rows of ld)
   float4* rec = nullptr;          // packed source records, 3 per particle (FP32 U/J passes)

@@ -45,6 +45,9 @@ struct PairArgs {
   const double* xt;
   int64_t ldt;
   double sigma_scale;
+  // FP64 Gaussian-erf D passes: 0, or the scale α of the test filter, and the D sums
+  // are then differences (every core scaled by α) - (α = 1) instead of derivatives.
+  double fd_alpha;
   // Decomposition without a table: targets [t_off, t_off+nt) x sources [0, ns).
   int64_t t_off, nt, ns, chunk;
   int32_t n_tb, n_chunk;

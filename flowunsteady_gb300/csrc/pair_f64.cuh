@@ -34,14 +34,15 @@ __device__ __forceinline__ void stage_table(double* dst, const double* src, int 
 // Constants of a source of core σ, staged once per tile.
 //   U/J  Gaussian-erf: a = 1/(2σ²), b = 1/σ³, c = 1/(3σ⁵); with the α-derivative also
 //        ea = -2048 log2(e)/(2σ²), dq = √(2/π)/σ³, dp = √(2/π)/σ⁵ (Dq = -dq e^{-ρ²/2},
-//        Dp = dp e^{-ρ²/2});
+//        Dp = dp e^{-ρ²/2}), or, for differences to the cores ασ (fd = α > 0), the
+//        constants a, b, c of ασ in ea, dq, dp;
 //        Winckelmans: a = σ², b = 3/2 σ², c = 5/2 σ²; ea = -15/2 σ⁴, dq = -35/2 σ⁴
 //        (Dq = ea s^{-7/2}, Dp = dq s^{-9/2}, s = r² + σ²).
-//   ζ    Gaussian-erf: a = -2048 log2(e)/(2σ²), b = ζ(0)/σ³, c = 1/σ²;
+//   ζ    Gaussian-erf: a = -2048 log2(e)/(2σ²), b = ζ(0)/σ³, c = 1/σ², or a of ασ;
 //        Winckelmans: as zeta_consts.
 template <int KERNEL, bool D>
 __device__ __forceinline__ void uj_consts_f64(double sig, double& a, double& b, double& c,
-                                              double& ea, double& dq, double& dp) {
+                                              double& ea, double& dq, double& dp, double fd = 0.0) {
   const double s2 = sig * sig;
   if constexpr (KERNEL == VPM_KERNEL_WINCKELMANS) {
     a = s2;
@@ -56,7 +57,12 @@ __device__ __forceinline__ void uj_consts_f64(double sig, double& a, double& b, 
     a = 0.5 * i2;
     b = i2 * i1;
     c = b * i2 * (1.0 / 3.0);
-    if constexpr (D) {
+    if (D && fd > 0.0) {
+      const double ia = 1.0 / fd, ia2 = ia * ia;
+      ea = a * ia2;
+      dq = b * (ia2 * ia);
+      dp = c * (ia2 * ia2 * ia);
+    } else if constexpr (D) {
       ea = -0.5 * kLog2e * double(kExp2Rows) / s2;
       dq = kSqrt2overPi * b;
       dp = dq * i2;
@@ -64,11 +70,12 @@ __device__ __forceinline__ void uj_consts_f64(double sig, double& a, double& b, 
   }
 }
 template <int KERNEL>
-__device__ __forceinline__ void zeta_consts_f64(double sig, double& a, double& b, double& c) {
+__device__ __forceinline__ void zeta_consts_f64(double sig, double& a, double& b, double& c,
+                                                double fd = 0.0) {
   zeta_consts<KERNEL, double>(sig, a, b);
   if constexpr (KERNEL == VPM_KERNEL_GAUSSIANERF) {
     a *= double(kExp2Rows);
-    c = 1.0 / (sig * sig);
+    c = fd > 0.0 ? a / (fd * fd) : 1.0 / (sig * sig);
   }
 }
 

@@ -193,11 +193,15 @@ __device__ __forceinline__ void finish_f32_sums(double* v) {
 
 // FP64 U/J passes: likewise, Gaussian-erf A sums hold p/(-3).
 template <int PASS, int KERNEL>
-__device__ __forceinline__ void finish_f64_sums(double* v) {
+__device__ __forceinline__ void finish_f64_sums(double* v, bool fd) {
   if constexpr (PASS == PASS_UJ || PASS == PASS_UJD) {
     if constexpr (KERNEL == VPM_KERNEL_GAUSSIANERF) {
 #pragma unroll
       for (int w = 3; w < 11; ++w) v[w] *= -3.0;
+      if (PASS == PASS_UJD && fd) {   // differences of the same sums
+#pragma unroll
+        for (int w = 15; w < 23; ++w) v[w] *= -3.0;
+      }
     }
     v[11] = -(v[3] + v[7]);
     if constexpr (PASS == PASS_UJD) v[23] = -(v[15] + v[19]);
@@ -600,10 +604,11 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
           qb.x = R(a.gs[jj]); qb.y = R(a.gs[a.lds + jj]); qb.z = R(a.gs[2 * a.lds + jj]);
           if constexpr (Tr::kUJ) {
             if constexpr (F32) source_consts<KERNEL, R>(sig, qa.w, qb.w);
-            else uj_consts_f64<KERNEL, PASS == PASS_UJD>(sig, qa.w, qb.w, qc.x, qc.y, qc.z, qc.w);
+            else uj_consts_f64<KERNEL, PASS == PASS_UJD>(sig, qa.w, qb.w, qc.x, qc.y, qc.z, qc.w,
+                                                         a.fd_alpha);
           } else {
             if constexpr (F32) zeta_consts_f32<KERNEL>(sig, qa.w, qb.w, qc.w);
-            else zeta_consts_f64<KERNEL>(sig, qa.w, qb.w, qc.w);
+            else zeta_consts_f64<KERNEL>(sig, qa.w, qb.w, qc.w, a.fd_alpha);
             if (a.vs) {
               qc.x = R(a.vs[jj]); qc.y = R(a.vs[a.lds + jj]); qc.z = R(a.vs[2 * a.lds + jj]);
             }
@@ -722,7 +727,8 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
           }
         }
       } else if constexpr (Tr::kUJ) {
-        // FP64 U/J (and DJ).
+        // FP64 U/J (and DJ, or the difference of J to the cores ασ).
+        const bool fd = PASS == PASS_UJD && KERNEL == VPM_KERNEL_GAUSSIANERF && a.fd_alpha > 0.0;
         {
 #pragma unroll 2
           for (int js = 0; js < cnt; ++js) {
@@ -737,9 +743,20 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
                 const R r2 = fma(dx, dx, fma(dy, dy, dz * dz));
                 uj_f64_gauss(r2, sa.w, sb.w, sc.x, core_tab, q, p);
                 if constexpr (PASS == PASS_UJD) {
-                  const R e = is_zero_f64(r2) ? 0.0 : exp2_f64(r2, sc.y, exp2_tab);
-                  dq = -sc.z * e;
-                  dp = sc.w * e;
+                  if (fd) {
+                    // Beyond both cores the two forms are the same 1/r³ and 1/r⁵.
+                    if (!core_is_near(r2 * sa.w) && !core_is_near(r2 * sc.y)) {
+                      accum_pair_f64(dx, dy, dz, q, p, sb.x, sb.y, sb.z, acc[k]);
+                      continue;
+                    }
+                    uj_f64_gauss(r2, sc.y, sc.z, sc.w, core_tab, dq, dp);
+                    dq -= q;
+                    dp -= p;
+                  } else {
+                    const R e = is_zero_f64(r2) ? 0.0 : exp2_f64(r2, sc.y, exp2_tab);
+                    dq = -sc.z * e;
+                    dp = sc.w * e;
+                  }
                 }
               } else {
                 const bool self = coincident_f64(dx, dy, dz);
@@ -802,6 +819,8 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
         }
       } else {
         // ζ passes, FP64 (Gaussian-erf: the strengths carry ζ(0)/σ³).
+        [[maybe_unused]] const R fd_i3 =
+            PASS == PASS_ZETAD && a.fd_alpha > 0.0 ? 1.0 / (a.fd_alpha * a.fd_alpha * a.fd_alpha) : 0.0;
         {
 #pragma unroll 2
           for (int js = 0; js < cnt; ++js) {
@@ -812,23 +831,32 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
             for (int k = 0; k < T; ++k) {
               const R dx = tx[k] - sa.x, dy = ty[k] - sa.y, dz = tz[k] - sa.z;
               const R r2 = fma(dx, dx, fma(dy, dy, dz * dz));
-              R z, dzz = 0;
+              R z, dzz = 0, zw = 0;   // zw: the ζ that w_q goes with
               if constexpr (KERNEL == VPM_KERNEL_GAUSSIANERF) {
                 z = is_zero_f64(r2) ? 0.0 : exp2_f64(r2, sa.w, exp2_tab);
-                if constexpr (PASS == PASS_ZETAD) dzz = z * fma(r2, sc.w, -3.0);
+                if constexpr (PASS == PASS_ZETAD) {
+                  if (a.fd_alpha > 0.0) {
+                    zw = is_zero_f64(r2) ? 0.0 : exp2_f64(r2, sc.w, exp2_tab) * fd_i3;
+                    dzz = zw - z;
+                  } else {
+                    zw = z;
+                    dzz = z * fma(r2, sc.w, -3.0);
+                  }
+                }
               } else if constexpr (PASS == PASS_ZETA) {
                 z = pair_zeta<KERNEL>(r2, sa.w, sb.w);
               } else {
                 pair_zeta_d<KERNEL>(r2, sa.w, sb.w, z, dzz);
+                zw = z;
               }
               acc[k][0] += z * sb.x; acc[k][1] += z * sb.y; acc[k][2] += z * sb.z;
               acc[k][3] += z * sc.x; acc[k][4] += z * sc.y; acc[k][5] += z * sc.z;
               if constexpr (PASS == PASS_ZETAD) {
                 const Quad<R> sd = tileD[js];
                 acc[k][6] += dzz * sb.x; acc[k][7] += dzz * sb.y; acc[k][8] += dzz * sb.z;
-                acc[k][9] += dzz * sc.x + z * sd.x;
-                acc[k][10] += dzz * sc.y + z * sd.y;
-                acc[k][11] += dzz * sc.z + z * sd.z;
+                acc[k][9] += dzz * sc.x + zw * sd.x;
+                acc[k][10] += dzz * sc.y + zw * sd.y;
+                acc[k][11] += dzz * sc.z + zw * sd.z;
               }
             }
           }
@@ -893,7 +921,7 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
         }
       }
       if constexpr (F32) finish_f32_sums<PASS, KERNEL>(v);
-      else finish_f64_sums<PASS, KERNEL>(v);
+      else finish_f64_sums<PASS, KERNEL>(v, a.fd_alpha > 0.0);
       if (slot >= 0) {
         const uint64_t pol = l2_policy(a.tile_done != nullptr);
 #pragma unroll

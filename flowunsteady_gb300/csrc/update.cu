@@ -72,10 +72,11 @@ __global__ void stretch_vw_kernel(int64_t n, int64_t ld, const double* __restric
 }
 
 // E = S(J, Ω) - V and DE = S(DJ, Ω) + S(J, DΩ) - DV from the raw sums of the
-// α-derivative ζ pass (rows 0..2 Ω, 3..5 V, 6..8 DΩ, 9..11 DV).
+// α-derivative ζ pass (rows 0..2 Ω, 3..5 V, 6..8 DΩ, 9..11 DV).  For differences
+// (fd) S(DJ, DΩ) belongs to DE too.
 __global__ void estr_finish_d_kernel(int64_t n, int64_t ld, const double* __restrict__ raw,
                                      const double* __restrict__ J, const double* __restrict__ DJ,
-                                     int transposed, double* E, double* DE) {
+                                     int transposed, int fd, double* E, double* DE) {
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const double o0 = raw[i], o1 = raw[ld + i], o2 = raw[2 * ld + i];
@@ -84,8 +85,10 @@ __global__ void estr_finish_d_kernel(int64_t n, int64_t ld, const double* __rest
   E[i] = s0 - raw[3 * ld + i];
   E[ld + i] = s1 - raw[4 * ld + i];
   E[2 * ld + i] = s2 - raw[5 * ld + i];
-  stretch_dev(DJ, ld, i, o0, o1, o2, transposed, s0, s1, s2);
-  stretch_dev(J, ld, i, raw[6 * ld + i], raw[7 * ld + i], raw[8 * ld + i], transposed, t0, t1, t2);
+  const double d0 = raw[6 * ld + i], d1 = raw[7 * ld + i], d2 = raw[8 * ld + i];
+  if (fd) stretch_dev(DJ, ld, i, o0 + d0, o1 + d1, o2 + d2, transposed, s0, s1, s2);
+  else stretch_dev(DJ, ld, i, o0, o1, o2, transposed, s0, s1, s2);
+  stretch_dev(J, ld, i, d0, d1, d2, transposed, t0, t1, t2);
   DE[i] = s0 + t0 - raw[9 * ld + i];
   DE[ld + i] = s1 + t1 - raw[10 * ld + i];
   DE[2 * ld + i] = s2 + t2 - raw[11 * ld + i];
@@ -112,8 +115,9 @@ __global__ void __launch_bounds__(256) sfs_dynamic_kernel(
   double a0, a1, a2, b0, b1, b2;
   double nume, deno;
   if (p.analytic) {
-    // Jt = DJ, Et = DE: the test-filter differences are (α-1)·D to first order.
-    const double h = p.alpha - 1.0;
+    // Jt = DJ, Et = DE: the test-filter differences are (α-1)·D to first order, or
+    // (analytic = 2) Jt and Et are the differences.
+    const double h = p.analytic == 2 ? 1.0 : p.alpha - 1.0;
     stretch_dev(Jt, ld, i, g0, g1, g2, p.transposed, a0, a1, a2);
     nume = h * (g0 * a0 + g1 * a1 + g2 * a2);
     deno = h * (g0 * Et[i] + g1 * Et[ld + i] + g2 * Et[2 * ld + i]);
@@ -397,10 +401,10 @@ cudaError_t launch_stretch_vw(int64_t n, int64_t ld, const double* J, const doub
 }
 
 cudaError_t launch_estr_finish_d(int64_t n, int64_t ld, const double* raw, const double* J,
-                                 const double* DJ, int transposed, double* E, double* DE,
+                                 const double* DJ, int transposed, int fd, double* E, double* DE,
                                  cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  estr_finish_d_kernel<<<grid_for(n, 256), 256, 0, st>>>(n, ld, raw, J, DJ, transposed, E, DE);
+  estr_finish_d_kernel<<<grid_for(n, 256), 256, 0, st>>>(n, ld, raw, J, DJ, transposed, fd, E, DE);
   return cudaGetLastError();
 }
 

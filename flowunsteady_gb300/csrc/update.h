@@ -14,7 +14,7 @@ struct SfsParams {
   double inv_zeta0;   // 1/ζ(0) (FP64 divides are scarce on the FP64 pipe)
   int transposed;
   int force_positive;
-  int analytic;   // Jt, Et hold DJ, DE (analytic α-derivatives)
+  int analytic;   // Jt, Et hold 1: DJ, DE (analytic α-derivatives), 2: the differences
 };
 
 struct UpdateParams {
@@ -45,7 +45,7 @@ cudaError_t launch_stretch_vw(int64_t n, int64_t ld, const double* J, const doub
                               const double* G, int transposed, double* V, double* W,
                               cudaStream_t st);
 cudaError_t launch_estr_finish_d(int64_t n, int64_t ld, const double* raw, const double* J,
-                                 const double* DJ, int transposed, double* E, double* DE,
+                                 const double* DJ, int transposed, int fd, double* E, double* DE,
                                  cudaStream_t st);
 // The per-particle kernels below visit particles [0, nv) and skip those whose
 // static flag stat[i] is nonzero (stat may be null: no static particles in range).

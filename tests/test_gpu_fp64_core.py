@@ -62,3 +62,26 @@ def test_bound_forces_at_the_edges_of_chunks(oracle, k, nb, nf):
         c.rc(c.lib.vpm_ffv_direct(c.p, k, nb, L.dptr(Xb), 3, L.dptr(Gb), 3, L.dptr(Sb), 1,
                                   L.dptr(M), 6))
     assert rel_l2(M, M0) <= 1e-12
+
+
+@pytest.mark.parametrize("alpha", [0.999, 0.6, 1.3])
+@pytest.mark.parametrize("n", [1, 127, 129, 700])
+def test_finite_difference_cd_in_one_pass(oracle, alpha, n):
+    # The dynamic C_d of the finite-difference form, whose differences the FP64
+    # Gaussian-erf passes sum directly.  Both sides carry the rounding of q, p and ζ
+    # (a few 2^-53 of each) over the difference, |1 - α| of them: 1e-11/|1 - α|.
+    rng = np.random.default_rng(n)
+    X, G = rng.uniform(-1, 1, (n, 3)), rng.normal(0, 0.1, (n, 3))
+    S = rng.uniform(0.1, 0.3, n)
+    s = scheme(kernel=L.KERNEL_GAUSSIANERF, prec=L.PREC_FP64, sfs=L.SFS_DYNAMIC, alpha=alpha,
+               flags=L.SFS_FORCE_POSITIVE, maxC=0.0)
+    Xo, Go, So, Co, Eo = oracle.step(s, X, G, S, None, 1e-3)
+    with Ctx(n) as c:
+        c.set(X, G, S)
+        c.step(s, 1e-3)
+        Xg, Gg, Sg = c.state()
+        C, E = c.sfs()
+    tol = 1e-11 / abs(1 - alpha)
+    assert rel_l2(C[:, 1:], Co[:, 1:]) <= tol
+    assert rel_l2(Xg, Xo) <= 1e-12 and rel_l2(E, Eo) <= max(tol, 1e-9)
+    assert rel_l2(Gg, Go) <= max(tol, 1e-9)
