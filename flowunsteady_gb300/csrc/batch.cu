@@ -266,10 +266,7 @@ int vpm_batch_get_field(vpm_batch* b, int f, double* X, int64_t sx, double* G, i
   if (f < 0 || f >= b->plan.nfields) return bfail(b, VPM_ERR_INVALID, "no such field");
   const int64_t n = b->plan.h_n[f], o = b->plan.h_off[f];
   vpm_ctx* c = b->ctx;
-  int rc = ctx_download_rows(c, c->X, 3, o, n, X, sx);
-  if (!rc) rc = ctx_download_rows(c, c->G, 3, o, n, G, sg);
-  if (!rc) rc = ctx_download_rows(c, c->S, 1, o, n, S, ss);
-  return from_ctx(b, rc);
+  return from_ctx(b, ctx_download_state(c, o, n, X, sx, G, sg, S, ss));
 }
 
 static int all_set(vpm_batch* b) {

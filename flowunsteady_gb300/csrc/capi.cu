@@ -8,6 +8,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <initializer_list>
 #include <map>
 #include <mutex>
 #include <string>
@@ -417,11 +418,9 @@ int upload(vpm_ctx* c, int64_t i0, int64_t n, const double* X, int64_t sx, const
     h[8 * n + i] = 1.0;
   }
   const size_t w = size_t(n) * sizeof(double), dp = size_t(c->ld) * sizeof(double);
-  CTX_CK(c, cudaMemcpy2DAsync(c->X + i0, dp, h, w, w, 3, cudaMemcpyHostToDevice, c->st));
-  CTX_CK(c, cudaMemcpy2DAsync(c->G + i0, dp, h + 3 * n, w, w, 3, cudaMemcpyHostToDevice, c->st));
-  CTX_CK(c, cudaMemcpyAsync(c->S + i0, h + 6 * n, w, cudaMemcpyHostToDevice, c->st));
-  CTX_CK(c, cudaMemcpyAsync(c->vol + i0, h + 7 * n, w, cudaMemcpyHostToDevice, c->st));
-  CTX_CK(c, cudaMemcpyAsync(c->circ + i0, h + 8 * n, w, cudaMemcpyHostToDevice, c->st));
+  // X 3, Γ 3, σ 1 and vol 1, circulation 1 are consecutive rows.
+  CTX_CK(c, cudaMemcpy2DAsync(c->X + i0, dp, h, w, w, 7, cudaMemcpyHostToDevice, c->st));
+  CTX_CK(c, cudaMemcpy2DAsync(c->vol + i0, dp, h + 7 * n, w, w, 2, cudaMemcpyHostToDevice, c->st));
   CTX_CK(c, cudaMemsetAsync(c->stat + i0, is_static ? 1 : 0, size_t(n), c->st));
   // Fresh particles start with empty SFS memory.
   CTX_CK(c, cudaMemset2DAsync(c->C + i0, dp, 0, w, 3, c->st));
@@ -478,22 +477,53 @@ int validate_host(vpm_ctx* c, int64_t n, const double* X, int64_t sx, const doub
   return VPM_OK;
 }
 
-// Download rows [i0, i0+n) of `rows` consecutive device rows (ld apart) into
-// the host array out[i*stride + k].
-int download_rows(vpm_ctx* c, const double* dev, int rows, int64_t i0, int64_t n, double* out,
-                  int64_t stride) {
-  if (!out || n == 0) return VPM_OK;
-  if (stride < rows) return ctx_fail(c, VPM_ERR_INVALID, "stride too small");
-  int rc = ensure_stage(c, size_t(rows) * n);
+// Host array of `rows` columns, element k of particle i at out[i*stride + k] (null: not
+// wanted).
+struct HostRows {
+  double* out;
+  int rows;
+  int64_t stride;
+};
+
+// Download particles [i0, i0+n) of the consecutive device rows at dev (ld apart) into
+// the host arrays that they make up in turn: one copy and one wait for all of them.
+int download_arrays(vpm_ctx* c, const double* dev, int64_t i0, int64_t n,
+                    std::initializer_list<HostRows> arrays) {
+  if (n == 0) return VPM_OK;
+  int first = -1, end = 0, at = 0;   // the rows wanted
+  for (const HostRows& a : arrays) {
+    if (a.out) {
+      if (a.stride < a.rows) return ctx_fail(c, VPM_ERR_INVALID, "stride too small");
+      if (first < 0) first = at;
+      end = at + a.rows;
+    }
+    at += a.rows;
+  }
+  if (first < 0) return VPM_OK;
+  int rc = ensure_stage(c, size_t(end - first) * n);
   if (rc) return rc;
   const size_t w = size_t(n) * sizeof(double), sp = size_t(c->ld) * sizeof(double);
-  CTX_CK(c, cudaMemcpy2DAsync(c->h_stage, w, dev + i0, sp, w, rows, cudaMemcpyDeviceToHost, c->st));
+  CTX_CK(c, cudaMemcpy2DAsync(c->h_stage, w, dev + int64_t(first) * c->ld + i0, sp, w, end - first,
+                              cudaMemcpyDeviceToHost, c->st));
   CTX_CK(c, cudaStreamSynchronize(c->st));
-  const double* h = c->h_stage;
+  at = 0;
+  for (const HostRows& a : arrays) {
+    const double* h = c->h_stage + (at - first) * n;
+    at += a.rows;
+    if (!a.out) continue;
+    double* out = a.out;
+    const int rows = a.rows;
+    const int64_t stride = a.stride;
 #pragma omp parallel for schedule(static) if (n >= kHostParallelMin)
-  for (int64_t i = 0; i < n; ++i)
-    for (int k = 0; k < rows; ++k) out[i * stride + k] = h[k * n + i];
+    for (int64_t i = 0; i < n; ++i)
+      for (int k = 0; k < rows; ++k) out[i * stride + k] = h[k * n + i];
+  }
   return VPM_OK;
+}
+
+int download_rows(vpm_ctx* c, const double* dev, int rows, int64_t i0, int64_t n, double* out,
+                  int64_t stride) {
+  return download_arrays(c, dev, i0, n, {{out, rows, stride}});
 }
 
 bool valid_kernel(int k) { return k == VPM_KERNEL_WINCKELMANS || k == VPM_KERNEL_GAUSSIANERF; }
@@ -959,9 +989,12 @@ static cudaError_t enqueue_step(vpm_ctx* c, const vpm_scheme* s, double dt, bool
 }
 
 static int check_status(vpm_ctx* c) {
-  int st = 0;
-  CTX_CK(c, cudaMemcpyAsync(&st, c->status, sizeof(int), cudaMemcpyDeviceToHost, c->st));
+  int rc = ensure_stage(c, 1);   // page-locked: the copy does not wait on its own
+  if (rc) return rc;
+  CTX_CK(c, cudaMemcpyAsync(c->h_stage, c->status, sizeof(int), cudaMemcpyDeviceToHost, c->st));
   CTX_CK(c, cudaStreamSynchronize(c->st));
+  int st = 0;
+  std::memcpy(&st, c->h_stage, sizeof(int));
   if (st) {
     CTX_CK(c, cudaMemsetAsync(c->status, 0, sizeof(int), c->st));
     CTX_CK(c, cudaStreamSynchronize(c->st));
@@ -1000,10 +1033,10 @@ int ctx_set_static_flags(vpm_ctx* c, const uint8_t* flags, int64_t n) {
   }
   return VPM_OK;
 }
-int ctx_download_rows(vpm_ctx* c, const double* dev, int rows, int64_t i0, int64_t n, double* out,
-                      int64_t stride) {
+int ctx_download_state(vpm_ctx* c, int64_t i0, int64_t n, double* X, int64_t sx, double* G,
+                       int64_t sg, double* S, int64_t ss) {
   DeviceGuard dg(c->device);
-  return download_rows(c, dev, rows, i0, n, out, stride);
+  return download_arrays(c, c->X, i0, n, {{X, 3, sx}, {G, 3, sg}, {S, 1, ss}});
 }
 // Size the pair-pass scratch for a UJ pass over all particles.
 int ctx_prepare_scratch(vpm_ctx* c, int kernel, int precision) {
@@ -1212,10 +1245,7 @@ int vpm_get_state(vpm_ctx* c, int64_t n, double* X, int64_t sx, double* G, int64
   if (!c) return set_error(nullptr, VPM_ERR_INVALID, "null context");
   if (n < 0 || n > c->n) return ctx_fail(c, VPM_ERR_INVALID, "range beyond particle count");
   DeviceGuard dg(c->device);
-  int rc = download_rows(c, c->X, 3, 0, n, X, sx);
-  if (!rc) rc = download_rows(c, c->G, 3, 0, n, G, sg);
-  if (!rc) rc = download_rows(c, c->S, 1, 0, n, S, ss);
-  return rc;
+  return download_arrays(c, c->X, 0, n, {{X, 3, sx}, {G, 3, sg}, {S, 1, ss}});
 }
 
 int vpm_get_sfs(vpm_ctx* c, int64_t n, double* C, int64_t sc, double* E, int64_t se) {
@@ -1348,9 +1378,7 @@ int vpm_get_UJ(vpm_ctx* c, int64_t i0, int64_t n, double* U, int64_t su, double*
   if (n > 0 && (i0 < c->uj_lo || i0 + n > c->uj_hi))
     return ctx_fail(c, VPM_ERR_STATE, "range not covered by the last U/J evaluation");
   DeviceGuard dg(c->device);
-  int rc = download_rows(c, c->U, 3, i0, n, U, su);
-  if (!rc) rc = download_rows(c, c->J, 9, i0, n, J, sj);
-  return rc;
+  return download_arrays(c, c->U, i0, n, {{U, 3, su}, {J, 9, sj}});
 }
 
 int vpm_eval_sfs(vpm_ctx* c, const vpm_scheme* s) {
@@ -1486,8 +1514,10 @@ int vpm_diagnostics(vpm_ctx* c, int kernel, int precision, double* out) {
   CTX_CK(c, launch_diagnostics(n, nf, stat, c->ld, c->X, c->G, c->S, c->C, c->raw, zeta0_of(kernel),
                                partial, dout, c->st));
   c->launches += 2;
-  double v[kDiagSlots];
-  CTX_CK(c, cudaMemcpyAsync(v, dout, sizeof v, cudaMemcpyDeviceToHost, c->st));
+  if ((rc = ensure_stage(c, kDiagSlots))) return rc;
+  const double* v = c->h_stage;
+  CTX_CK(c, cudaMemcpyAsync(c->h_stage, dout, kDiagSlots * sizeof(double), cudaMemcpyDeviceToHost,
+                            c->st));
   CTX_CK(c, cudaStreamSynchronize(c->st));
   out[VPM_DIAG_ENSTROPHY] = v[DS_ENS];
   out[VPM_DIAG_IMPULSE_X] = v[DS_IX];

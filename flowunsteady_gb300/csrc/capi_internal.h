@@ -228,6 +228,6 @@ int ctx_upload(vpm_ctx* c, int64_t i0, int64_t n, const double* X, int64_t sx, c
 // Static flags of particles [0, n) from a host array (nonzero = static); the
 // particles must already be on the device.
 int ctx_set_static_flags(vpm_ctx* c, const uint8_t* flags, int64_t n);
-int ctx_download_rows(vpm_ctx* c, const double* dev, int rows, int64_t i0, int64_t n, double* out,
-                      int64_t stride);
+int ctx_download_state(vpm_ctx* c, int64_t i0, int64_t n, double* X, int64_t sx, double* G,
+                       int64_t sg, double* S, int64_t ss);
 int ctx_prepare_scratch(vpm_ctx* c, int kernel, int precision);
