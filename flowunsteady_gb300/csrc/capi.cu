@@ -185,6 +185,11 @@ static int plan_cluster(int device, const PairCall& pc, Shape sh, int64_t n_tb,
 constexpr int kSmallWaves = 8;
 constexpr int kLargeWaves = 64;
 constexpr int64_t kLargeField = 131072;
+// Largest field whose reduction takes the particles' updates along: up to about two
+// blocks of 32 particles per SM.  With the updates a block needs 75 to 86 registers a
+// thread and one fits on an SM, where the plain sum has three at a time; a larger
+// field's reduction is bound by reading its partial sums and wants those.
+constexpr int64_t kPostInReduce = 8192;
 
 // Plan and enqueue one pair pass.  `need_part` (elements) is raised to what
 // the launch needs; when dry, nothing is launched.  A split source range goes
@@ -267,6 +272,8 @@ cudaError_t run_pair(const PairCall& pc, int device, int num_sms, const Shape* p
   plan.cluster = cluster;
   const int fmode = fused_reduce_mode();
   plan.fused = plan.slots() > 1 && (fmode == 1 || (fmode < 0 && large && pc.pass == PASS_UJ));
+  plan.post = pc.post && plan.slots() > 1 && !plan.fused && pc.t0 == 0 && nt == pc.ns &&
+              nt <= kPostInReduce;
   const int nv = nval_of(pc.pass);
   const size_t slot_elems = plan.slots() > 1 ? size_t(plan.slots()) * nv * size_t(ldp) : 0;
   // One 32-bit counter per target tile after the slots (two per double).
@@ -303,7 +310,7 @@ cudaError_t run_pair(const PairCall& pc, int device, int num_sms, const Shape* p
   if (e != cudaSuccess) return e;
   if (plan.slots() > 1 && !plan.fused) {
     e = launch_reduce(pc.pass, pc.kernel, pc.prec, part, ldp, nullptr, nullptr, 0, n_chunk, pc.t0, pc.t1,
-                      pc.u, pc.j, pc.dj, pc.ldo, st);
+                      pc.u, pc.j, pc.dj, pc.ldo, plan.post ? pc.post : nullptr, st);
   }
   return e;
 }
@@ -758,7 +765,7 @@ cudaError_t ctx_pair(vpm_ctx* c, int pass, int kernel, int prec, int64_t t0, int
     }
     if (bp->max_chunks > 1) {
       e = launch_reduce(pass, kernel, prec, c->part, ld, bp->d_foff, bp->d_fchunks, bp->nfields, 0,
-                        0, c->n, uo, jo, djo, ld, c->st);
+                        0, c->n, uo, jo, djo, ld, nullptr, c->st);
       c->launches += 1;
       if (e != cudaSuccess) return e;
     }
@@ -776,8 +783,11 @@ cudaError_t ctx_pair(vpm_ctx* c, int pass, int kernel, int prec, int64_t t0, int
   pc.u = u; pc.j = j; pc.ldo = c->ld;
   pc.ws = ws; pc.dj = dj;
   pc.status = c->status;
+  const bool packed = c->rec_pass == pass && c->rec_scale == scale;   // by the update before
+  if (!c->dry) c->rec_pass = -1;
+  pc.post = c->post;
   if (prec != VPM_PREC_FP64 && (pass == PASS_UJ || pass == PASS_UJD)) {
-    if (!c->dry) {
+    if (!c->dry && !packed) {
       cudaError_t e = launch_pack_sources(kernel, c->n, c->X, c->G, c->S, c->ld, scale, c->rec,
                                           c->st);
       if (e != cudaSuccess) return e;
@@ -785,7 +795,7 @@ cudaError_t ctx_pair(vpm_ctx* c, int pass, int kernel, int prec, int64_t t0, int
     }
     pc.rec = c->rec;
   } else if (prec != VPM_PREC_FP64) {
-    if (!c->dry) {
+    if (!c->dry && !packed) {
       cudaError_t e = launch_pack_zeta_sources(kernel, pass == PASS_ZETAD, c->n, c->X, c->G, c->S,
                                                vs, ws, c->ld, scale, c->rec, c->st);
       if (e != cudaSuccess) return e;
@@ -798,7 +808,10 @@ cudaError_t ctx_pair(vpm_ctx* c, int pass, int kernel, int prec, int64_t t0, int
   PairPlan plan;
   cudaError_t e = run_pair(pc, c->device, c->num_sms, pinned, c->part, c->ld, c->part_elems,
                            &c->part_need, c->dry, c->st, &plan);
-  if (!c->dry && e == cudaSuccess && t1 > t0) c->launches += plan.launches();
+  if (!c->dry && e == cudaSuccess && t1 > t0) {
+    c->launches += plan.launches();
+    c->post_taken = plan.post;
+  }
   return e;
 }
 
@@ -867,14 +880,36 @@ static cudaError_t zeta_pass(vpm_ctx* c, const vpm_scheme* s, bool d, const doub
   return ctx_pair(c, PASS_ZETA, s->kernel, s->precision, 0, c->n, 1.0, c->V, c->raw, nullptr);
 }
 
-// U/J and the SFS pass of a stage (the first stage of a dynamic step also
-// computes C_d).  In the analytic form the first stage runs the α-derivative
-// passes (U/J + DJ, then ζ + Dζ) instead of separate passes at σ and ασ.
-static cudaError_t enqueue_uj_sfs_passes(vpm_ctx* c, const vpm_scheme* s, int stage) {
+// A pair pass, then the operations of p on the particles: within the pass's reduction
+// where that takes them, else in a launch of their own.  rec_pass: the pass whose
+// records p packs, or -1.
+template <typename Pass>
+static cudaError_t pass_then(vpm_ctx* c, int kernel, const PostArgs& p, int rec_pass, Pass pass) {
+  c->post = p.flags ? &p : nullptr;
+  c->post_taken = false;
+  const cudaError_t e = pass();
+  c->post = nullptr;
+  if (e != cudaSuccess || c->dry || !p.flags) return e;
+  if (!c->post_taken) {
+    const cudaError_t e2 = launch_post(kernel, p, c->st);
+    if (e2 != cudaSuccess) return e2;
+    c->launches += 1;
+  }
+  if (rec_pass >= 0) {
+    c->rec_pass = rec_pass;
+    c->rec_scale = p.rec_scale;
+  }
+  return cudaSuccess;
+}
+
+// U/J and the SFS passes of a stage (the first stage of a dynamic step also computes
+// C_d), each with the particle operations that follow it; `last` (the update of the
+// stage, or nothing) joins those of the last pass.  In the analytic form the first
+// stage runs the α-derivative passes (U/J + DJ, then ζ + Dζ) instead of separate passes
+// at σ and ασ.
+static cudaError_t enqueue_passes(vpm_ctx* c, const vpm_scheme* s, int stage, int last,
+                                  const UpdateParams& up) {
   const int64_t n = c->n, ld = c->ld;
-  int64_t nf = 0;
-  const uint8_t* stat = nullptr;
-  update_range(c, &nf, &stat);
   const int K = s->kernel, P = s->precision;
   const bool sfs = s->sfs != VPM_SFS_NONE;
   const bool dyn0 = s->sfs == VPM_SFS_DYNAMIC && stage == 0;
@@ -885,60 +920,84 @@ static cudaError_t enqueue_uj_sfs_passes(vpm_ctx* c, const vpm_scheme* s, int st
   // carry the rounding of the two large sums.  Step of two rings of 7,600 particles:
   // 25.3 -> 22.2 ms.
   const bool fd64 = dyn0 && !analytic && P == VPM_PREC_FP64 && K == VPM_KERNEL_GAUSSIANERF;
+  // Packed records belong to the unsorted single-field FP32 passes.
+  const bool recs = P != VPM_PREC_FP64 && !c->bp && !sorted_pass(c, 0, n) &&
+                    s->uj_method != VPM_UJ_TREE;
+  PostArgs base;
+  base.n = n; base.ld = ld; base.transposed = s->transposed;
+  update_range(c, &base.nv, &base.stat);
+  base.X = c->X; base.G = c->G; base.S = c->S; base.C = c->C; base.Q = c->Q; base.V = c->V;
+  base.U = c->U; base.J = base.Js = c->J; base.Jt = c->Jt; base.E = base.Eo = c->E; base.Et = c->Et;
+  base.raw = c->raw;
+  base.cd = s->sfs_Cd;
+  base.up = up;
+  base.rec = c->rec;
+  base.status = c->status;
+  SfsParams& sp = base.sfs;
+  sp.alpha = s->sfs_alpha; sp.rlxf = s->sfs_rlxf; sp.minC = s->sfs_minC; sp.maxC = s->sfs_maxC;
+  sp.zeta0 = zeta0_of(K); sp.inv_zeta0 = 1.0 / sp.zeta0; sp.transposed = s->transposed;
+  sp.force_positive = (s->sfs_flags & VPM_SFS_FORCE_POSITIVE) ? 1 : 0;
+  sp.analytic = fd64 ? 2 : analytic ? 1 : 0;
+  const int uj_rec = recs ? POST_UJ_REC : 0, zeta_rec = recs ? POST_ZETA_REC : 0;
+  const int uj_next = recs ? PASS_UJ : -1;
+  // After the last pass: C_d, the update, and the records of the next stage's U/J.
+  const int tail = (s->sfs == VPM_SFS_CONSTANT ? POST_CONSTANT : 0) | (dyn0 ? POST_DYNAMIC : 0) |
+                   last | (last ? uj_rec : 0);
+  const int tail_rec = last ? uj_next : -1;
   double* W = c->V + 3 * ld;
-  if (fd64) {
-    // Jt := J(ασ) - J(σ), Et := E(ασ) - E(σ).
-    c->fd_alpha = s->sfs_alpha;
-    cudaError_t e = ctx_pair(c, PASS_UJD, K, P, 0, n, 1.0, nullptr, c->U, c->J, nullptr, c->Jt);
-    if (e == cudaSuccess && !c->dry)
-      e = launch_stretch_vw(n, ld, c->J, c->Jt, c->G, s->transposed, c->V, W, c->st);
-    if (e == cudaSuccess) e = ctx_pair(c, PASS_ZETAD, K, P, 0, n, 1.0, c->V, c->raw, nullptr, W, nullptr);
+  if (analytic || fd64) {
+    // Jt := DJ, Et := DE, or the differences J(ασ) - J(σ), E(ασ) - E(σ).
+    PostArgs p = base;
+    p.flags = POST_STRETCH | POST_STRETCH_D | zeta_rec;
+    c->fd_alpha = fd64 ? s->sfs_alpha : 0.0;
+    cudaError_t e = pass_then(c, K, p, recs ? PASS_ZETAD : -1, [&] {
+      return fd64 ? ctx_pair(c, PASS_UJD, K, P, 0, n, 1.0, nullptr, c->U, c->J, nullptr, c->Jt)
+                  : ujd_pass(c, s);
+    });
+    if (e == cudaSuccess) {
+      p = base;
+      p.flags = POST_ESTR | POST_ESTR_D | tail;
+      e = pass_then(c, K, p, tail_rec, [&] {
+        return fd64 ? ctx_pair(c, PASS_ZETAD, K, P, 0, n, 1.0, c->V, c->raw, nullptr, W, nullptr)
+                    : zeta_pass(c, s, true, W);
+      });
+    }
     c->fd_alpha = 0.0;
-    ENQP(c, e);
-    if (!c->dry) c->launches += 1;
-    ENQ(c, launch_estr_finish_d(n, ld, c->raw, c->J, c->Jt, s->transposed, 1, c->E, c->Et, c->st));
-  } else if (analytic) {
-    // Jt := DJ, Et := DE.
-    ENQP(c, ujd_pass(c, s));
-    ENQ(c, launch_stretch_vw(n, ld, c->J, c->Jt, c->G, s->transposed, c->V, W, c->st));
-    ENQP(c, zeta_pass(c, s, true, W));
-    ENQ(c, launch_estr_finish_d(n, ld, c->raw, c->J, c->Jt, s->transposed, 0, c->E, c->Et, c->st));
-  } else {
-    // The finite-difference C_d takes the difference of the passes at σ and at
-    // ασ (amplifying errors by 1/(1-α)): both come from the direct sum.
-    const bool fd = dyn0 && !analytic;
-    ENQP(c, uj_pass(c, s, fd));
-    if (sfs) {
-      ENQ(c, launch_stretch_v(n, ld, c->J, c->G, s->transposed, c->V, c->st));
-      ENQP(c, zeta_pass(c, s, false, nullptr, fd));
-      ENQ(c, launch_estr_finish(n, ld, c->raw, c->J, s->transposed, c->E, c->st));
-    }
+    return e;
   }
-  if (s->sfs == VPM_SFS_CONSTANT) {
-    ENQ(c, launch_sfs_constant(nf, stat, s->sfs_Cd, c->C, c->st));
-  } else if (dyn0) {
-    const double al = s->sfs_alpha;
-    if (!analytic && !fd64) {
-      ENQP(c, ctx_pair(c, PASS_UJ, K, P, 0, n, al, nullptr, c->Ut, c->Jt));
-      ENQ(c, launch_stretch_v(n, ld, c->Jt, c->G, s->transposed, c->V, c->st));
-      ENQP(c, ctx_pair(c, PASS_ZETA, K, P, 0, n, al, c->V, c->raw, nullptr));
-      ENQ(c, launch_estr_finish(n, ld, c->raw, c->Jt, s->transposed, c->Et, c->st));
-    }
-    SfsParams sp;
-    sp.alpha = al; sp.rlxf = s->sfs_rlxf; sp.minC = s->sfs_minC; sp.maxC = s->sfs_maxC;
-    sp.zeta0 = zeta0_of(K); sp.inv_zeta0 = 1.0 / sp.zeta0; sp.transposed = s->transposed;
-    sp.force_positive = (s->sfs_flags & VPM_SFS_FORCE_POSITIVE) ? 1 : 0;
-    sp.analytic = fd64 ? 2 : analytic ? 1 : 0;
-    ENQ(c, launch_sfs_dynamic(nf, stat, ld, c->G, c->S, c->J, c->Jt, c->E, c->Et, c->C, sp,
-                              c->st));
-  }
-  return cudaSuccess;
+  // The finite-difference C_d takes the difference of the passes at σ and at
+  // ασ (amplifying errors by 1/(1-α)): both come from the direct sum.
+  const bool fd = dyn0;
+  PostArgs p = base;
+  p.flags = sfs ? POST_STRETCH | zeta_rec : tail;
+  ENQP(c, pass_then(c, K, p, sfs ? (recs ? PASS_ZETA : -1) : tail_rec,
+                    [&] { return uj_pass(c, s, fd); }));
+  if (!sfs) return cudaSuccess;
+  p = base;
+  p.flags = POST_ESTR | (fd ? uj_rec : tail);
+  if (fd) p.rec_scale = s->sfs_alpha;
+  ENQP(c, pass_then(c, K, p, fd ? uj_next : tail_rec, [&] { return zeta_pass(c, s, false, nullptr, fd); }));
+  if (!fd) return cudaSuccess;
+  const double al = s->sfs_alpha;
+  p = base;
+  p.Js = c->Jt;
+  p.rec_scale = al;
+  p.flags = POST_STRETCH | zeta_rec;
+  ENQP(c, pass_then(c, K, p, recs ? PASS_ZETA : -1,
+                    [&] { return ctx_pair(c, PASS_UJ, K, P, 0, n, al, nullptr, c->Ut, c->Jt); }));
+  p = base;
+  p.Js = c->Jt;
+  p.Eo = c->Et;
+  p.flags = POST_ESTR | tail;
+  return pass_then(c, K, p, tail_rec,
+                   [&] { return ctx_pair(c, PASS_ZETA, K, P, 0, n, al, c->V, c->raw, nullptr); });
 }
 
-static cudaError_t enqueue_uj_sfs(vpm_ctx* c, const vpm_scheme* s, int stage) {
+static cudaError_t enqueue_uj_sfs(vpm_ctx* c, const vpm_scheme* s, int stage, int last = 0,
+                                  const UpdateParams& up = UpdateParams()) {
   c->share_sort = true;
   c->sort_fresh = false;
-  const cudaError_t e = enqueue_uj_sfs_passes(c, s, stage);
+  const cudaError_t e = enqueue_passes(c, s, stage, last, up);
   c->share_sort = c->sort_fresh = false;
   return e;
 }
@@ -946,32 +1005,25 @@ static cudaError_t enqueue_uj_sfs(vpm_ctx* c, const vpm_scheme* s, int stage) {
 // One stage of a step: U/J, SFS, fused update.
 static cudaError_t enqueue_stage(vpm_ctx* c, const vpm_scheme* s, double dt, double a, double b,
                                  int stage) {
-  const int64_t ld = c->ld;
-  int64_t nf = 0;
-  const uint8_t* stat = nullptr;
-  update_range(c, &nf, &stat);
-  const int K = s->kernel;
   const bool sfs = s->sfs != VPM_SFS_NONE;
-  ENQP(c, enqueue_uj_sfs(c, s, stage));
   UpdateParams up;
   up.a = a; up.b = b; up.dt = dt;
   up.uinf0 = s->uinf[0]; up.uinf1 = s->uinf[1]; up.uinf2 = s->uinf[2];
   up.zs = (s->f + s->g) / (1.0 + 3.0 * s->f);
   up.ze = s->f / (1.0 + 3.0 * s->f);
-  up.zeta0 = zeta0_of(K);
+  up.zeta0 = zeta0_of(s->kernel);
   up.inv_zeta0 = 1.0 / up.zeta0;
   up.nu = s->nu;
   up.transposed = s->transposed;
   up.sfs = sfs ? 1 : 0;
   up.clip_backscatter = (sfs && (s->sfs_flags & VPM_SFS_CLIP_BACKSCATTER)) ? 1 : 0;
-  ENQ(c, launch_rk_update(nf, stat, ld, c->X, c->G, c->S, c->U, c->J, c->E, c->C, c->Q, up,
-                          c->status, c->st));
-  return cudaSuccess;
+  return enqueue_uj_sfs(c, s, stage, POST_UPDATE, up);
 }
 
 static cudaError_t enqueue_step(vpm_ctx* c, const vpm_scheme* s, double dt, bool relax) {
   static const double A[3] = {0.0, -5.0 / 9.0, -153.0 / 128.0};
   static const double B[3] = {1.0 / 3.0, 15.0 / 16.0, 8.0 / 15.0};
+  c->rec_pass = -1;   // the particles may have changed since the last step
   if (s->integration == VPM_INTEGRATION_RK3) {
     for (int st = 0; st < 3; ++st) ENQP(c, enqueue_stage(c, s, dt, A[st], B[st], st));
   } else {
@@ -985,6 +1037,7 @@ static cudaError_t enqueue_step(vpm_ctx* c, const vpm_scheme* s, double dt, bool
     update_range(c, &nf, &stat);
     ENQ(c, launch_relax(nf, stat, c->ld, c->J, c->G, s->relax_factor, c->st));
   }
+  c->rec_pass = -1;
   return cudaSuccess;
 }
 
@@ -1397,7 +1450,9 @@ int vpm_eval_sfs(vpm_ctx* c, const vpm_scheme* s) {
   enqueue_uj_sfs(c, s, 0);
   c->dry = false;
   if ((rc = ensure_part(c, c->part_need))) return rc;
+  c->rec_pass = -1;
   CTX_CK(c, enqueue_uj_sfs(c, s, 0));
+  c->rec_pass = -1;
   if (s->sfs_flags & VPM_SFS_CLIP_BACKSCATTER) {
     // A step applies the backscatter clipping inside its update kernel; here
     // it is applied on its own, so C_d comes back as the SFS model leaves it.

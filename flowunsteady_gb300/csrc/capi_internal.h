@@ -37,6 +37,9 @@ struct PairCall {
   // U/J, launch_pack_zeta_sources for ζ), or null to read the FP64 rows in the
   // kernel.  Bulk copies stage the U/J records.
   const float4* rec = nullptr;
+  // Operations on the targets' particles that a reduction launch may take along
+  // (PairPlan::post says whether it did).
+  const PostArgs* post = nullptr;
   int* status = nullptr;
 };
 
@@ -49,6 +52,7 @@ struct PairPlan {
   // The last CTA of each target tile sums its partial slots (no reduction
   // launch); the tiles' counters follow the slots in the scratch.
   bool fused = false;
+  bool post = false;    // the reduction launch takes PairCall::post along
   // Partial slots the plan writes (and a reduction launch, or the fused form, sums).
   int slots() const { return (n_chunk > 1 && cluster <= 1) ? n_chunk : 1; }
   // Kernel launches of the pass: the pair kernel, and the reduction unless fused.
@@ -190,6 +194,12 @@ struct vpm_ctx {
   // the gathered state of the first serve the others (sort_fresh).
   bool share_sort = false, sort_fresh = false;
   const int* sort_perm = nullptr;
+  // Operations that may follow the pass being enqueued within its reduction, whether
+  // they did, and the pass whose packed records are in rec already (-1: none).
+  const vpm::PostArgs* post = nullptr;
+  bool post_taken = false;
+  int rec_pass = -1;
+  double rec_scale = 1.0;
   double fd_alpha = 0.0;          // of the pair passes being enqueued (PairArgs::fd_alpha)
   double* srt = nullptr;          // Morton-ordered inputs: X3 Γ3 σ1 v3 w3 (13 rows of ld)
   double* sout = nullptr;         // Morton-ordered outputs: U3 J9 DJ9 or ζ sums (21 rows of ld)

@@ -95,6 +95,8 @@ bool farfield_enabled();
 // Bulk-copy staging of the packed records is on unless VPM_NO_TMA is set (to
 // non-zero); the kernels then read the records with plain loads.
 bool tma_disabled();
+struct PostArgs;   // update.h
+
 struct Shape {
   int block;   // threads per CTA
   int tpt;     // targets per thread
@@ -134,7 +136,8 @@ cudaError_t launch_pack_zeta_sources(int kernel, bool d, int64_t n, const double
 cudaError_t launch_reduce(int pass, int kernel, int precision, const double* part, int64_t ldp,
                           const int64_t* foff, const int32_t* fchunks, int nfields,
                           int scalar_chunks, int64_t t_begin, int64_t t_end, double* u,
-                          double* j, double* dj, int64_t ldo, cudaStream_t st);
+                          double* j, double* dj, int64_t ldo, const PostArgs* post,
+                          cudaStream_t st);
 
 // The D passes live in pair_d.cu; launch_pair/launch_reduce/pair_ctas_per_sm
 // forward to these for PASS_UJD and PASS_ZETAD.
@@ -143,7 +146,8 @@ cudaError_t launch_pair_d(int pass, int kernel, int precision, Shape shape, cons
 cudaError_t launch_reduce_d(int pass, int kernel, int precision, const double* part, int64_t ldp,
                             const int64_t* foff, const int32_t* fchunks, int nfields,
                             int scalar_chunks, int64_t t_begin, int64_t t_end, double* u,
-                            double* j, double* dj, int64_t ldo, cudaStream_t st);
+                            double* j, double* dj, int64_t ldo, const PostArgs* post,
+                          cudaStream_t st);
 int pair_ctas_per_sm_d(int pass, int kernel, int precision, Shape shape);
 
 }  // namespace vpm

@@ -29,57 +29,21 @@ cudaError_t launch_pair(int pass, int kernel, int precision, Shape s, const Pair
   return launch_pair_d(pass, kernel, precision, s, a, grid, st);
 }
 
-// Packed source records of the FP32 U/J passes, per source
-//   (xh, yh, zh, a), (xl, yl, zl, b), (Γx, Γy, Γz, 0)
-// with x ≈ xh + xl (split_f32) and (a, b) the kernel constants of σ·scale.
 template <int KERNEL>
-__global__ void __launch_bounds__(256) pack_sources_kernel(int64_t n, const double* __restrict__ X,
-                                                           const double* __restrict__ G,
-                                                           const double* __restrict__ S, int64_t ld,
-                                                           double scale, float4* __restrict__ rec) {
+__global__ void __launch_bounds__(kPostThreads) pack_sources_kernel(
+    int64_t n, const double* __restrict__ X, const double* __restrict__ G,
+    const double* __restrict__ S, int64_t ld, double scale, float4* __restrict__ rec) {
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const bool valid = i < n;
-  float xh = 0.f, xl, yh = 0.f, yl, zh = 0.f, zl, ka = -INFINITY, kb;
-  if (valid) {
-    split_f32(X[i], xh, xl);
-    split_f32(X[ld + i], yh, yl);
-    split_f32(X[2 * ld + i], zh, zl);
-    source_consts<KERNEL, float>(S[i] * scale, ka, kb);
-    rec[3 * i] = make_float4(xh, yh, zh, ka);
-    rec[3 * i + 1] = make_float4(xl, yl, zl, kb);
-    rec[3 * i + 2] = make_float4(float(G[i]), float(G[ld + i]), float(G[2 * ld + i]), 0.f);
-  }
+  if (i < n) uj_record_at<KERNEL>(i, ld, X, G, S, scale, rec);
 }
 
-// Packed source records of the FP32 ζ passes, per source
-//   (xh, yh, zh, a), (xl, yl, zl, b), (Γx, Γy, Γz, c), (v_q, 0) [, (w_q, 0)]
-// with (a, b, c) the ζ constants of σ·scale (zeta_consts_f32) and v_q, w_q
-// from the rows V, W (zero when V is null).  Staging these instead of the FP64
-// rows keeps FP64 arithmetic (differences, the constants' divisions, and for
-// Winckelmans a pow) out of the pair kernels, where every CTA would repeat it
-// for every source it stages.
 template <int KERNEL, bool D>
-__global__ void __launch_bounds__(256) pack_zeta_sources_kernel(
+__global__ void __launch_bounds__(kPostThreads) pack_zeta_sources_kernel(
     int64_t n, const double* __restrict__ X, const double* __restrict__ G,
     const double* __restrict__ S, const double* __restrict__ V, const double* __restrict__ W,
     int64_t ld, double scale, float4* __restrict__ rec) {
-  constexpr int Q = D ? 5 : 4;
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float xh, xl, yh, yl, zh, zl, ka, kb, kc;
-  split_f32(X[i], xh, xl);
-  split_f32(X[ld + i], yh, yl);
-  split_f32(X[2 * ld + i], zh, zl);
-  zeta_consts_f32<KERNEL>(S[i] * scale, ka, kb, kc);
-  float4* r = rec + Q * i;
-  r[0] = make_float4(xh, yh, zh, ka);
-  r[1] = make_float4(xl, yl, zl, kb);
-  r[2] = make_float4(float(G[i]), float(G[ld + i]), float(G[2 * ld + i]), kc);
-  r[3] = V ? make_float4(float(V[i]), float(V[ld + i]), float(V[2 * ld + i]), 0.f)
-           : make_float4(0.f, 0.f, 0.f, 0.f);
-  if (D)
-    r[Q - 1] = W ? make_float4(float(W[i]), float(W[ld + i]), float(W[2 * ld + i]), 0.f)
-                 : make_float4(0.f, 0.f, 0.f, 0.f);
+  if (i < n) zeta_record_at<KERNEL>(i, ld, D, X, G, S, V, W, scale, rec);
 }
 
 cudaError_t launch_pack_zeta_sources(int kernel, bool d, int64_t n, const double* X,
@@ -87,8 +51,8 @@ cudaError_t launch_pack_zeta_sources(int kernel, bool d, int64_t n, const double
                                      const double* W, int64_t ld, double scale, float4* rec,
                                      cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  const int grid = int((n + 255) / 256);
-  auto go = [&](auto kern) { kern<<<grid, 256, 0, st>>>(n, X, G, S, V, W, ld, scale, rec); };
+  const int grid = int((n + kPostThreads - 1) / kPostThreads);
+  auto go = [&](auto kern) { kern<<<grid, kPostThreads, 0, st>>>(n, X, G, S, V, W, ld, scale, rec); };
   if (kernel == VPM_KERNEL_WINCKELMANS) {
     if (d) go(pack_zeta_sources_kernel<VPM_KERNEL_WINCKELMANS, true>);
     else go(pack_zeta_sources_kernel<VPM_KERNEL_WINCKELMANS, false>);
@@ -103,26 +67,27 @@ cudaError_t launch_pack_sources(int kernel, int64_t n, const double* X, const do
                                 const double* S, int64_t ld, double scale, float4* rec,
                                 cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
-  const int grid = int((n + 255) / 256);
+  const int grid = int((n + kPostThreads - 1) / kPostThreads);
   if (kernel == VPM_KERNEL_WINCKELMANS)
-    pack_sources_kernel<VPM_KERNEL_WINCKELMANS><<<grid, 256, 0, st>>>(n, X, G, S, ld, scale, rec);
+    pack_sources_kernel<VPM_KERNEL_WINCKELMANS><<<grid, kPostThreads, 0, st>>>(n, X, G, S, ld, scale, rec);
   else
-    pack_sources_kernel<VPM_KERNEL_GAUSSIANERF><<<grid, 256, 0, st>>>(n, X, G, S, ld, scale, rec);
+    pack_sources_kernel<VPM_KERNEL_GAUSSIANERF><<<grid, kPostThreads, 0, st>>>(n, X, G, S, ld, scale, rec);
   return cudaGetLastError();
 }
 
 cudaError_t launch_reduce(int pass, int kernel, int precision, const double* part, int64_t ldp,
                           const int64_t* foff, const int32_t* fchunks, int nfields,
                           int scalar_chunks, int64_t t_begin, int64_t t_end, double* u,
-                          double* j, double* dj, int64_t ldo, cudaStream_t st) {
+                          double* j, double* dj, int64_t ldo, const PostArgs* post,
+                          cudaStream_t st) {
   if (pass == PASS_UJ)
     return reduce<PASS_UJ>(kernel, precision, part, ldp, foff, fchunks, nfields, scalar_chunks, t_begin,
-                           t_end, u, j, dj, ldo, st);
+                           t_end, u, j, dj, ldo, post, st);
   if (pass == PASS_ZETA)
     return reduce<PASS_ZETA>(kernel, precision, part, ldp, foff, fchunks, nfields, scalar_chunks, t_begin,
-                             t_end, u, j, dj, ldo, st);
+                             t_end, u, j, dj, ldo, post, st);
   return launch_reduce_d(pass, kernel, precision, part, ldp, foff, fchunks, nfields, scalar_chunks, t_begin,
-                         t_end, u, j, dj, ldo, st);
+                         t_end, u, j, dj, ldo, post, st);
 }
 
 }  // namespace vpm

@@ -37,6 +37,7 @@
 #include "internal.h"
 #include "pair_f64.cuh"
 #include "update.h"
+#include "update_dev.cuh"
 #include "vpm_device.cuh"
 
 namespace vpm {
@@ -967,11 +968,13 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
 __host__ __device__ constexpr int reduce_rows(int nv) { return nv <= 32 ? nv : (nv + 1) / 2; }
 constexpr int kReduceLoads = 8;
 
-template <int PASS, int KERNEL, bool F2>
+// POST: each target's particle then goes through the operations of `post`
+// (update_dev.cuh), which saves a small field the launches of its updates.
+template <int PASS, int KERNEL, bool F2, bool POST>
 __global__ void __launch_bounds__(32 * reduce_rows(nval_of(PASS))) reduce_kernel(
     const double* __restrict__ part, int64_t ldp, const int64_t* __restrict__ foff,
     const int32_t* __restrict__ fchunks, int nfields, int scalar_chunks, int64_t t_begin,
-    int64_t t_end, PairArgs out) {
+    int64_t t_end, PairArgs out, const PostArgs post) {
   constexpr int NV = nval_of(PASS);
   constexpr int kRows = reduce_rows(NV);
   __shared__ double sv[NV][33];
@@ -1040,6 +1043,7 @@ __global__ void __launch_bounds__(32 * reduce_rows(nval_of(PASS))) reduce_kernel
     for (int w = 0; w < NV; ++w) v[w] = sv[w][tx];
     if constexpr (F2) finish_f32_sums<PASS, KERNEL>(v);
     write_final<PASS, KERNEL>(v, out, i);
+    if constexpr (POST) post_particle<KERNEL>(post, i);
   }
 }
 
@@ -1192,7 +1196,7 @@ template <int PASS>
 cudaError_t reduce(int kernel, int precision, const double* part, int64_t ldp,
                    const int64_t* foff, const int32_t* fchunks, int nfields, int scalar_chunks,
                    int64_t t_begin, int64_t t_end, double* u, double* j, double* dj,
-                   int64_t ldo, cudaStream_t st) {
+                   int64_t ldo, const PostArgs* post, cudaStream_t st) {
   const int64_t n = t_end - t_begin;
   if (n <= 0) return cudaSuccess;
   PairArgs out;
@@ -1203,14 +1207,19 @@ cudaError_t reduce(int kernel, int precision, const double* part, int64_t ldp,
   const bool f2 = precision != VPM_PREC_FP64;   // float-pair slots (PairSum)
   auto go = [&](auto kern) {
     kern<<<grid, bs, 0, st>>>(part, ldp, foff, fchunks, nfields, scalar_chunks, t_begin, t_end,
-                              out);
+                              out, post ? *post : PostArgs());
   };
-  if (kernel == VPM_KERNEL_WINCKELMANS) {
-    if (f2) go(reduce_kernel<PASS, VPM_KERNEL_WINCKELMANS, true>);
-    else go(reduce_kernel<PASS, VPM_KERNEL_WINCKELMANS, false>);
+  constexpr int W = VPM_KERNEL_WINCKELMANS, G = VPM_KERNEL_GAUSSIANERF;
+  if (kernel == W) {
+    if (f2 && post) go(reduce_kernel<PASS, W, true, true>);
+    else if (f2) go(reduce_kernel<PASS, W, true, false>);
+    else if (post) go(reduce_kernel<PASS, W, false, true>);
+    else go(reduce_kernel<PASS, W, false, false>);
   } else {
-    if (f2) go(reduce_kernel<PASS, VPM_KERNEL_GAUSSIANERF, true>);
-    else go(reduce_kernel<PASS, VPM_KERNEL_GAUSSIANERF, false>);
+    if (f2 && post) go(reduce_kernel<PASS, G, true, true>);
+    else if (f2) go(reduce_kernel<PASS, G, true, false>);
+    else if (post) go(reduce_kernel<PASS, G, false, true>);
+    else go(reduce_kernel<PASS, G, false, false>);
   }
   return cudaGetLastError();
 }

@@ -37,30 +37,41 @@ enum {
 };
 constexpr int kRedBlocks = 304;   // 2 x 152 SMs
 
-cudaError_t launch_stretch_v(int64_t n, int64_t ld, const double* J, const double* G,
-                             int transposed, double* V, cudaStream_t st);
-cudaError_t launch_estr_finish(int64_t n, int64_t ld, const double* raw, const double* J,
-                               int transposed, double* E, cudaStream_t st);
-cudaError_t launch_stretch_vw(int64_t n, int64_t ld, const double* J, const double* DJ,
-                              const double* G, int transposed, double* V, double* W,
-                              cudaStream_t st);
-cudaError_t launch_estr_finish_d(int64_t n, int64_t ld, const double* raw, const double* J,
-                                 const double* DJ, int transposed, int fd, double* E, double* DE,
-                                 cudaStream_t st);
+// What happens to the particles between two pair passes (update_dev.cuh), in this
+// order.  Js and Eo: the J that the stretching and E_str take, and where E_str goes
+// (J and E, or at the test-filter level Jt and Et).
+enum : int {
+  POST_STRETCH = 1,      // rows V 0..2 = S(Js, Γ)
+  POST_STRETCH_D = 2,    // rows V 3..5 = S(Jt, Γ)
+  POST_ZETA_REC = 4,     // packed ζ records at rec_scale (with w_q if POST_STRETCH_D)
+  POST_ESTR = 8,         // Eo from raw and Js
+  POST_ESTR_D = 16,      // Et from raw, Js and Jt
+  POST_CONSTANT = 32,    // C_d = cd
+  POST_DYNAMIC = 64,     // C_d from J, Jt, E, Et
+  POST_UPDATE = 128,     // the Runge-Kutta stage
+  POST_UJ_REC = 256      // packed U/J records at rec_scale
+};
+struct PostArgs {
+  int flags = 0, transposed = 0;
+  int64_t n = 0, nv = 0, ld = 0;    // C_d and the update visit [0, nv) where stat is 0
+  const uint8_t* stat = nullptr;
+  double *X = nullptr, *G = nullptr, *S = nullptr, *C = nullptr, *Q = nullptr, *V = nullptr;
+  const double *U = nullptr, *J = nullptr, *Jt = nullptr, *E = nullptr, *raw = nullptr;
+  const double* Js = nullptr;
+  double *Eo = nullptr, *Et = nullptr;
+  double cd = 0.0;
+  SfsParams sfs;
+  UpdateParams up;
+  float4* rec = nullptr;
+  double rec_scale = 1.0;
+  int* status = nullptr;
+};
+constexpr int kPostThreads = 128;
+cudaError_t launch_post(int kernel, const PostArgs& p, cudaStream_t st);
 // The per-particle kernels below visit particles [0, nv) and skip those whose
 // static flag stat[i] is nonzero (stat may be null: no static particles in range).
-cudaError_t launch_sfs_dynamic(int64_t nv, const uint8_t* stat, int64_t ld, const double* G,
-                               const double* S, const double* J, const double* Jt,
-                               const double* E, const double* Et, double* C, const SfsParams& p,
-                               cudaStream_t st);
-cudaError_t launch_sfs_constant(int64_t nv, const uint8_t* stat, double cd, double* C,
-                                cudaStream_t st);
 cudaError_t launch_sfs_clip(int64_t nv, const uint8_t* stat, int64_t ld, const double* G,
                             const double* E, double* C, cudaStream_t st);
-cudaError_t launch_rk_update(int64_t nv, const uint8_t* stat, int64_t ld, double* X, double* G,
-                             double* S, const double* U, const double* J, const double* E,
-                             double* C, double* Q, const UpdateParams& p, int* status,
-                             cudaStream_t st);
 cudaError_t launch_relax(int64_t nv, const uint8_t* stat, int64_t ld, const double* J, double* G,
                          double r, cudaStream_t st);
 cudaError_t launch_zero(double* p, int64_t n, cudaStream_t st);
