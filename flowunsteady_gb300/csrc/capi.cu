@@ -264,6 +264,14 @@ cudaError_t run_pair(const PairCall& pc, int device, int num_sms, const Shape* p
   }
   if (cluster <= 1 && pc.max_chunks > 0 && n_chunk > pc.max_chunks)
     n_chunk = plan_chunks(n_tb, pc.ns, sh.block, resident, &chunk, pc.max_chunks);
+  // The U/J passes of a step of a small field: at one tile of 128 sources an item, 1,200
+  // particles are 50 CTAs, each a chain of 128 sources; items of 16 are 380, and the
+  // step 30 µs shorter.  (Other callers keep whole tiles: a chunk is what the FP32 sums
+  // are folded over, and their results are compared between paths bit for bit.)
+  if (pc.fine && pc.prec == VPM_PREC_FP32C && cluster <= 1 && pc.chunk <= 0 && chunk == sh.block) {
+    while (chunk > 16 && n_tb * ceil_div(pc.ns, chunk) < resident) chunk /= 2;
+    n_chunk = int(ceil_div(pc.ns, chunk));
+  }
   PairPlan plan;
   plan.shape = sh;
   plan.n_tb = n_tb;
@@ -275,6 +283,8 @@ cudaError_t run_pair(const PairCall& pc, int device, int num_sms, const Shape* p
   plan.post = pc.post && plan.slots() > 1 && !plan.fused && pc.t0 == 0 && nt == pc.ns &&
               nt <= kPostInReduce;
   const int nv = nval_of(pc.pass);
+  // Few blocks of targets (less than two a SM) with many slots each.
+  if (plan.slots() >= 32 && nt < 2 * 32 * int64_t(num_sms)) plan.segs = reduce_segs(nv);
   const size_t slot_elems = plan.slots() > 1 ? size_t(plan.slots()) * nv * size_t(ldp) : 0;
   // One 32-bit counter per target tile after the slots (two per double).
   const size_t need = slot_elems + (plan.fused ? size_t((n_tb + 1) / 2) : 0);
@@ -290,7 +300,7 @@ cudaError_t run_pair(const PairCall& pc, int device, int num_sms, const Shape* p
   a.fd_alpha = pc.fd_alpha;
   a.dj = pc.dj;
   a.t_off = pc.t0; a.nt = nt; a.ns = pc.ns; a.chunk = chunk;
-  a.n_tb = int(n_tb); a.n_chunk = n_chunk;
+  a.n_tb = int(n_tb); a.n_chunk = n_chunk; a.segs = plan.segs;
   a.items = nullptr; a.n_items = 0; a.counter = nullptr;
   a.u = pc.u; a.j = pc.j; a.ldo = pc.ldo;
   a.part = part; a.ldp = ldp;
@@ -309,8 +319,8 @@ cudaError_t run_pair(const PairCall& pc, int device, int num_sms, const Shape* p
   e = launch_pair(pc.pass, pc.kernel, pc.prec, sh, a, int(n_tb * n_chunk), st);
   if (e != cudaSuccess) return e;
   if (plan.slots() > 1 && !plan.fused) {
-    e = launch_reduce(pc.pass, pc.kernel, pc.prec, part, ldp, nullptr, nullptr, 0, n_chunk, pc.t0, pc.t1,
-                      pc.u, pc.j, pc.dj, pc.ldo, plan.post ? pc.post : nullptr, st);
+    e = launch_reduce(pc.pass, pc.kernel, pc.prec, part, ldp, nullptr, nullptr, 0, n_chunk,
+                      plan.segs, pc.t0, pc.t1, pc.u, pc.j, pc.dj, pc.ldo, plan.post ? pc.post : nullptr, st);
   }
   return e;
 }
@@ -764,7 +774,7 @@ cudaError_t ctx_pair(vpm_ctx* c, int pass, int kernel, int prec, int64_t t0, int
       c->launches += 1;
     }
     if (bp->max_chunks > 1) {
-      e = launch_reduce(pass, kernel, prec, c->part, ld, bp->d_foff, bp->d_fchunks, bp->nfields, 0,
+      e = launch_reduce(pass, kernel, prec, c->part, ld, bp->d_foff, bp->d_fchunks, bp->nfields, 0, 1,
                         0, c->n, uo, jo, djo, ld, nullptr, c->st);
       c->launches += 1;
       if (e != cudaSuccess) return e;
@@ -786,6 +796,7 @@ cudaError_t ctx_pair(vpm_ctx* c, int pass, int kernel, int prec, int64_t t0, int
   const bool packed = c->rec_pass == pass && c->rec_scale == scale;   // by the update before
   if (!c->dry) c->rec_pass = -1;
   pc.post = c->post;
+  pc.fine = c->fine;
   if (prec != VPM_PREC_FP64 && (pass == PASS_UJ || pass == PASS_UJD)) {
     if (!c->dry && !packed) {
       cudaError_t e = launch_pack_sources(kernel, c->n, c->X, c->G, c->S, c->ld, scale, c->rec,
@@ -970,8 +981,11 @@ static cudaError_t enqueue_passes(vpm_ctx* c, const vpm_scheme* s, int stage, in
   const bool fd = dyn0;
   PostArgs p = base;
   p.flags = sfs ? POST_STRETCH | zeta_rec : tail;
-  ENQP(c, pass_then(c, K, p, sfs ? (recs ? PASS_ZETA : -1) : tail_rec,
-                    [&] { return uj_pass(c, s, fd); }));
+  c->fine = !sfs;   // (finite-difference C_d would amplify another rounding)
+  const cudaError_t e = pass_then(c, K, p, sfs ? (recs ? PASS_ZETA : -1) : tail_rec,
+                                  [&] { return uj_pass(c, s, fd); });
+  c->fine = false;
+  ENQP(c, e);
   if (!sfs) return cudaSuccess;
   p = base;
   p.flags = POST_ESTR | (fd ? uj_rec : tail);

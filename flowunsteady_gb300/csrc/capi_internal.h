@@ -33,6 +33,7 @@ struct PairCall {
   int64_t ldo;
   int max_chunks = 0;   // upper bound on source chunks (0 = planner's choice)
   int64_t chunk = 0;    // pinned source chunk length (0 = planner's choice)
+  bool fine = false;    // chunks below a tile where the field leaves the GPU idle
   // FP32 passes: packed records of the ns sources (launch_pack_sources for
   // U/J, launch_pack_zeta_sources for ζ), or null to read the FP64 rows in the
   // kernel.  Bulk copies stage the U/J records.
@@ -52,6 +53,7 @@ struct PairPlan {
   // The last CTA of each target tile sums its partial slots (no reduction
   // launch); the tiles' counters follow the slots in the scratch.
   bool fused = false;
+  int segs = 1;         // runs that the slots of a target are summed in
   bool post = false;    // the reduction launch takes PairCall::post along
   // Partial slots the plan writes (and a reduction launch, or the fused form, sums).
   int slots() const { return (n_chunk > 1 && cluster <= 1) ? n_chunk : 1; }
@@ -198,6 +200,7 @@ struct vpm_ctx {
   // they did, and the pass whose packed records are in rec already (-1: none).
   const vpm::PostArgs* post = nullptr;
   bool post_taken = false;
+  bool fine = false;              // PairCall::fine of the pass being enqueued
   int rec_pass = -1;
   double rec_scale = 1.0;
   double fd_alpha = 0.0;          // of the pair passes being enqueued (PairArgs::fd_alpha)

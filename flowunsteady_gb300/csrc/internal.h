@@ -24,6 +24,9 @@ __host__ __device__ constexpr int nval_of(int pass) {
                             : kNvalZetaD;
 }
 
+// Runs of slots that a pass of nv values may be summed in (see reduce_kernel).
+__host__ __device__ constexpr int reduce_segs(int nv) { return nv <= 15 ? 4 : 2; }
+
 // One work item: targets [t0, t1) against sources [s0, s1).  slot < 0 means the
 // item covers all sources of its targets and writes final values; otherwise it
 // writes raw sums into partial slot `slot`.
@@ -51,6 +54,7 @@ struct PairArgs {
   // Decomposition without a table: targets [t_off, t_off+nt) x sources [0, ns).
   int64_t t_off, nt, ns, chunk;
   int32_t n_tb, n_chunk;
+  int32_t segs;   // runs that the slots of a target are summed in
   // Decomposition from a table (batches): n_items entries, dynamic queue when
   // counter != null.
   const PairItem* items;
@@ -135,7 +139,7 @@ cudaError_t launch_pack_zeta_sources(int kernel, bool d, int64_t n, const double
                                      cudaStream_t st);
 cudaError_t launch_reduce(int pass, int kernel, int precision, const double* part, int64_t ldp,
                           const int64_t* foff, const int32_t* fchunks, int nfields,
-                          int scalar_chunks, int64_t t_begin, int64_t t_end, double* u,
+                          int scalar_chunks, int segs, int64_t t_begin, int64_t t_end, double* u,
                           double* j, double* dj, int64_t ldo, const PostArgs* post,
                           cudaStream_t st);
 
@@ -145,7 +149,7 @@ cudaError_t launch_pair_d(int pass, int kernel, int precision, Shape shape, cons
                           int grid, cudaStream_t st);
 cudaError_t launch_reduce_d(int pass, int kernel, int precision, const double* part, int64_t ldp,
                             const int64_t* foff, const int32_t* fchunks, int nfields,
-                            int scalar_chunks, int64_t t_begin, int64_t t_end, double* u,
+                            int scalar_chunks, int segs, int64_t t_begin, int64_t t_end, double* u,
                             double* j, double* dj, int64_t ldo, const PostArgs* post,
                           cudaStream_t st);
 int pair_ctas_per_sm_d(int pass, int kernel, int precision, Shape shape);

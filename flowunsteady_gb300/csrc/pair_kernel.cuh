@@ -178,6 +178,12 @@ struct PairSum {
   __device__ __forceinline__ double value() const { return double(s) + double(c); }
 };
 
+// The slots of a target are summed in PairArgs::segs runs of consecutive slots, each in
+// slot order, and the runs in order; every form of the sum takes the same runs.
+__host__ __device__ inline int seg_begin(int nc, int seg, int segs) {
+  return int(int64_t(nc) * seg / segs);
+}
+
 // FP32 U/J passes: the Gaussian-erf A sums carry a scale, and A22 (DA22) is not
 // accumulated (the pairs are trace-free); both are applied to the FP64 sums.
 template <int PASS, int KERNEL>
@@ -294,33 +300,34 @@ __device__ __noinline__ void tile_reduce(const PairArgs& a, int64_t t0, int64_t 
     double v[NV];
 #pragma unroll
     for (int w0 = 0; w0 < NV; w0 += G) {
-      if constexpr (F2) {
-        PairSum s[G];
-        const float2* p = reinterpret_cast<const float2*>(a.part) + int64_t(w0) * a.ldp + i;
+      using Sum = typename std::conditional<F2, PairSum, double>::type;
+      Sum all[G] = {};
+      for (int seg = 0; seg < a.segs; ++seg) {
+        Sum s[G] = {};
+        const int c1 = seg_begin(a.n_chunk, seg + 1, a.segs);
+        int c = seg_begin(a.n_chunk, seg, a.segs);
+        const double* p = a.part + int64_t(w0) * a.ldp + i + int64_t(c) * step;
 #pragma unroll 2
-        for (int c = 0; c < a.n_chunk; ++c, p += step) {
+        for (; c < c1; ++c, p += step) {
 #pragma unroll
-          for (int g = 0; g < G; ++g)
-            if (w0 + g < NV) s[g].add(__ldcg(p + int64_t(g) * a.ldp));
+          for (int g = 0; g < G; ++g) {
+            if (w0 + g >= NV) continue;
+            if constexpr (F2) s[g].add(__ldcg(reinterpret_cast<const float2*>(p + int64_t(g) * a.ldp)));
+            else s[g] += __ldcg(p + int64_t(g) * a.ldp);
+          }
         }
 #pragma unroll
-        for (int g = 0; g < G; ++g)
-          if (w0 + g < NV) v[w0 + g] = s[g].value();
-      } else {
-        double s[G];
-#pragma unroll
-        for (int g = 0; g < G; ++g) s[g] = 0.0;
-        const double* p = a.part + int64_t(w0) * a.ldp + i;
-#pragma unroll 2
-        for (int c = 0; c < a.n_chunk; ++c, p += step) {
-#pragma unroll
-          for (int g = 0; g < G; ++g)
-            if (w0 + g < NV) s[g] += __ldcg(p + int64_t(g) * a.ldp);
+        for (int g = 0; g < G; ++g) {
+          if constexpr (F2) all[g].add(make_float2(s[g].s, s[g].c));
+          else all[g] += s[g];
         }
-#pragma unroll
-        for (int g = 0; g < G; ++g)
-          if (w0 + g < NV) v[w0 + g] = s[g];
       }
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+        if (w0 + g < NV) {
+          if constexpr (F2) v[w0 + g] = all[g].value();
+          else v[w0 + g] = all[g];
+        }
     }
     if constexpr (F2) finish_f32_sums<PASS, KERNEL>(v);
     write_final<PASS, KERNEL>(v, a, i);
@@ -958,28 +965,30 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
   }
 }
 
-// Fixed-order sum of the partial slots.  A block holds 32 targets (x) and
-// reduce_rows(NV) value rows (y): thread (x, y) sums rows y, y + rows, ... of
-// its target over the chunks in chunk order, loading kReduceLoads chunks ahead
-// (the same additions in the same order as one thread per target walking every
-// row, so the result is bitwise that one), and one warp then forms the final
-// values from shared memory.  F2: the FP32 passes' float-pair slots, summed
-// with PairSum; otherwise FP64 slots and FP64 additions.
-__host__ __device__ constexpr int reduce_rows(int nv) { return nv <= 32 ? nv : (nv + 1) / 2; }
-constexpr int kReduceLoads = 8;
-
+// Fixed-order sum of the partial slots.  A block holds COLS targets (x) times the NV
+// values (y) times SEGS runs of slots (z): thread (x, y, z) sums its run in slot order,
+// kReduceLoads slots loaded ahead, and one thread per target adds the runs in order and
+// forms the final values from shared memory.  F2: the FP32 passes' float-pair slots,
+// summed with PairSum; otherwise FP64 slots and FP64 additions.  tile_reduce adds in
+// the same order.
+//   SEGS 1, COLS 32: a field of many blocks, bound by reading the slots.
+//   SEGS 4, COLS 16 (reduce_segs): few targets with many slots each, where one thread
+//   per value would walk them alone.
 // POST: each target's particle then goes through the operations of `post`
 // (update_dev.cuh), which saves a small field the launches of its updates.
-template <int PASS, int KERNEL, bool F2, bool POST>
-__global__ void __launch_bounds__(32 * reduce_rows(nval_of(PASS))) reduce_kernel(
-    const double* __restrict__ part, int64_t ldp, const int64_t* __restrict__ foff,
-    const int32_t* __restrict__ fchunks, int nfields, int scalar_chunks, int64_t t_begin,
-    int64_t t_end, PairArgs out, const PostArgs post) {
-  constexpr int NV = nval_of(PASS);
-  constexpr int kRows = reduce_rows(NV);
-  __shared__ double sv[NV][33];
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int64_t i = t_begin + int64_t(blockIdx.x) * 32 + tx;
+constexpr int kReduceLoads = 8;
+constexpr int reduce_threads(int nv, int segs) { return (segs == 1 ? 32 : 16) * nv * segs; }
+
+template <int PASS, int KERNEL, bool F2, bool POST, int SEGS>
+__global__ void __launch_bounds__(reduce_threads(nval_of(PASS), SEGS),
+                                  POST ? 1 : 1536 / reduce_threads(nval_of(PASS), SEGS))
+    reduce_kernel(const double* __restrict__ part, int64_t ldp, const int64_t* __restrict__ foff,
+                  const int32_t* __restrict__ fchunks, int nfields, int scalar_chunks,
+                  int64_t t_begin, int64_t t_end, PairArgs out, const PostArgs post) {
+  constexpr int NV = nval_of(PASS), COLS = SEGS == 1 ? 32 : 16;
+  __shared__ double sv[SEGS][NV][COLS + 1];
+  const int tx = threadIdx.x, w = threadIdx.y, seg = threadIdx.z;
+  const int64_t i = t_begin + int64_t(blockIdx.x) * COLS + tx;
   int nc = 0;
   if (i < t_end) {
     nc = scalar_chunks;
@@ -994,53 +1003,48 @@ __global__ void __launch_bounds__(32 * reduce_rows(nval_of(PASS))) reduce_kernel
   }
   const bool live = nc > 1;
   if (live) {
+    using T = typename std::conditional<F2, float2, double>::type;
+    typename std::conditional<F2, PairSum, double>::type sum{};
+    auto add = [&](T x) {
+      if constexpr (F2) sum.add(x);
+      else sum += x;
+    };
     const int64_t step = int64_t(NV) * ldp;
-    for (int w = ty; w < NV; w += kRows) {
-      int c = 0;
-      if constexpr (F2) {
-        const float2* p = reinterpret_cast<const float2*>(part) + int64_t(w) * ldp + i;
-        PairSum sum;
-        for (; c + kReduceLoads <= nc; c += kReduceLoads) {
-          float2 a[kReduceLoads];
+    const T* p = reinterpret_cast<const T*>(part) + int64_t(w) * ldp + i;
+    int c = seg_begin(nc, seg, SEGS);
+    const int c1 = seg_begin(nc, seg + 1, SEGS);
+    T a[kReduceLoads];
+    for (; c + kReduceLoads <= c1; c += kReduceLoads) {
 #pragma unroll
-          for (int l = 0; l < kReduceLoads; ++l) a[l] = p[int64_t(c + l) * step];
+      for (int l = 0; l < kReduceLoads; ++l) a[l] = p[int64_t(c + l) * step];
 #pragma unroll
-          for (int l = 0; l < kReduceLoads; ++l) sum.add(a[l]);
-        }
-        float2 a[kReduceLoads];   // the rest in flight together too
-#pragma unroll
-        for (int l = 0; l < kReduceLoads; ++l)
-          if (c + l < nc) a[l] = p[int64_t(c + l) * step];
-#pragma unroll
-        for (int l = 0; l < kReduceLoads; ++l)
-          if (c + l < nc) sum.add(a[l]);
-        sv[w][tx] = sum.value();
-      } else {
-        const double* p = part + int64_t(w) * ldp + i;
-        double v = 0.0;
-        for (; c + kReduceLoads <= nc; c += kReduceLoads) {
-          double a[kReduceLoads];
-#pragma unroll
-          for (int l = 0; l < kReduceLoads; ++l) a[l] = p[int64_t(c + l) * step];
-#pragma unroll
-          for (int l = 0; l < kReduceLoads; ++l) v += a[l];
-        }
-        double a[kReduceLoads];
-#pragma unroll
-        for (int l = 0; l < kReduceLoads; ++l)
-          if (c + l < nc) a[l] = p[int64_t(c + l) * step];
-#pragma unroll
-        for (int l = 0; l < kReduceLoads; ++l)
-          if (c + l < nc) v += a[l];
-        sv[w][tx] = v;
-      }
+      for (int l = 0; l < kReduceLoads; ++l) add(a[l]);
     }
+#pragma unroll
+    for (int l = 0; l < kReduceLoads; ++l)   // the rest in flight together too
+      if (c + l < c1) a[l] = p[int64_t(c + l) * step];
+#pragma unroll
+    for (int l = 0; l < kReduceLoads; ++l)
+      if (c + l < c1) add(a[l]);
+    if constexpr (F2) reinterpret_cast<float2&>(sv[seg][w][tx]) = make_float2(sum.s, sum.c);
+    else sv[seg][w][tx] = sum;
   }
   __syncthreads();
-  if (ty == 0 && live) {
+  if (w == 0 && seg == 0 && live) {
     double v[NV];
 #pragma unroll
-    for (int w = 0; w < NV; ++w) v[w] = sv[w][tx];
+    for (int k = 0; k < NV; ++k) {
+      if constexpr (F2) {
+        PairSum sum;
+#pragma unroll
+        for (int z = 0; z < SEGS; ++z) sum.add(reinterpret_cast<const float2&>(sv[z][k][tx]));
+        v[k] = sum.value();
+      } else {
+        v[k] = sv[0][k][tx];
+#pragma unroll
+        for (int z = 1; z < SEGS; ++z) v[k] += sv[z][k][tx];
+      }
+    }
     if constexpr (F2) finish_f32_sums<PASS, KERNEL>(v);
     write_final<PASS, KERNEL>(v, out, i);
     if constexpr (POST) post_particle<KERNEL>(post, i);
@@ -1192,34 +1196,41 @@ int max_active_clusters(int kernel, int precision, Shape s, int cluster) {
   return n;
 }
 
+template <int PASS, int KERNEL, bool F2, int SEGS>
+void start_reduce(const double* part, int64_t ldp, const int64_t* foff, const int32_t* fchunks,
+                  int nfields, int scalar_chunks, int64_t t_begin, int64_t t_end,
+                  const PairArgs& out, const PostArgs* post, cudaStream_t st) {
+  constexpr int COLS = SEGS == 1 ? 32 : 16;
+  const dim3 bs(COLS, nval_of(PASS), SEGS);
+  const int grid = int((t_end - t_begin + COLS - 1) / COLS);
+  if (post)
+    reduce_kernel<PASS, KERNEL, F2, true, SEGS><<<grid, bs, 0, st>>>(
+        part, ldp, foff, fchunks, nfields, scalar_chunks, t_begin, t_end, out, *post);
+  else
+    reduce_kernel<PASS, KERNEL, F2, false, SEGS><<<grid, bs, 0, st>>>(
+        part, ldp, foff, fchunks, nfields, scalar_chunks, t_begin, t_end, out, PostArgs());
+}
+
 template <int PASS>
 cudaError_t reduce(int kernel, int precision, const double* part, int64_t ldp,
                    const int64_t* foff, const int32_t* fchunks, int nfields, int scalar_chunks,
-                   int64_t t_begin, int64_t t_end, double* u, double* j, double* dj,
+                   int segs, int64_t t_begin, int64_t t_end, double* u, double* j, double* dj,
                    int64_t ldo, const PostArgs* post, cudaStream_t st) {
-  const int64_t n = t_end - t_begin;
-  if (n <= 0) return cudaSuccess;
+  if (t_end <= t_begin) return cudaSuccess;
   PairArgs out;
   memset(&out, 0, sizeof(out));
   out.u = u; out.j = j; out.dj = dj; out.ldo = ldo;
-  const dim3 bs(32, reduce_rows(nval_of(PASS)));
-  const int grid = int((n + 31) / 32);
-  const bool f2 = precision != VPM_PREC_FP64;   // float-pair slots (PairSum)
-  auto go = [&](auto kern) {
-    kern<<<grid, bs, 0, st>>>(part, ldp, foff, fchunks, nfields, scalar_chunks, t_begin, t_end,
-                              out, post ? *post : PostArgs());
+  constexpr int W = VPM_KERNEL_WINCKELMANS, G = VPM_KERNEL_GAUSSIANERF, M = reduce_segs(nval_of(PASS));
+  auto go = [&](auto fn) {
+    fn(part, ldp, foff, fchunks, nfields, scalar_chunks, t_begin, t_end, out, post, st);
   };
-  constexpr int W = VPM_KERNEL_WINCKELMANS, G = VPM_KERNEL_GAUSSIANERF;
+  const bool f2 = precision != VPM_PREC_FP64;   // float-pair slots (PairSum)
   if (kernel == W) {
-    if (f2 && post) go(reduce_kernel<PASS, W, true, true>);
-    else if (f2) go(reduce_kernel<PASS, W, true, false>);
-    else if (post) go(reduce_kernel<PASS, W, false, true>);
-    else go(reduce_kernel<PASS, W, false, false>);
+    if (f2) go(segs > 1 ? start_reduce<PASS, W, true, M> : start_reduce<PASS, W, true, 1>);
+    else go(segs > 1 ? start_reduce<PASS, W, false, M> : start_reduce<PASS, W, false, 1>);
   } else {
-    if (f2 && post) go(reduce_kernel<PASS, G, true, true>);
-    else if (f2) go(reduce_kernel<PASS, G, true, false>);
-    else if (post) go(reduce_kernel<PASS, G, false, true>);
-    else go(reduce_kernel<PASS, G, false, false>);
+    if (f2) go(segs > 1 ? start_reduce<PASS, G, true, M> : start_reduce<PASS, G, true, 1>);
+    else go(segs > 1 ? start_reduce<PASS, G, false, M> : start_reduce<PASS, G, false, 1>);
   }
   return cudaGetLastError();
 }
