@@ -28,7 +28,7 @@
 //      regularised kernels of the direct sum (FP32 pair routines on positions
 //      relative to the group's first particle, or FP64);
 //   7. the far field: one thread per target over the unmarked far cells of its
-//      group (M2P, tree.cuh); 5 and 7 run beside 6 on a second stream;
+//      group (M2P, tree.cuh); 5 and 7 run beside 6 on streams of their own;
 //   8. near field, far field and the local expansion at every target (L2P)
 //      added, in the original order.
 // The far field uses the singular kernel, as FLOWVPM's nonzero_sigma=false;
@@ -107,8 +107,9 @@ struct FmmWork {
   int* far_list = nullptr;    // far cell ids per target group (M2P at every target)
   int2* near_list = nullptr;  // near source ranges [x, y) per target group
   int* loc_list = nullptr;    // far cell ids per target group taken by its local expansion
-  cudaStream_t aux = nullptr; // far field and local expansions, beside the near field
-  cudaEvent_t fork = nullptr, join = nullptr;
+  // far field [0] and local expansions [1], beside the near field
+  cudaStream_t aux[2] = {nullptr, nullptr};
+  cudaEvent_t fork = nullptr, join[2] = {nullptr, nullptr};
   void* cub_tmp = nullptr;
   size_t cub_bytes = 0;
   int h_counters[kNumCounters];
@@ -128,9 +129,11 @@ void fmm_free(FmmWork* w) {
                   w->leaves, w->ggeom, w->cgeom, w->front, w->pairs, w->counters, w->box,
                   w->box_part, w->wcnt, w->gtot, w->gbase, w->gorder, w->totals, w->far_list,
                   w->near_list, w->cub_tmp, w->loc, w->loc_list};
-  if (w->aux) cudaStreamDestroy(w->aux);
   if (w->fork) cudaEventDestroy(w->fork);
-  if (w->join) cudaEventDestroy(w->join);
+  for (int k = 0; k < 2; ++k) {
+    if (w->aux[k]) cudaStreamDestroy(w->aux[k]);
+    if (w->join[k]) cudaEventDestroy(w->join[k]);
+  }
   for (void* p : ptrs) cudaFree(p);
   delete w;
 }
@@ -1467,7 +1470,7 @@ __global__ void __launch_bounds__(kM2lThreads) m2l_kernel(int ngroups, const int
 }
 
 // ---------------------------------------------------------------- far field --
-// One thread per target (CTA per target group, the longest far lists first: they
+// One CTA per target group, one thread per target or two, the longest far lists first (they
 // are ten times the average, and one that starts last runs alone): the moments of
 // the group's far cells at the target (M2P; the cells of the group's local expansion
 // are on their own list).  U and J of the far field, without the 1/(4π), go to rows
@@ -1480,8 +1483,15 @@ __host__ __device__ constexpr int far_chunk() {
   return 12288 / int(ncoef(P) * sizeof(M4<M>)) > 0 ? 12288 / int(ncoef(P) * sizeof(M4<M>)) : 1;
 }
 
-template <int P, typename R, typename M>
-__global__ void __launch_bounds__(kTreeBlock) far_kernel(
+// PAIR (FP32, P <= 4): two targets per thread (m2p2), one warp a group.  Half the issue
+// slots, so the better form where the SMs are full: N = 500,009 (7,813 groups) 14.5 ->
+// 12.6 ms.  A field of one wave of groups ends with its longest list, which one warp
+// with every target walks slower than two (938 groups: 1.5 -> 1.9 ms); two waves of its
+// eight groups per SM is where the line lies.
+constexpr int kFarPairGroups = 2 * 8 * 152;
+
+template <int P, typename R, typename M, bool PAIR>
+__global__ void __launch_bounds__(PAIR ? kTreeBlock / 2 : kTreeBlock) far_kernel(
     int64_t n, int ngroups, const int* __restrict__ gorder, const int* __restrict__ gbase,
     const int* __restrict__ gtot, const int* __restrict__ far_list,
     const double* __restrict__ geom, const M* __restrict__ mom, const double* __restrict__ sorted,
@@ -1502,27 +1512,34 @@ __global__ void __launch_bounds__(kTreeBlock) far_kernel(
   const double ox = sorted[a], oy = sorted[ldw + a], oz = sorted[2 * ldw + a];
   const int f0 = gbase[g], fn = gtot[g];
   if (threadIdx.x == 0) atomicAdd(&pairs[1], (unsigned long long)fn * (unsigned long long)(b - a));
+  constexpr int THREADS = PAIR ? kTreeBlock / 2 : kTreeBlock;
+  using V = typename std::conditional<PAIR, float2, R>::type;   // a value of the thread's targets
   const int i = a + int(threadIdx.x);
-  const bool active = i < b;
   {
-    const int ii = active ? i : a;
-    const R x = R(sorted[ii] - ox), y = R(sorted[ldw + ii] - oy), z = R(sorted[2 * ldw + ii] - oz);
-    R dp[9], dd[18];
-#pragma unroll
-    for (int k = 0; k < 9; ++k) dp[k] = R(0);
-#pragma unroll
-    for (int k = 0; k < 18; ++k) dd[k] = R(0);
+    // Target i, and with PAIR target i + 32 beside it.
+    auto coordinate = [&](int d, double o) {
+      const int i0 = i < b ? i : a;
+      const R x0 = R(sorted[d * ldw + i0] - o);
+      if constexpr (PAIR) {
+        const int i1 = i + THREADS < b ? i + THREADS : a;
+        return make_float2(x0, R(sorted[d * ldw + i1] - o));
+      } else {
+        return x0;
+      }
+    };
+    const V x = coordinate(0, ox), y = coordinate(1, oy), z = coordinate(2, oz);
+    V dp[9] = {}, dd[18] = {};
     for (int c0 = 0; c0 < fn; c0 += FCH) {
       const int cnt = min(FCH, fn - c0);
       __syncthreads();   // previous chunk consumed
-      for (int e = int(threadIdx.x); e < cnt * ROWM; e += kTreeBlock) {
+      for (int e = int(threadIdx.x); e < cnt * ROWM; e += THREADS) {
         const int c = e / ROWM, k = e - c * ROWM;
         const int s = far_list[f0 + c0 + c];
         const int m = k / NC;
         reinterpret_cast<M*>(&smom[c * NC + (k - m * NC)])[m] =
             (s < 0 || s >= ncells) ? M(0) : mom[int64_t(s) * ROWM + k];
       }
-      for (int c = int(threadIdx.x); c < cnt; c += kTreeBlock) {
+      for (int c = int(threadIdx.x); c < cnt; c += THREADS) {
         const int s = far_list[f0 + c0 + c];
         double sx = 1e18, sy = 0.0, sz = 0.0, sr;   // far away: finite, negligible terms
         if (s < 0 || s >= ncells) {   // a list entry outside the tree: record, skip (zero moments)
@@ -1534,18 +1551,38 @@ __global__ void __launch_bounds__(kTreeBlock) far_kernel(
       }
       __syncthreads();
       for (int c = 0; c < cnt; ++c) {
-        R bk[ncoef(P + 2)];
-        taylor_coefficients<P + 2, R>(x - sctr[c][0], y - sctr[c][1], z - sctr[c][2], bk);
-        m2p_accumulate<P, R, M>(bk, smom + c * NC, dp, dd);
+        if constexpr (PAIR) {
+          const float cx = sctr[c][0], cy = sctr[c][1], cz = sctr[c][2];
+          m2p2<P>(add2(x, bc2(-cx)), add2(y, bc2(-cy)), add2(z, bc2(-cz)), smom + c * NC, dp, dd);
+        } else {
+          R bk[ncoef(P + 2)];
+          taylor_coefficients<P + 2, R>(x - sctr[c][0], y - sctr[c][1], z - sctr[c][2], bk);
+          m2p_accumulate<P, R, M>(bk, smom + c * NC, dp, dd);
+        }
       }
     }
-    if (!active) return;
-    R uf[3], jf[9];
-    curl_from_potential<R>(dp, dd, uf, jf);
+    auto store = [&](int t, const R (&p1)[9], const R (&p2)[18]) {
+      if (t >= b) return;
+      R uf[3], jf[9];
+      curl_from_potential<R>(p1, p2, uf, jf);
 #pragma unroll
-    for (int k = 0; k < 3; ++k) pot[k * ldp + i] = uf[k];
+      for (int k = 0; k < 3; ++k) pot[k * ldp + t] = uf[k];
 #pragma unroll
-    for (int k = 0; k < 9; ++k) pot[(3 + k) * ldp + i] = jf[k];
+      for (int k = 0; k < 9; ++k) pot[(3 + k) * ldp + t] = jf[k];
+    };
+    if constexpr (PAIR) {
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        R p1[9], p2[18];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) p1[k] = h ? dp[k].y : dp[k].x;
+#pragma unroll
+        for (int k = 0; k < 18; ++k) p2[k] = h ? dd[k].y : dd[k].x;
+        store(i + h * THREADS, p1, p2);
+      }
+    } else {
+      store(i, dp, dd);
+    }
   }
 }
 
@@ -1644,9 +1681,13 @@ cudaError_t reserve_particles(FmmWork* w, int64_t n) {
     w->cap = 0;
     return e;
   }
-  if (!w->aux) e = cudaStreamCreateWithFlags(&w->aux, cudaStreamNonBlocking);
-  if (e == cudaSuccess && !w->fork) e = cudaEventCreateWithFlags(&w->fork, cudaEventDisableTiming);
-  if (e == cudaSuccess && !w->join) e = cudaEventCreateWithFlags(&w->join, cudaEventDisableTiming);
+  if (!w->fork) e = cudaEventCreateWithFlags(&w->fork, cudaEventDisableTiming);
+  for (int k = 0; k < 2; ++k) {
+    if (e == cudaSuccess && !w->aux[k])
+      e = cudaStreamCreateWithFlags(&w->aux[k], cudaStreamNonBlocking);
+    if (e == cudaSuccess && !w->join[k])
+      e = cudaEventCreateWithFlags(&w->join[k], cudaEventDisableTiming);
+  }
   if (e != cudaSuccess) {
     w->cap = 0;
     return e;
@@ -1696,14 +1737,22 @@ void launch_m2l(FmmWork* w, int ngroups, int ncells, cudaStream_t st) {
 template <int P>
 void launch_far(FmmWork* w, bool f64, int64_t n, int ngroups, int ncells, int64_t ldw,
                 cudaStream_t st) {
-  if (f64)
-    far_kernel<P, double, double><<<ngroups, kTreeBlock, 0, st>>>(
-        n, ngroups, w->gorder, w->gbase, w->gtot, w->far_list, w->geom, w->mom, w->sorted, ldw,
-        w->pot, ldw, ncells, w->counters, w->pairs);
-  else
-    far_kernel<P, float, float><<<ngroups, kTreeBlock, 0, st>>>(
-        n, ngroups, w->gorder, w->gbase, w->gtot, w->far_list, w->geom, w->momf, w->sorted, ldw,
-        reinterpret_cast<float*>(w->pot), ldw, ncells, w->counters, w->pairs);
+  auto go = [&](auto kernel, int threads, auto* mom, auto* pot) {
+    kernel<<<ngroups, threads, 0, st>>>(n, ngroups, w->gorder, w->gbase, w->gtot, w->far_list, w->geom,
+                                        mom, w->sorted, ldw, pot, ldw, ncells, w->counters, w->pairs);
+  };
+  if (f64) {
+    go(far_kernel<P, double, double, false>, kTreeBlock, w->mom, w->pot);
+    return;
+  }
+  float* pot = reinterpret_cast<float*>(w->pot);
+  if constexpr (P <= 4) {
+    if (ngroups >= kFarPairGroups) {
+      go(far_kernel<P, float, float, true>, kTreeBlock / 2, w->momf, pot);
+      return;
+    }
+  }
+  go(far_kernel<P, float, float, false>, kTreeBlock, w->momf, pot);
 }
 
 template <int KERNEL, typename R, bool D, int Q>
@@ -1822,7 +1871,8 @@ cudaError_t fmm_eval(vpm_ctx* c, int kernel, int prec, int p, int ncrit, double 
   // 2. tree, generation by generation
   stage = "tree build";
   tree_init_kernel<<<1, 1, 0, st>>>(n, w->lo, w->hi, w->skip, w->counters);
-  const int split_grid = int(std::min<int64_t>((w->cell_cap + 255) / 256, 4 * 152));
+  // (32 cells a block; most of the launches find an empty generation.)
+  const int split_grid = int(std::min<int64_t>((w->cell_cap + 31) / 32, 152));
   for (int g = 0; g < kMaxGen - 1; ++g) {
     tree_split_kernel<<<split_grid, 256, 0, st>>>(g, ncrit, w->cell_cap, codes, w->lo, w->hi,
                                                   w->child, w->nchild, w->skip, w->leaves, w->counters);
@@ -1932,17 +1982,20 @@ cudaError_t fmm_eval(vpm_ctx* c, int kernel, int prec, int p, int ncrit, double 
                                                w->counters, ncells);
   if ((e = launched(1)) != cudaSuccess) return e;
 
-  // 5.-7. far field (M2P) and local expansions (M2L) on the second stream, the near
-  // field on the context's: they share nothing that is written, each leaves parts of
-  // the chip idle at its end, and the M2L kernel (a warp per group) all along.
+  // 5.-7. far field (M2P) and local expansions (M2L) on streams of their own, the near
+  // field on the context's: they share nothing that is written.  The far field goes
+  // first: its CTAs leave room for M2L's (96 registers of 64 threads, bound by shared
+  // memory) but not for the near field's (168 of 128), which fill the SMs as the far
+  // field's shorter lists end.
   e = cudaEventRecord(w->fork, st);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(w->aux, w->fork, 0);
+  for (int k = 0; k < 2; ++k)
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(w->aux[k], w->fork, 0);
   if (e != cudaSuccess) return e;
   stage = "far field";
-  if (p == 2) launch_far<2>(w, f64, n, ngroups, ncells, ldw, w->aux);
-  else if (p == 4) launch_far<4>(w, f64, n, ngroups, ncells, ldw, w->aux);
-  else launch_far<6>(w, f64, n, ngroups, ncells, ldw, w->aux);
-  if (local) launch_m2l<4, kLocalOrder>(w, ngroups, ncells, w->aux);
+  if (p == 2) launch_far<2>(w, f64, n, ngroups, ncells, ldw, w->aux[0]);
+  else if (p == 4) launch_far<4>(w, f64, n, ngroups, ncells, ldw, w->aux[0]);
+  else launch_far<6>(w, f64, n, ngroups, ncells, ldw, w->aux[0]);
+  if (local) launch_m2l<4, kLocalOrder>(w, ngroups, ncells, w->aux[1]);
   if (f64) {
     if (kernel == VPM_KERNEL_WINCKELMANS)
       near_f64_kernel<VPM_KERNEL_WINCKELMANS><<<ngroups, kTreeBlock, 0, st>>>(
@@ -1958,10 +2011,13 @@ cudaError_t fmm_eval(vpm_ctx* c, int kernel, int prec, int p, int ncrit, double 
     launch_near<VPM_KERNEL_GAUSSIANERF, PASS_UJ>(ngroups, items, w, nullptr, 0, n, w->pairs, st);
   }
   const cudaError_t le = launched(2 + local);
-  // The second stream always rejoins, whatever failed.
-  e = cudaEventRecord(w->join, w->aux);
-  if (e == cudaSuccess) e = cudaStreamWaitEvent(st, w->join, 0);
-  if (e != cudaSuccess) cudaStreamSynchronize(w->aux);
+  // The other streams always rejoin, whatever failed.
+  for (int k = 0; k < 2; ++k) {
+    cudaError_t je = cudaEventRecord(w->join[k], w->aux[k]);
+    if (je == cudaSuccess) je = cudaStreamWaitEvent(st, w->join[k], 0);
+    if (je != cudaSuccess) cudaStreamSynchronize(w->aux[k]);
+    if (e == cudaSuccess) e = je;
+  }
   if (le != cudaSuccess) return le;
   if (e != cudaSuccess) return e;
 

@@ -50,6 +50,16 @@ __device__ __forceinline__ void monomials(R dx, R dy, R dz, R (&p)[ncoef(Q)]) {
       }
 }
 
+// x/n correctly rounded, for the constants 1..8 of the recurrence: in FP32 by
+// Markstein's correction of x·RN(1/n) (Brisebarre, Muller & Raina, IEEE Trans.
+// Computers 53 (2004), for a divisor known in advance; checked over all mantissas), three
+// operations where the general division is a dozen, in FP64 the division.
+__device__ __forceinline__ float div_const(float x, int n) {
+  const float y = 1.f / float(n), q = __fmul_rn(x, y);
+  return __fmaf_rn(__fmaf_rn(-q, float(n), x), y, q);
+}
+__device__ __forceinline__ double div_const(double x, int n) { return x / double(n); }
+
 // Taylor coefficients b_k(R) of 1/|x - y| for |k| <= Q (see the header).
 template <int Q, typename R>
 __device__ __forceinline__ void taylor_coefficients(R rx, R ry, R rz, R (&bk)[ncoef(Q)]) {
@@ -58,8 +68,8 @@ __device__ __forceinline__ void taylor_coefficients(R rx, R ry, R rz, R (&bk)[nc
   bk[0] = sqrt(ir2);
 #pragma unroll
   for (int n = 1; n <= Q; ++n) {
-    const R f1 = R(2 * n - 1) * ir2 / R(n);
-    const R f2 = R(n - 1) * ir2 / R(n);
+    const R f1 = div_const(R(2 * n - 1) * ir2, n);
+    const R f2 = div_const(R(n - 1) * ir2, n);
 #pragma unroll
     for (int a = n; a >= 0; --a)
 #pragma unroll
@@ -118,6 +128,104 @@ __device__ __forceinline__ void m2p_accumulate(const R (&bk)[ncoef(P + 2)], cons
         ddpsi[12] += h12 * m0; ddpsi[13] += h12 * m1; ddpsi[14] += h12 * m2;
         ddpsi[15] += h22 * m0; ddpsi[16] += h22 * m1; ddpsi[17] += h22 * m2;
       }
+}
+
+// ---- M2P for two targets per thread, packed FP32 --------------------------------
+// taylor_coefficients and m2p_accumulate for the target pair in the lanes of a float2,
+// with the packed instructions of sm_100+ and the scalar form's operations in its order
+// (each multiply-add fused as there), so each lane has its bits.  Orders are formed and
+// contracted in step, three of them live at a time: 64 coefficients of the 84 (P = 4).
+
+// x/N as div_const.
+template <int N>
+__device__ __forceinline__ float2 div2_const(float2 x) {
+  constexpr float y = 1.f / float(N);
+  const float2 q = __fmul2_rn(x, make_float2(y, y));
+  if constexpr (N == 1 || N == 2 || N == 4) return q;
+  const float2 r = __ffma2_rn(q, make_float2(-float(N), -float(N)), x);
+  return __ffma2_rn(r, make_float2(y, y), q);
+}
+
+// Number of multi-indices of order n, and the place of (a, b, c) among them.
+__host__ __device__ constexpr int nord(int n) { return (n + 1) * (n + 2) / 2; }
+__host__ __device__ constexpr int oidx(int b, int c) { return (b + c) * (b + c + 1) / 2 + c; }
+
+// Coefficients of order N from those of N - 1 (b1) and N - 2 (b2).
+template <int N, int N1, int N2, int NN>
+__device__ __forceinline__ void taylor_order2(float2 rx, float2 ry, float2 rz, float2 ir2,
+                                              const float2 (&b1)[N1], const float2 (&b2)[N2],
+                                              float2 (&out)[NN]) {
+  const float2 zero = make_float2(0.f, 0.f);
+  const float2 f1 = div2_const<N>(__fmul2_rn(make_float2(2 * N - 1, 2 * N - 1), ir2));
+  const float2 f2 = div2_const<N>(__fmul2_rn(make_float2(N - 1, N - 1), ir2));
+#pragma unroll
+  for (int a = N; a >= 0; --a)
+#pragma unroll
+    for (int b = N - a; b >= 0; --b) {
+      const int c = N - a - b;
+      float2 s1 = zero, s2 = zero;
+      if (a > 0) s1 = __ffma2_rn(rx, b1[oidx(b, c)], s1);
+      if (b > 0) s1 = __ffma2_rn(ry, b1[oidx(b - 1, c)], s1);
+      if (c > 0) s1 = __ffma2_rn(rz, b1[oidx(b, c - 1)], s1);
+      if constexpr (N > 1) {
+        if (a > 1) s2 = __fadd2_rn(s2, b2[oidx(b, c)]);
+        if (b > 1) s2 = __fadd2_rn(s2, b2[oidx(b - 2, c)]);
+        if (c > 1) s2 = __fadd2_rn(s2, b2[oidx(b, c - 2)]);
+      }
+      const float2 t = __fmul2_rn(f2, s2);
+      out[oidx(b, c)] = __ffma2_rn(f1, s1, make_float2(-t.x, -t.y));
+    }
+}
+
+// Contract the moments of order N with the coefficients of orders N + 1 and N + 2, and
+// go on to order N + 1.  dp and dd as in m2p_accumulate.
+template <int N, int P, int N0, int N1>
+__device__ __forceinline__ void m2p_orders2(float2 rx, float2 ry, float2 rz, float2 ir2,
+                                            const float2 (&b0)[N0], const float2 (&b1)[N1],
+                                            const M4<float>* mom, float2 (&dp)[9], float2 (&dd)[18]) {
+  float2 b2[nord(N + 2)];
+  taylor_order2<N + 2>(rx, ry, rz, ir2, b1, b0, b2);
+#pragma unroll
+  for (int a = N; a >= 0; --a)
+#pragma unroll
+    for (int b = N - a; b >= 0; --b) {
+      const int c = N - a - b;
+      const M4<float> mk = mom[midx(a, b, c)];
+      const float2 m[3] = {make_float2(mk.x, mk.x), make_float2(mk.y, mk.y), make_float2(mk.z, mk.z)};
+      auto times = [](int f, float2 v) {
+        return __fmul2_rn(make_float2(float(f), float(f)), v);
+      };
+      const float2 g[3] = {times(-(a + 1), b1[oidx(b, c)]), times(-(b + 1), b1[oidx(b + 1, c)]),
+                           times(-(c + 1), b1[oidx(b, c + 1)])};
+      const float2 h[6] = {times((a + 1) * (a + 2), b2[oidx(b, c)]),
+                           times((a + 1) * (b + 1), b2[oidx(b + 1, c)]),
+                           times((a + 1) * (c + 1), b2[oidx(b, c + 1)]),
+                           times((b + 1) * (b + 2), b2[oidx(b + 2, c)]),
+                           times((b + 1) * (c + 1), b2[oidx(b + 1, c + 1)]),
+                           times((c + 1) * (c + 2), b2[oidx(b, c + 2)])};
+#pragma unroll
+      for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+          if (i != k) dp[3 * i + k] = __ffma2_rn(g[i], m[k], dp[3 * i + k]);   // (the curl takes no ∂_iψ_i)
+#pragma unroll
+      for (int i = 0; i < 6; ++i)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) dd[3 * i + k] = __ffma2_rn(h[i], m[k], dd[3 * i + k]);
+    }
+  if constexpr (N < P) m2p_orders2<N + 1, P>(rx, ry, rz, ir2, b1, b2, mom, dp, dd);
+}
+
+template <int P>
+__device__ __forceinline__ void m2p2(float2 rx, float2 ry, float2 rz, const M4<float>* mom,
+                                     float2 (&dp)[9], float2 (&dd)[18]) {
+  const float2 r2 = __ffma2_rn(rz, rz, __ffma2_rn(rx, rx, __fmul2_rn(ry, ry)));
+  const float2 ir2 = make_float2(__frcp_rn(r2.x), __frcp_rn(r2.y));
+  const float2 b0[1] = {make_float2(__fsqrt_rn(ir2.x), __fsqrt_rn(ir2.y))};
+  const float2 none[1] = {};
+  float2 b1[3];
+  taylor_order2<1>(rx, ry, rz, ir2, b0, none, b1);
+  m2p_orders2<0, P>(rx, ry, rz, ir2, b0, b1, mom, dp, dd);
 }
 
 // U = ∇ × ψ and J_ab = ∂_b U_a from ∂ψ and ∂∂ψ (already scaled by 1/(4π)).
