@@ -69,6 +69,9 @@ struct PairTraits {
   // differently, follows from the boxes.
   template <int KERNEL>
   static constexpr bool kWarpRuns = !(kUJ && KERNEL == VPM_KERNEL_WINCKELMANS && PREC != VPM_PREC_FP64);
+  // FP32 Gaussian-erf ζ passes: every warp stages its sources for itself.
+  template <int KERNEL>
+  static constexpr bool kWarpStage = !kUJ && KERNEL == VPM_KERNEL_GAUSSIANERF && PREC != VPM_PREC_FP64;
   // float4 per source record: U/J 3, ζ 4 (+ v_q), ζ + α-derivative 5 (+ w_q).
   static constexpr int kRecQuads = kUJ ? 3 : (PASS == PASS_ZETA ? 4 : 5);
   static constexpr int kRecBytes = 16 * kRecQuads;
@@ -541,7 +544,83 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
     int tiles = 0;
     bool aborted = false;
     if (use_tma && tid == 0 && s0 < s1) issue(s0, s1);
-    for (int64_t tile0 = s0; tile0 < s1; tile0 += BLOCK) {
+    // Fold the FP32 sums of the last kFoldSources sources into the (hi, lo) pairs.
+    auto fold = [&]() {
+#pragma unroll
+      for (int k = 0; k < T; ++k)
+#pragma unroll
+        for (int v = 0; v < NV; ++v) {
+          const int o = (v * T + k) * BLOCK + tid;
+          float s, e;
+          two_sum(fold_hi[o], float(acc[k][v]), s, e);
+          fold_hi[o] = s;
+          fold_lo[o] += e;
+          acc[k][v] = R(0);
+        }
+    };
+    // Gaussian-erf ζ vanishes beyond 13.3 σ: at 50,021 particles of a wake seven in ten
+    // (warp, source) pairs are skipped, and which ones differs from warp to warp.  With
+    // tiles staged for the block, the warps waited for one another at every tile (a
+    // quarter of their time).  So a warp takes 32 sources at a time by itself: lane j
+    // reads the position of source j and classes it; where any is left the warp stages
+    // them in its own 32 places, and there is no block barrier.  The diagnostics call of
+    // that field, most of it the ζ pass: 756 -> 726 µs.  (The U/J passes, which take every
+    // source, lose by it, each source being formed once per warp: a wake of 50,021
+    // particles 22.43 -> 22.68 ms a step.)
+    constexpr bool WSTAGE = Tr::template kWarpStage<KERNEL>;
+    if constexpr (WSTAGE) {
+      constexpr bool DD = PASS == PASS_ZETAD;
+      const int lane = tid & 31;
+      float4* ta = reinterpret_cast<float4*>(tileA) + warp * 32;
+      float4* tb = reinterpret_cast<float4*>(tileB) + warp * 32;
+      float4* tc = reinterpret_cast<float4*>(tileC) + warp * 32;
+      float4* td = DD ? reinterpret_cast<float4*>(tileD) + warp * 32 : tc;
+      float4 r0 = make_float4(0.f, 0.f, 0.f, 0.f), r1 = r0;
+      auto fetch = [&](int64_t b) {   // the position record of this lane's source
+        const int64_t jj = min(b + lane, s1 - 1);
+        r0 = a.rec[Tr::kRecQuads * jj];
+        r1 = a.rec[Tr::kRecQuads * jj + 1];
+      };
+      __syncwarp();   // the target box
+      if (live && s0 < s1) fetch(s0);
+      int blocks = 0;
+      for (int64_t b0 = s0; live && b0 < s1; b0 += 32) {
+        const int n32 = int(min(int64_t(32), s1 - b0));
+        const float4 qa = make_float4(rel_f32(r0.x, r1.x, chx, clx), rel_f32(r0.y, r1.y, chy, cly),
+                                      rel_f32(r0.z, r1.z, chz, clz), r0.w);
+        const float b = r1.w;
+        if (b0 + 32 < s1) fetch(b0 + 32);
+        const SourceMasks m = source_masks(tbox + 2 * warp, qa, use_far);
+        if (m.zero != 0xffffffffu) {
+          // (A lane past the last source holds that one again.)
+          const float4* r = a.rec + Tr::kRecQuads * min(b0 + lane, s1 - 1);
+          const float4 r2 = r[2], r3 = r[3];
+          __syncwarp();   // the last 32 are done
+          ta[lane] = qa;
+          tb[lane] = make_float4(r2.x, r2.y, r2.z, b);
+          tc[lane] = make_float4(r3.x, r3.y, r3.z, r2.w);
+          if constexpr (DD) td[lane] = r[4];
+          __syncwarp();
+          for (int js = 0; js < n32;) {
+            // (A zero source is never inside.)
+            const int je = min(n32, min(mask_run(m.zero, js), mask_run(m.inside, js)));
+            if ((m.zero >> js) & 1u) {
+              js = je;
+            } else if ((m.inside >> js) & 1u) {
+#pragma unroll 2
+              for (; js < je; ++js)
+                zeta_source<KERNEL, T, true, DD, false>(ta[js], tb[js], tc[js], td[js], tx, ty, tz, acc);
+            } else {
+#pragma unroll 2
+              for (; js < je; ++js)
+                zeta_source<KERNEL, T, false, DD, false>(ta[js], tb[js], tc[js], td[js], tx, ty, tz, acc);
+            }
+          }
+        }
+        if (COMP && (++blocks % (kFoldSources / 32) == 0 || b0 + 32 >= s1)) fold();
+      }
+    }
+    if constexpr (!WSTAGE) for (int64_t tile0 = s0; tile0 < s1; tile0 += BLOCK) {
       // ---- stage one tile of sources -------------------------------------
       __syncthreads();  // previous tile fully consumed
       if constexpr (Tr::kTma) {
@@ -684,18 +763,15 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
             // Gaussian-erf masks coincident pairs in its series branch, which
             // every warp holding a pair with ρ² < 3/2 takes.
             // Gaussian-erf by runs of sources of one class: far sources skip
-            // erfcx/exp, vote sources decide by their true distances.
+            // erfcx/exp.
             SourceMasks m;
             for (int js = 0; js < cnt;) {
               const int b = js & 31;
-              if (b == 0) m = source_masks(tbox + 2 * warp, ta + js, kVoteSpan * kArgFar, use_far);
+              if (b == 0) m = source_masks(tbox + 2 * warp, ta[js + (tid & 31)], use_far);
               const int je = min(cnt, js - b + mask_run(m.far, b));
               if ((m.far >> b) & 1u) {
 #pragma unroll 2
                 for (; js < je; ++js) uj_source_gauss_far<T>(ta[js], tb[js], tx, ty, tz, acc);
-              } else if (m.vote) {
-#pragma unroll 2
-                for (; js < je; ++js) uj_source_gauss<T, true>(ta[js], tb[js], tx, ty, tz, acc);
               } else {
 #pragma unroll 2
                 for (; js < je; ++js) uj_source_gauss<T, false>(ta[js], tb[js], tx, ty, tz, acc);
@@ -719,15 +795,13 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
             SourceMasks m;
             for (int js = 0; js < cnt;) {
               const int b = js & 31;
-              if (b == 0) m = source_masks(tbox + 2 * warp, ta + js, kVoteSpan * kArgFar, use_far);
+              if (b == 0) m = source_masks(tbox + 2 * warp, ta[js + (tid & 31)], use_far);
               // (Zero sources are far too.)
               const int je = min(cnt, js - b + min(mask_run(m.zero, b), mask_run(m.far, b)));
               if ((m.zero >> b) & 1u) {
                 for (; js < je; ++js) uj_source_gauss_far<T>(ta[js], tb[js], tx, ty, tz, acc);
               } else if ((m.far >> b) & 1u) {
                 for (; js < je; ++js) ujd_source_gauss_far<T>(ta[js], tb[js], tx, ty, tz, acc);
-              } else if (m.vote) {
-                for (; js < je; ++js) ujd_source_gauss<T, true>(ta[js], tb[js], tx, ty, tz, acc);
               } else {
                 for (; js < je; ++js) ujd_source_gauss<T, false>(ta[js], tb[js], tx, ty, tz, acc);
               }
@@ -794,31 +868,22 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
           }
         }
       } else if constexpr (F32) {
-        // ζ passes, FP32.
+        // ζ passes, FP32 Winckelmans: a source inside the target box may coincide with
+        // a target (masked).
         const float4* ta = reinterpret_cast<const float4*>(tileA);
         const float4* tb = reinterpret_cast<const float4*>(tileB);
         const float4* tc = reinterpret_cast<const float4*>(tileC);
         const float4* td = reinterpret_cast<const float4*>(PASS == PASS_ZETAD ? tileD : tileC);
         constexpr bool DD = PASS == PASS_ZETAD;
-        // Sources whose ζ is exactly zero at every target of the warp (Gaussian-erf)
-        // are skipped; a source inside the target box may coincide with a target
-        // (masked); the others take votes where the targets are compact.
         SourceMasks m;
         for (int js = 0; js < cnt;) {
           const int b = js & 31;
-          if (b == 0) m = source_masks(tbox + 2 * warp, ta + js, kVoteSpan * kArgZero, use_far);
-          // (A zero source is never inside.)
-          const int je = min(cnt, js - b + min(mask_run(m.zero, b), mask_run(m.inside, b)));
-          if ((m.zero >> b) & 1u) {
-            js = je;
-          } else if ((m.inside >> b) & 1u) {
+          if (b == 0) m = source_masks(tbox + 2 * warp, ta[js + (tid & 31)], false);
+          const int je = min(cnt, js - b + mask_run(m.inside, b));
+          if ((m.inside >> b) & 1u) {
 #pragma unroll 2
             for (; js < je; ++js)
               zeta_source<KERNEL, T, true, DD, false>(ta[js], tb[js], tc[js], td[js], tx, ty, tz, acc);
-          } else if (m.vote) {
-#pragma unroll 2
-            for (; js < je; ++js)
-              zeta_source<KERNEL, T, false, DD, true>(ta[js], tb[js], tc[js], td[js], tx, ty, tz, acc);
           } else {
 #pragma unroll 2
             for (; js < je; ++js)
@@ -871,20 +936,7 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
         }
       }
 
-      if (COMP && (++tiles % FOLD_TILES == 0 || tile0 + BLOCK >= s1)) {
-        // Fold the FP32 sums of the last kFoldSources sources into the (hi, lo) pairs.
-#pragma unroll
-        for (int k = 0; k < T; ++k)
-#pragma unroll
-          for (int v = 0; v < NV; ++v) {
-            const int o = (v * T + k) * BLOCK + tid;
-            float s, e;
-            two_sum(fold_hi[o], float(acc[k][v]), s, e);
-            fold_hi[o] = s;
-            fold_lo[o] += e;
-            acc[k][v] = R(0);
-          }
-      }
+      if (COMP && (++tiles % FOLD_TILES == 0 || tile0 + BLOCK >= s1)) fold();
     }
 
     // A CTA whose copy timed out leaves without results (the status word
@@ -1164,6 +1216,9 @@ cudaError_t launch(int kernel, int precision, Shape s, const PairArgs& a, int gr
   PairFn f = pick_kernel<PASS>(kernel, precision, s);
   if (!f) return cudaErrorInvalidConfiguration;
   if (grid <= 0) return cudaSuccess;
+  // The Gaussian-erf ζ passes read nothing but records.
+  if (precision != VPM_PREC_FP64 && (PASS == PASS_ZETA || PASS == PASS_ZETAD) && !a.rec)
+    return cudaErrorInvalidValue;
   if (a.cluster > 1) {
     // One item per CTA, every CTA of a cluster on the same target tile.
     f = pick_cluster<PASS>(kernel, precision, s);

@@ -591,9 +591,9 @@ __device__ __forceinline__ void uj_source_gauss(const float4 sa, const float4 sb
 // The classification is made per warp and staged source (source_masks): the gap g²
 // between the source and the box of the warp's targets satisfies g² <= r² for every
 // pair in the same FP32 arithmetic (rounding is monotone), so g²·a >= arg for every
-// pair.  Sources that do not pass are classified again by warp votes on the true
-// distances (uj_source_gauss, ujd_source_gauss, zeta_source).  Every form gives the
-// same bits where it applies.  kArgFar and kArgZero are defined above
+// pair.  The near field of the treecode takes warp votes on the true distances instead
+// (VOTE of uj_source_gauss, ujd_source_gauss, zeta_source).  Every form gives the same
+// bits where it applies.  kArgFar and kArgZero are defined above
 // uj_source_gauss.
 // q = 1/r³, p = -3/r⁵ for one source against T targets; acc holds the plain
 // sums first (U 0..2, A 3..10, W 12..14), so the α-derivative layout works too.
@@ -674,29 +674,24 @@ __device__ __forceinline__ void warp_source_box(float x, float y, float z, float
   }
 }
 
-// Per-source votes are used where the target box's extent argument is above
-// kVoteSpan times the vote's threshold (both negative).
-constexpr float kVoteSpan = 4.f;
-
-// Classes of the 32 staged sources at ta[0..31] for one warp, a bit per source: lane j
-// tests source j against the box of the warp's targets (tbox[0..1]).
+// Classes of 32 sources for one warp, a bit per source: lane j tests its source q
+// (x, y, z, a) against the box of the warp's targets (tbox[0..1]).
 //   zero    arg <= kArgZero at every target;     far    arg <= kArgFar at every target;
 //   inside  the source lies in the box, the only place where a target can have the
-//           same position (comparisons only: exact);
-//   vote    (for all of them) votes on the others pay: the exponent argument of the
-//           box's own diagonal is at most kVoteSpan times the vote's threshold
-//           (vote_span, negative) for one of the sources.
-// zero, far and vote are 0 when `on` is false.  About 25 instructions for 32 sources;
-// classifying whole blocks by their own boxes (60 shuffles and minima per warp and
-// staged tile) left most sources of a block that straddles the limit to votes of 8 to
-// 20 instructions each: ζ pass of 50,021 particles 785 -> 670 µs.
+//           same position (comparisons only: exact).
+// zero and far are 0 when `on` is false.  About 25 instructions for 32 sources.  Whole
+// blocks classified by their own boxes (60 shuffles and minima per warp and staged tile)
+// left most sources of a block that straddles the limit to votes: diagnostics of 50,021
+// particles 872 -> 756 µs.  A warp vote on the true distances of the rest, as the
+// treecode's near field takes, finds few more (2 % of what is left of that wake for ζ,
+// one in ten of the near sources of a wake of 14,003) and splits the straight-line code:
+// without it 726 -> 650 µs there, and 2.30 -> 2.16 ms for a dynamic-SFS step of 14,003.
 struct SourceMasks {
   uint32_t zero, far, inside;
-  bool vote;
 };
-__device__ __forceinline__ SourceMasks source_masks(const float4* tbox, const float4* ta,
-                                                    float vote_span, bool on) {
-  const float4 tl = tbox[0], th = tbox[1], q = ta[threadIdx.x & 31];
+__device__ __forceinline__ SourceMasks source_masks(const float4* tbox, const float4 q,
+                                                    bool on) {
+  const float4 tl = tbox[0], th = tbox[1];
   const float gx = fmaxf(0.f, fmaxf(q.x - th.x, tl.x - q.x));
   const float gy = fmaxf(0.f, fmaxf(q.y - th.y, tl.y - q.y));
   const float gz = fmaxf(0.f, fmaxf(q.z - th.z, tl.z - q.z));
@@ -705,7 +700,6 @@ __device__ __forceinline__ SourceMasks source_masks(const float4* tbox, const fl
   SourceMasks m;
   m.zero = __ballot_sync(0xffffffffu, on && arg <= kArgZero);
   m.far = __ballot_sync(0xffffffffu, on && arg <= kArgFar);
-  m.vote = __any_sync(0xffffffffu, on && tl.w * q.w >= vote_span);
   m.inside = __ballot_sync(0xffffffffu, !(g2 > 0.f));
   return m;
 }
