@@ -155,9 +155,12 @@ __device__ __forceinline__ double exp2_f64(double r2, double a2048, const double
   const double r = fma(v, g, v);
   // The high word of t is that of 1.5·2^52 or one less for -2^32 <= n <= 0 (a low word
   // above 0 is an n below -2^31); larger for NaN, whose low word is 0.
+  // A vote, so that the product by 2^-128 is not formed for every pair (an FP64 ring step
+  // 22.2 -> 21.6 ms): all 32 lanes call this together.
   const bool in = __double2hiint(t) >= 0x4337ffff && n <= 0;
-  if (in && !low) return r;
-  return in && ex >= -1100 ? r * 0x1p-128 : 0.0;
+  if (!__any_sync(0xffffffffu, low || !in)) return r;
+  if (!in || ex < -1100) return 0.0;
+  return low ? r * 0x1p-128 : r;
 }
 
 // Accumulate one U/J pair: U 0..2, A 3..10 (A22 = -(A00 + A11): the pairs are

@@ -835,7 +835,8 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
                     dq -= q;
                     dp -= p;
                   } else {
-                    const R e = is_zero_f64(r2) ? 0.0 : exp2_f64(r2, sc.y, exp2_tab);
+                    R e = exp2_f64(r2, sc.y, exp2_tab);
+                    if (is_zero_f64(r2)) e = 0.0;
                     dq = -sc.z * e;
                     dp = sc.w * e;
                   }
@@ -906,10 +907,13 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
               const R r2 = fma(dx, dx, fma(dy, dy, dz * dz));
               R z, dzz = 0, zw = 0;   // zw: the ζ that w_q goes with
               if constexpr (KERNEL == VPM_KERNEL_GAUSSIANERF) {
-                z = is_zero_f64(r2) ? 0.0 : exp2_f64(r2, sa.w, exp2_tab);
+                const bool self = is_zero_f64(r2);
+                z = exp2_f64(r2, sa.w, exp2_tab);
+                if (self) z = 0.0;
                 if constexpr (PASS == PASS_ZETAD) {
                   if (a.fd_alpha > 0.0) {
-                    zw = is_zero_f64(r2) ? 0.0 : exp2_f64(r2, sc.w, exp2_tab) * fd_i3;
+                    zw = exp2_f64(r2, sc.w, exp2_tab) * fd_i3;
+                    if (self) zw = 0.0;
                     dzz = zw - z;
                   } else {
                     zw = z;
