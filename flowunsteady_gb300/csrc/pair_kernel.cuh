@@ -64,11 +64,11 @@ struct PairTraits {
   static constexpr bool kRec = PREC != VPM_PREC_FP64;
   static constexpr bool kTma = PASS == PASS_UJ && PREC != VPM_PREC_FP64;
   // Targets of a warp: consecutive (32·T of them), so that its box is as small as
-  // the particles' order allows.  Only the FP32 Winckelmans U/J passes keep the T
-  // runs of 32 a block apart: which of their pairs take the masked form, rounded
-  // differently, follows from the boxes.
+  // the particles' order allows.  Only the FP32 Winckelmans passes keep the T runs of 32
+  // a block apart: which of their U/J pairs take the masked form, rounded differently,
+  // follows from the boxes, and their ζ has nothing to skip.
   template <int KERNEL>
-  static constexpr bool kWarpRuns = !(kUJ && KERNEL == VPM_KERNEL_WINCKELMANS && PREC != VPM_PREC_FP64);
+  static constexpr bool kWarpRuns = KERNEL == VPM_KERNEL_GAUSSIANERF || PREC == VPM_PREC_FP64;
   // FP32 Gaussian-erf ζ passes: every warp stages its sources for itself.
   template <int KERNEL>
   static constexpr bool kWarpStage = !kUJ && KERNEL == VPM_KERNEL_GAUSSIANERF && PREC != VPM_PREC_FP64;
@@ -184,7 +184,7 @@ struct PairSum {
 // The slots of a target are summed in PairArgs::segs runs of consecutive slots, each in
 // slot order, and the runs in order; every form of the sum takes the same runs.
 __host__ __device__ inline int seg_begin(int nc, int seg, int segs) {
-  return int(int64_t(nc) * seg / segs);
+  return nc / segs * seg + nc % segs * seg / segs;   // (a 64-bit product and division spill)
 }
 
 // FP32 U/J passes: the Gaussian-erf A sums carry a scale, and A22 (DA22) is not
@@ -590,7 +590,10 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
                                       rel_f32(r0.z, r1.z, chz, clz), r0.w);
         const float b = r1.w;
         if (b0 + 32 < s1) fetch(b0 + 32);
-        const SourceMasks m = source_masks(tbox + 2 * warp, qa, use_far);
+        SourceMasks m = source_masks(tbox + 2 * warp, qa, use_far);
+        // In a field without order most sources are inside the box: all are masked then,
+        // as runs of one or two cost more (ζ pass of a box of 20,000: 347 -> 284 µs).
+        if (__popc(m.inside) > 4) m.inside = 0xffffffffu;
         if (m.zero != 0xffffffffu) {
           // (A lane past the last source holds that one again.)
           const float4* r = a.rec + Tr::kRecQuads * min(b0 + lane, s1 - 1);
@@ -869,19 +872,16 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
           }
         }
       } else if constexpr (F32) {
-        // ζ passes, FP32 Winckelmans: a source inside the target box may coincide with
-        // a target (masked).
+        // ζ passes, FP32 Winckelmans: by runs of blocks, masked where the boxes intersect.
         const float4* ta = reinterpret_cast<const float4*>(tileA);
         const float4* tb = reinterpret_cast<const float4*>(tileB);
         const float4* tc = reinterpret_cast<const float4*>(tileC);
         const float4* td = reinterpret_cast<const float4*>(PASS == PASS_ZETAD ? tileD : tileC);
         constexpr bool DD = PASS == PASS_ZETAD;
-        SourceMasks m;
+        const uint32_t cls = overlap_codes<BLOCK / 32>(ovl, 1u);
         for (int js = 0; js < cnt;) {
-          const int b = js & 31;
-          if (b == 0) m = source_masks(tbox + 2 * warp, ta[js + (tid & 31)], false);
-          const int je = min(cnt, js - b + mask_run(m.inside, b));
-          if ((m.inside >> b) & 1u) {
+          const int je = block_run_end(cls, js, cnt, [](uint32_t c) { return c; });
+          if ((ovl >> (js >> 5)) & 1u) {
 #pragma unroll 2
             for (; js < je; ++js)
               zeta_source<KERNEL, T, true, DD, false>(ta[js], tb[js], tc[js], td[js], tx, ty, tz, acc);

@@ -640,7 +640,7 @@ __device__ __forceinline__ void warp_box_reduce(float& lx, float& ly, float& lz,
   }
 }
 
-// Box of the T·32 targets of a warp, stored as (lo, extent²), (hi, 0) at box[0..1].
+// Box of the T·32 targets of a warp, stored as (lo, 0), (hi, 0) at box[0..1].
 template <int T>
 __device__ __forceinline__ void warp_target_box(const float (&tx)[T], const float (&ty)[T],
                                                 const float (&tz)[T], float4* box) {
@@ -652,8 +652,7 @@ __device__ __forceinline__ void warp_target_box(const float (&tx)[T], const floa
   }
   warp_box_reduce(lx, ly, lz, hx, hy, hz);
   if ((threadIdx.x & 31) == 0) {
-    const float ex = hx - lx, ey = hy - ly, ez = hz - lz;
-    box[0] = make_float4(lx, ly, lz, fmaf(ex, ex, fmaf(ey, ey, ez * ez)));
+    box[0] = make_float4(lx, ly, lz, 0.f);
     box[1] = make_float4(hx, hy, hz, 0.f);
   }
 }
