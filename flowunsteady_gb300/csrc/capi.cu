@@ -185,11 +185,16 @@ static int plan_cluster(int device, const PairCall& pc, Shape sh, int64_t n_tb,
 constexpr int kSmallWaves = 8;
 constexpr int kLargeWaves = 64;
 constexpr int64_t kLargeField = 131072;
-// Largest field whose reduction takes the particles' updates along: up to about two
-// blocks of 32 particles per SM.  With the updates a block needs 75 to 86 registers a
-// thread and one fits on an SM, where the plain sum has three at a time; a larger
-// field's reduction is bound by reading its partial sums and wants those.
-constexpr int64_t kPostInReduce = 8192;
+// Largest field whose reduction takes the particles' updates along: one block of 32
+// particles per SM.  With the updates one block fits on an SM, where the plain sum has
+// three; a larger field's reduction is bound by reading its partial sums and wants
+// those.  A step without SFS at 3,001 / 4,001 / 5,001 particles, launches of their own
+// against this: 103 / 145 / 186 and 100 / 137 / 203 µs.
+constexpr int64_t kPostInReduce = 4096;
+// Targets whose slots are summed in runs side by side (kReduceSegs): one block of 16
+// targets per SM, each with kSegSlots slots or more.
+constexpr int64_t kSegTargets = 16;
+constexpr int kSegSlots = 32;
 
 // Plan and enqueue one pair pass.  `need_part` (elements) is raised to what
 // the launch needs; when dry, nothing is launched.  A split source range goes
@@ -266,10 +271,14 @@ cudaError_t run_pair(const PairCall& pc, int device, int num_sms, const Shape* p
     n_chunk = plan_chunks(n_tb, pc.ns, sh.block, resident, &chunk, pc.max_chunks);
   // The U/J passes of a step of a small field: at one tile of 128 sources an item, 1,200
   // particles are 50 CTAs, each a chain of 128 sources; items of 16 are 380, and the
-  // step 30 µs shorter.  (Other callers keep whole tiles: a chunk is what the FP32 sums
+  // step 30 to 50 µs shorter.  Up to three items per SM, and where the slots are summed
+  // in runs: beyond either, summing more slots costs what the shorter chains give
+  // (2,001 particles, 128 / 64 / 32 / 16 sources: 125 / 103 / 99 / 104 µs; 3,001: 136 /
+  // 149 / 160 / 185).  (Other callers keep whole tiles: a chunk is what the FP32 sums
   // are folded over, and their results are compared between paths bit for bit.)
-  if (pc.fine && pc.prec == VPM_PREC_FP32C && cluster <= 1 && pc.chunk <= 0 && chunk == sh.block) {
-    while (chunk > 16 && n_tb * ceil_div(pc.ns, chunk) < resident) chunk /= 2;
+  if (pc.fine && pc.prec == VPM_PREC_FP32C && cluster <= 1 && pc.chunk <= 0 && chunk == sh.block &&
+      nt <= kSegTargets * num_sms) {
+    while (chunk > 16 && n_tb * ceil_div(pc.ns, chunk / 2) <= 3 * int64_t(num_sms)) chunk /= 2;
     n_chunk = int(ceil_div(pc.ns, chunk));
   }
   PairPlan plan;
@@ -283,8 +292,8 @@ cudaError_t run_pair(const PairCall& pc, int device, int num_sms, const Shape* p
   plan.post = pc.post && plan.slots() > 1 && !plan.fused && pc.t0 == 0 && nt == pc.ns &&
               nt <= kPostInReduce;
   const int nv = nval_of(pc.pass);
-  // Few blocks of targets (less than two a SM) with many slots each.
-  if (plan.slots() >= 32 && nt < 2 * 32 * int64_t(num_sms)) plan.segs = reduce_segs(nv);
+  if (pc.pass == PASS_UJ && plan.slots() >= kSegSlots && nt <= kSegTargets * num_sms)
+    plan.segs = kReduceSegs;
   const size_t slot_elems = plan.slots() > 1 ? size_t(plan.slots()) * nv * size_t(ldp) : 0;
   // One 32-bit counter per target tile after the slots (two per double).
   const size_t need = slot_elems + (plan.fused ? size_t((n_tb + 1) / 2) : 0);

@@ -24,8 +24,8 @@ __host__ __device__ constexpr int nval_of(int pass) {
                             : kNvalZetaD;
 }
 
-// Runs of slots that a pass of nv values may be summed in (see reduce_kernel).
-__host__ __device__ constexpr int reduce_segs(int nv) { return nv <= 15 ? 4 : 2; }
+// Runs of slots that a U/J pass may be summed in (see reduce_kernel).
+constexpr int kReduceSegs = 4;
 
 // One work item: targets [t0, t1) against sources [s0, s1).  slot < 0 means the
 // item covers all sources of its targets and writes final values; otherwise it

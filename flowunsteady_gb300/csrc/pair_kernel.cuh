@@ -305,10 +305,11 @@ __device__ __noinline__ void tile_reduce(const PairArgs& a, int64_t t0, int64_t 
     for (int w0 = 0; w0 < NV; w0 += G) {
       using Sum = typename std::conditional<F2, PairSum, double>::type;
       Sum all[G] = {};
-      for (int seg = 0; seg < a.segs; ++seg) {
+      const int segs = PASS == PASS_UJ ? a.segs : 1;
+      for (int seg = 0; seg < segs; ++seg) {
         Sum s[G] = {};
-        const int c1 = seg_begin(a.n_chunk, seg + 1, a.segs);
-        int c = seg_begin(a.n_chunk, seg, a.segs);
+        const int c1 = seg_begin(a.n_chunk, seg + 1, segs);
+        int c = seg_begin(a.n_chunk, seg, segs);
         const double* p = a.part + int64_t(w0) * a.ldp + i + int64_t(c) * step;
 #pragma unroll 2
         for (; c < c1; ++c, p += step) {
@@ -1028,7 +1029,7 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
 // summed with PairSum; otherwise FP64 slots and FP64 additions.  tile_reduce adds in
 // the same order.
 //   SEGS 1, COLS 32: a field of many blocks, bound by reading the slots.
-//   SEGS 4, COLS 16 (reduce_segs): few targets with many slots each, where one thread
+//   SEGS 4, COLS 16 (U/J, kReduceSegs): few targets with many slots each, where one thread
 //   per value would walk them alone.
 // POST: each target's particle then goes through the operations of `post`
 // (update_dev.cuh), which saves a small field the launches of its updates.
@@ -1279,7 +1280,7 @@ cudaError_t reduce(int kernel, int precision, const double* part, int64_t ldp,
   PairArgs out;
   memset(&out, 0, sizeof(out));
   out.u = u; out.j = j; out.dj = dj; out.ldo = ldo;
-  constexpr int W = VPM_KERNEL_WINCKELMANS, G = VPM_KERNEL_GAUSSIANERF, M = reduce_segs(nval_of(PASS));
+  constexpr int W = VPM_KERNEL_WINCKELMANS, G = VPM_KERNEL_GAUSSIANERF, M = PASS == PASS_UJ ? kReduceSegs : 1;
   auto go = [&](auto fn) {
     fn(part, ldp, foff, fchunks, nfields, scalar_chunks, t_begin, t_end, out, post, st);
   };
