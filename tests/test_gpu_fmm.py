@@ -248,3 +248,20 @@ def test_near_items_cover_every_range_once(oracle, k, n, ncrit):
         st = all_stats(c)
     assert st["far_entries"] == 0 and st["near_pairs"] == n * n
     assert rel_l2(U[idx], U0) <= 1e-5 and rel_l2(J[idx], J0) <= 1e-5
+
+
+@pytest.mark.parametrize("p", [2, 4])
+@pytest.mark.parametrize("groups,last", [(2431, 64), (2432, 1), (2432, 33), (2433, 64)])
+def test_far_field_with_two_targets_a_thread(p, groups, last):
+    # From 2,432 groups of 64 on; the same lists in FP64 (one target a thread) are the
+    # reference, and FP32C sums are within 1e-5.
+    n = 64 * (groups - 1) + last
+    X, G, S = helical_wake(n)
+    with Ctx(n) as c:
+        c.set(X, G, S)
+        U0, J0 = eval_fmm(c, 1, L.PREC_FP64, fmm(p=p))
+        far = stats(c)[2]
+        U, J = eval_fmm(c, 1, L.PREC_FP32C, fmm(p=p))
+        assert stats(c)[2] == far > 0
+    assert rel_l2(U, U0) <= 1e-5 and rel_l2(J, J0) <= 1e-5
+    assert rel_l2(U[-last:], U0[-last:]) <= 1e-4
