@@ -69,9 +69,11 @@ struct PairTraits {
   // follows from the boxes, and their ζ has nothing to skip.
   template <int KERNEL>
   static constexpr bool kWarpRuns = KERNEL == VPM_KERNEL_GAUSSIANERF || PREC == VPM_PREC_FP64;
-  // FP32 Gaussian-erf ζ passes: every warp stages its sources for itself.
-  template <int KERNEL>
-  static constexpr bool kWarpStage = !kUJ && KERNEL == VPM_KERNEL_GAUSSIANERF && PREC != VPM_PREC_FP64;
+  // FP32 Gaussian-erf ζ passes of four targets a thread (fields of 32,768 particles and
+  // more): every warp stages its sources for itself.
+  template <int KERNEL, int T>
+  static constexpr bool kWarpStage =
+      !kUJ && KERNEL == VPM_KERNEL_GAUSSIANERF && PREC != VPM_PREC_FP64 && T >= 4;
   // float4 per source record: U/J 3, ζ 4 (+ v_q), ζ + α-derivative 5 (+ w_q).
   static constexpr int kRecQuads = kUJ ? 3 : (PASS == PASS_ZETA ? 4 : 5);
   static constexpr int kRecBytes = 16 * kRecQuads;
@@ -565,10 +567,11 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
     // quarter of their time).  So a warp takes 32 sources at a time by itself: lane j
     // reads the position of source j and classes it; where any is left the warp stages
     // them in its own 32 places, and there is no block barrier.  The diagnostics call of
-    // that field, most of it the ζ pass: 756 -> 726 µs.  (The U/J passes, which take every
-    // source, lose by it, each source being formed once per warp: a wake of 50,021
-    // particles 22.43 -> 22.68 ms a step.)
-    constexpr bool WSTAGE = Tr::template kWarpStage<KERNEL>;
+    // that field, most of it the ζ pass: 756 -> 726 µs.  Forming each source once per warp
+    // has its price: with two targets a thread a wake of 14,003 gains nothing and a box of
+    // 30,000, where nothing is skipped, loses 7 %; the U/J passes, which take every source,
+    // lose too (a wake of 50,021 particles 22.43 -> 22.68 ms a step).
+    constexpr bool WSTAGE = Tr::template kWarpStage<KERNEL, T>;
     if constexpr (WSTAGE) {
       constexpr bool DD = PASS == PASS_ZETAD;
       const int lane = tid & 31;
@@ -591,10 +594,7 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
                                       rel_f32(r0.z, r1.z, chz, clz), r0.w);
         const float b = r1.w;
         if (b0 + 32 < s1) fetch(b0 + 32);
-        SourceMasks m = source_masks(tbox + 2 * warp, qa, use_far);
-        // In a field without order most sources are inside the box: all are masked then,
-        // as runs of one or two cost more (ζ pass of a box of 20,000: 347 -> 284 µs).
-        if (__popc(m.inside) > 4) m.inside = 0xffffffffu;
+        const SourceMasks m = zeta_masks(tbox + 2 * warp, qa, use_far);
         if (m.zero != 0xffffffffu) {
           // (A lane past the last source holds that one again.)
           const float4* r = a.rec + Tr::kRecQuads * min(b0 + lane, s1 - 1);
@@ -606,7 +606,6 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
           if constexpr (DD) td[lane] = r[4];
           __syncwarp();
           for (int js = 0; js < n32;) {
-            // (A zero source is never inside.)
             const int je = min(n32, min(mask_run(m.zero, js), mask_run(m.inside, js)));
             if ((m.zero >> js) & 1u) {
               js = je;
@@ -873,16 +872,34 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
           }
         }
       } else if constexpr (F32) {
-        // ζ passes, FP32 Winckelmans: by runs of blocks, masked where the boxes intersect.
+        // ζ passes, FP32.
         const float4* ta = reinterpret_cast<const float4*>(tileA);
         const float4* tb = reinterpret_cast<const float4*>(tileB);
         const float4* tc = reinterpret_cast<const float4*>(tileC);
         const float4* td = reinterpret_cast<const float4*>(PASS == PASS_ZETAD ? tileD : tileC);
         constexpr bool DD = PASS == PASS_ZETAD;
-        const uint32_t cls = overlap_codes<BLOCK / 32>(ovl, 1u);
+        // Winckelmans by runs of blocks, masked where the boxes intersect; Gaussian-erf
+        // by runs of sources, skipped where ζ is zero and masked inside the target box.
+        [[maybe_unused]] uint32_t cls = 0;
+        [[maybe_unused]] SourceMasks m;
+        if constexpr (KERNEL == VPM_KERNEL_WINCKELMANS) cls = overlap_codes<BLOCK / 32>(ovl, 1u);
         for (int js = 0; js < cnt;) {
-          const int je = block_run_end(cls, js, cnt, [](uint32_t c) { return c; });
-          if ((ovl >> (js >> 5)) & 1u) {
+          int je;
+          bool inside;
+          if constexpr (KERNEL == VPM_KERNEL_WINCKELMANS) {
+            je = block_run_end(cls, js, cnt, [](uint32_t c) { return c; });
+            inside = (ovl >> (js >> 5)) & 1u;
+          } else {
+            const int b = js & 31;
+            if (b == 0) m = zeta_masks(tbox + 2 * warp, ta[js + (tid & 31)], use_far);
+            je = min(cnt, js - b + min(mask_run(m.zero, b), mask_run(m.inside, b)));
+            inside = (m.inside >> b) & 1u;
+            if ((m.zero >> b) & 1u) {
+              js = je;
+              continue;
+            }
+          }
+          if (inside) {
 #pragma unroll 2
             for (; js < je; ++js)
               zeta_source<KERNEL, T, true, DD, false>(ta[js], tb[js], tc[js], td[js], tx, ty, tz, acc);
