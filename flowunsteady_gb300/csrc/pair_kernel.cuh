@@ -230,7 +230,7 @@ __device__ __forceinline__ int tile_target(int k, int tid) {
 // final, rank r forms the values of the targets [r·per, (r+1)·per) of the
 // tile from every rank's pairs, in rank order, as FP64 sums of each rank's
 // hi + lo (the partial-slot form sums the same pairs as a double-float).
-template <int PASS, int KERNEL, int PREC, int BLOCK, int T>
+template <int PASS, int KERNEL, int PREC, int BLOCK, int T, bool RUNS>
 __device__ __forceinline__ void cluster_epilogue(const PairArgs& a, const float* fold_hi,
                                               const float* fold_lo, int64_t t0, int64_t t1) {
   using Tr = PairTraits<PASS, PREC>;
@@ -243,7 +243,6 @@ __device__ __forceinline__ void cluster_epilogue(const PairArgs& a, const float*
   for (int t = int(rank) * per + tid; t < tend; t += BLOCK) {
     const int64_t i = t0 + t;
     if (i >= t1) break;
-    constexpr bool RUNS = Tr::template kWarpRuns<KERNEL>;
     const int k = RUNS ? t / 32 % T : t / BLOCK;
     const int j = RUNS ? t / (32 * T) * 32 + t % 32 : t % BLOCK;
     // Rank q's value w, as the partial-slot epilogue forms it.
@@ -353,8 +352,9 @@ __device__ __noinline__ void tile_reduce(const PairArgs& a, int64_t t0, int64_t 
 }
 
 // CLU: the split-source cluster form (FP32C only; launched with a cluster
-// dimension of a.cluster CTAs, one item per CTA).
-template <int PASS, int KERNEL, int PREC, int BLOCK, int T, bool CLU = false>
+// dimension of a.cluster CTAs, one item per CTA).  STRIDED: a warp's targets a block
+// apart (see launch).
+template <int PASS, int KERNEL, int PREC, int BLOCK, int T, bool CLU = false, bool STRIDED = false>
 __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
     pair_kernel(const PairArgs a) {
   static_assert(!CLU || PREC == VPM_PREC_FP32C, "the cluster form sums compensated pairs");
@@ -407,9 +407,9 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
   constexpr bool kFarKernel = F32 && KERNEL == VPM_KERNEL_GAUSSIANERF;
   const bool use_far = kFarKernel && a.far != 0;
   const int warp = tid >> 5;
-  constexpr bool RUNS = Tr::template kWarpRuns<KERNEL>;
-  // Source boxes serve the block-wise masks of the passes without RUNS only.
-  constexpr bool kBoxes = F32 && !RUNS;
+  constexpr bool RUNS = Tr::template kWarpRuns<KERNEL> && !STRIDED;
+  // Source boxes serve the block-wise masks of the Winckelmans passes only.
+  constexpr bool kBoxes = F32 && !Tr::template kWarpRuns<KERNEL>;
   uint32_t phase = 0;
   if (use_tma) {
     if (tid == 0) mbar_init(bar, 1);
@@ -969,7 +969,7 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
     if constexpr (CLU) {
       // Every rank's (hi, lo) pairs are final after the first barrier.
       cluster_sync_all();
-      if (!aborted) cluster_epilogue<PASS, KERNEL, PREC, BLOCK, T>(a, fold_hi, fold_lo, t0, t1);
+      if (!aborted) cluster_epilogue<PASS, KERNEL, PREC, BLOCK, T, RUNS>(a, fold_hi, fold_lo, t0, t1);
       cluster_sync_all();   // remote reads done before any CTA leaves
       return;
     }
@@ -1128,30 +1128,41 @@ __global__ void __launch_bounds__(reduce_threads(nval_of(PASS), SEGS),
 // ---------------------------------------------------------------- dispatch --
 typedef void (*PairFn)(const PairArgs);
 
-template <int PASS, int KERNEL, int PREC, int BLOCK, int T, bool CLU = false>
+template <int PASS, int KERNEL, int PREC, int BLOCK, int T, bool CLU = false, bool STRIDED = false>
 PairFn fn_ready() {
   static bool once = [] {
-    cudaFuncSetAttribute(pair_kernel<PASS, KERNEL, PREC, BLOCK, T, CLU>,
+    cudaFuncSetAttribute(pair_kernel<PASS, KERNEL, PREC, BLOCK, T, CLU, STRIDED>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                          int(smem_bytes<PASS, KERNEL, PREC>(BLOCK, T)));
     // Clusters of up to 16 CTAs (beyond the portable 8) for the split-source form.
     if (CLU)
-      cudaFuncSetAttribute(pair_kernel<PASS, KERNEL, PREC, BLOCK, T, CLU>,
+      cudaFuncSetAttribute(pair_kernel<PASS, KERNEL, PREC, BLOCK, T, CLU, STRIDED>,
                            cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     return true;
   }();
   (void)once;
-  return pair_kernel<PASS, KERNEL, PREC, BLOCK, T, CLU>;
+  return pair_kernel<PASS, KERNEL, PREC, BLOCK, T, CLU, STRIDED>;
+}
+
+// The same with a warp's targets a block apart where `strided` asks for it: the FP32
+// Gaussian-erf U/J passes at the shape that small fields take.
+template <int PASS, int KERNEL, int PREC, int BLOCK, int T, bool CLU = false>
+PairFn fn_of(bool strided) {
+  if constexpr (PairTraits<PASS, PREC>::kUJ && KERNEL == VPM_KERNEL_GAUSSIANERF &&
+                PREC != VPM_PREC_FP64 && BLOCK == 128 && T == 2) {
+    if (strided) return fn_ready<PASS, KERNEL, PREC, BLOCK, T, CLU, true>();
+  }
+  return fn_ready<PASS, KERNEL, PREC, BLOCK, T, CLU>();
 }
 
 // Compiled shapes: FP64 {128x1}; FP32 and FP32C {128x2, 128x4, 256x2}.
 template <int PASS, int KERNEL, int PREC>
-PairFn pick(Shape s) {
+PairFn pick(Shape s, bool strided) {
   if constexpr (PREC == VPM_PREC_FP64) {
     if (s.block == 128 && s.tpt == 1) return fn_ready<PASS, KERNEL, PREC, 128, 1>();
     return nullptr;
   } else {
-    if (s.block == 128 && s.tpt == 2) return fn_ready<PASS, KERNEL, PREC, 128, 2>();
+    if (s.block == 128 && s.tpt == 2) return fn_of<PASS, KERNEL, PREC, 128, 2>(strided);
     if (s.block == 128 && s.tpt == 4) return fn_ready<PASS, KERNEL, PREC, 128, 4>();
     if (s.block == 256 && s.tpt == 2) return fn_ready<PASS, KERNEL, PREC, 256, 2>();
     return nullptr;
@@ -1159,36 +1170,36 @@ PairFn pick(Shape s) {
 }
 
 template <int PASS, int KERNEL>
-PairFn pick_prec(int prec, Shape s) {
+PairFn pick_prec(int prec, Shape s, bool strided) {
   switch (prec) {
-    case VPM_PREC_FP64: return pick<PASS, KERNEL, VPM_PREC_FP64>(s);
-    case VPM_PREC_FP32: return pick<PASS, KERNEL, VPM_PREC_FP32>(s);
-    case VPM_PREC_FP32C: return pick<PASS, KERNEL, VPM_PREC_FP32C>(s);
+    case VPM_PREC_FP64: return pick<PASS, KERNEL, VPM_PREC_FP64>(s, strided);
+    case VPM_PREC_FP32: return pick<PASS, KERNEL, VPM_PREC_FP32>(s, strided);
+    case VPM_PREC_FP32C: return pick<PASS, KERNEL, VPM_PREC_FP32C>(s, strided);
   }
   return nullptr;
 }
 
 template <int PASS>
-PairFn pick_kernel(int kernel, int prec, Shape s) {
-  return kernel == VPM_KERNEL_WINCKELMANS ? pick_prec<PASS, VPM_KERNEL_WINCKELMANS>(prec, s)
-                                          : pick_prec<PASS, VPM_KERNEL_GAUSSIANERF>(prec, s);
+PairFn pick_kernel(int kernel, int prec, Shape s, bool strided = false) {
+  return kernel == VPM_KERNEL_WINCKELMANS ? pick_prec<PASS, VPM_KERNEL_WINCKELMANS>(prec, s, strided)
+                                          : pick_prec<PASS, VPM_KERNEL_GAUSSIANERF>(prec, s, strided);
 }
 
 // The cluster form of an FP32C shape (null for other precisions and shapes).
 template <int PASS, int KERNEL>
-PairFn pick_cluster_k(Shape s) {
+PairFn pick_cluster_k(Shape s, bool strided) {
   constexpr int P = VPM_PREC_FP32C;
-  if (s.block == 128 && s.tpt == 2) return fn_ready<PASS, KERNEL, P, 128, 2, true>();
+  if (s.block == 128 && s.tpt == 2) return fn_of<PASS, KERNEL, P, 128, 2, true>(strided);
   if (s.block == 128 && s.tpt == 4) return fn_ready<PASS, KERNEL, P, 128, 4, true>();
   if (s.block == 256 && s.tpt == 2) return fn_ready<PASS, KERNEL, P, 256, 2, true>();
   return nullptr;
 }
 
 template <int PASS>
-PairFn pick_cluster(int kernel, int prec, Shape s) {
+PairFn pick_cluster(int kernel, int prec, Shape s, bool strided = false) {
   if (prec != VPM_PREC_FP32C) return nullptr;
-  return kernel == VPM_KERNEL_WINCKELMANS ? pick_cluster_k<PASS, VPM_KERNEL_WINCKELMANS>(s)
-                                          : pick_cluster_k<PASS, VPM_KERNEL_GAUSSIANERF>(s);
+  return kernel == VPM_KERNEL_WINCKELMANS ? pick_cluster_k<PASS, VPM_KERNEL_WINCKELMANS>(s, strided)
+                                          : pick_cluster_k<PASS, VPM_KERNEL_GAUSSIANERF>(s, strided);
 }
 
 template <int PASS>
@@ -1235,15 +1246,20 @@ inline cudaLaunchConfig_t cluster_config(int grid, int block, size_t smem, cudaS
 template <int PASS>
 cudaError_t launch(int kernel, int precision, Shape s, const PairArgs& a, int grid,
                    cudaStream_t st) {
-  PairFn f = pick_kernel<PASS>(kernel, precision, s);
+  // At one CTA per SM or less a launch lasts as long as its slowest warp.  The sources of
+  // a chunk near its own targets take the series; with consecutive targets per warp they
+  // are all one warp's, with strided ones they are shared: U/J of 50 to 2,000 particles
+  // 3 to 4 µs shorter.  In a longer launch the SMs are full and compact warps win.
+  const bool strided = !a.items && grid <= 152;
+  PairFn f = pick_kernel<PASS>(kernel, precision, s, strided);
   if (!f) return cudaErrorInvalidConfiguration;
   if (grid <= 0) return cudaSuccess;
-  // The Gaussian-erf ζ passes read nothing but records.
+  // The ζ passes that stage per warp read nothing but records.
   if (precision != VPM_PREC_FP64 && (PASS == PASS_ZETA || PASS == PASS_ZETAD) && !a.rec)
     return cudaErrorInvalidValue;
   if (a.cluster > 1) {
     // One item per CTA, every CTA of a cluster on the same target tile.
-    f = pick_cluster<PASS>(kernel, precision, s);
+    f = pick_cluster<PASS>(kernel, precision, s, strided);
     if (!f || a.items || a.counter || grid % a.cluster != 0 ||
         int64_t(grid) != int64_t(a.n_tb) * a.n_chunk || a.n_chunk != a.cluster)
       return cudaErrorInvalidConfiguration;
