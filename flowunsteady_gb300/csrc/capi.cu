@@ -292,7 +292,7 @@ cudaError_t run_pair(const PairCall& pc, int device, int num_sms, const Shape* p
   plan.post = pc.post && plan.slots() > 1 && !plan.fused && pc.t0 == 0 && nt == pc.ns &&
               nt <= kPostInReduce;
   const int nv = nval_of(pc.pass);
-  if (pc.pass == PASS_UJ && plan.slots() >= kSegSlots && nt <= kSegTargets * num_sms)
+  if (pc.pass == PASS_UJ && !plan.fused && plan.slots() >= kSegSlots && nt <= kSegTargets * num_sms)
     plan.segs = kReduceSegs;
   const size_t slot_elems = plan.slots() > 1 ? size_t(plan.slots()) * nv * size_t(ldp) : 0;
   // One 32-bit counter per target tile after the slots (two per double).
@@ -309,7 +309,7 @@ cudaError_t run_pair(const PairCall& pc, int device, int num_sms, const Shape* p
   a.fd_alpha = pc.fd_alpha;
   a.dj = pc.dj;
   a.t_off = pc.t0; a.nt = nt; a.ns = pc.ns; a.chunk = chunk;
-  a.n_tb = int(n_tb); a.n_chunk = n_chunk; a.segs = plan.segs;
+  a.n_tb = int(n_tb); a.n_chunk = n_chunk;
   a.items = nullptr; a.n_items = 0; a.counter = nullptr;
   a.u = pc.u; a.j = pc.j; a.ldo = pc.ldo;
   a.part = part; a.ldp = ldp;
@@ -990,7 +990,8 @@ static cudaError_t enqueue_passes(vpm_ctx* c, const vpm_scheme* s, int stage, in
   const bool fd = dyn0;
   PostArgs p = base;
   p.flags = sfs ? POST_STRETCH | zeta_rec : tail;
-  c->fine = !sfs;   // (finite-difference C_d would amplify another rounding)
+  // (A finite-difference C_d or the relaxation would amplify another rounding.)
+  c->fine = !sfs && s->relaxation == VPM_RELAX_NONE;
   const cudaError_t e = pass_then(c, K, p, sfs ? (recs ? PASS_ZETA : -1) : tail_rec,
                                   [&] { return uj_pass(c, s, fd); });
   c->fine = false;
@@ -1192,7 +1193,6 @@ int vpm_ctx_create(int device, int64_t capacity, vpm_ctx** out) {
   if (e == cudaSuccess) e = cudaMemset(c->stat, 0, size_t(c->ld));
   // Packed source records: 3 float4 per particle for the U/J passes, up to 5 for ζ.
   if (e == cudaSuccess) e = cudaMalloc(&c->rec, 5 * ld * sizeof(float4));
-  // Until the first packing the particle order counts as coherent.
   if (e == cudaSuccess) e = cudaMalloc(&c->status, sizeof(int));
   if (e == cudaSuccess) e = cudaMemset(c->status, 0, sizeof(int));
   if (e == cudaSuccess) e = cudaMalloc(&c->red, (size_t(kRedBlocks) + 1) * kDiagSlots * sizeof(double));

@@ -54,7 +54,6 @@ struct PairArgs {
   // Decomposition without a table: targets [t_off, t_off+nt) x sources [0, ns).
   int64_t t_off, nt, ns, chunk;
   int32_t n_tb, n_chunk;
-  int32_t segs;   // runs that the slots of a target are summed in
   // Decomposition from a table (batches): n_items entries, dynamic queue when
   // counter != null.
   const PairItem* items;

@@ -183,10 +183,9 @@ struct PairSum {
   __device__ __forceinline__ double value() const { return double(s) + double(c); }
 };
 
-// The slots of a target are summed in PairArgs::segs runs of consecutive slots, each in
-// slot order, and the runs in order; every form of the sum takes the same runs.
+// First slot of run `seg` of `segs` runs of consecutive slots (reduce_kernel).
 __host__ __device__ inline int seg_begin(int nc, int seg, int segs) {
-  return nc / segs * seg + nc % segs * seg / segs;   // (a 64-bit product and division spill)
+  return int(int64_t(nc) * seg / segs);
 }
 
 // FP32 U/J passes: the Gaussian-erf A sums carry a scale, and A22 (DA22) is not
@@ -304,34 +303,22 @@ __device__ __noinline__ void tile_reduce(const PairArgs& a, int64_t t0, int64_t 
     double v[NV];
 #pragma unroll
     for (int w0 = 0; w0 < NV; w0 += G) {
-      using Sum = typename std::conditional<F2, PairSum, double>::type;
-      Sum all[G] = {};
-      const int segs = PASS == PASS_UJ ? a.segs : 1;
-      for (int seg = 0; seg < segs; ++seg) {
-        Sum s[G] = {};
-        const int c1 = seg_begin(a.n_chunk, seg + 1, segs);
-        int c = seg_begin(a.n_chunk, seg, segs);
-        const double* p = a.part + int64_t(w0) * a.ldp + i + int64_t(c) * step;
+      typename std::conditional<F2, PairSum, double>::type s[G] = {};
+      const double* p = a.part + int64_t(w0) * a.ldp + i;
 #pragma unroll 2
-        for (; c < c1; ++c, p += step) {
-#pragma unroll
-          for (int g = 0; g < G; ++g) {
-            if (w0 + g >= NV) continue;
-            if constexpr (F2) s[g].add(__ldcg(reinterpret_cast<const float2*>(p + int64_t(g) * a.ldp)));
-            else s[g] += __ldcg(p + int64_t(g) * a.ldp);
-          }
-        }
+      for (int c = 0; c < a.n_chunk; ++c, p += step) {
 #pragma unroll
         for (int g = 0; g < G; ++g) {
-          if constexpr (F2) all[g].add(make_float2(s[g].s, s[g].c));
-          else all[g] += s[g];
+          if (w0 + g >= NV) continue;
+          if constexpr (F2) s[g].add(__ldcg(reinterpret_cast<const float2*>(p + int64_t(g) * a.ldp)));
+          else s[g] += __ldcg(p + int64_t(g) * a.ldp);
         }
       }
 #pragma unroll
       for (int g = 0; g < G; ++g)
         if (w0 + g < NV) {
-          if constexpr (F2) v[w0 + g] = all[g].value();
-          else v[w0 + g] = all[g];
+          if constexpr (F2) v[w0 + g] = s[g].value();
+          else v[w0 + g] = s[g];
         }
     }
     if constexpr (F2) finish_f32_sums<PASS, KERNEL>(v);
@@ -1043,8 +1030,8 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
 // values (y) times SEGS runs of slots (z): thread (x, y, z) sums its run in slot order,
 // kReduceLoads slots loaded ahead, and one thread per target adds the runs in order and
 // forms the final values from shared memory.  F2: the FP32 passes' float-pair slots,
-// summed with PairSum; otherwise FP64 slots and FP64 additions.  tile_reduce adds in
-// the same order.
+// summed with PairSum; otherwise FP64 slots and FP64 additions.  With one run tile_reduce
+// adds in the same order.
 //   SEGS 1, COLS 32: a field of many blocks, bound by reading the slots.
 //   SEGS 4, COLS 16 (U/J, kReduceSegs): few targets with many slots each, where one thread
 //   per value would walk them alone.
@@ -1246,11 +1233,12 @@ inline cudaLaunchConfig_t cluster_config(int grid, int block, size_t smem, cudaS
 template <int PASS>
 cudaError_t launch(int kernel, int precision, Shape s, const PairArgs& a, int grid,
                    cudaStream_t st) {
-  // At one CTA per SM or less a launch lasts as long as its slowest warp.  The sources of
-  // a chunk near its own targets take the series; with consecutive targets per warp they
-  // are all one warp's, with strided ones they are shared: U/J of 50 to 2,000 particles
-  // 3 to 4 µs shorter.  In a longer launch the SMs are full and compact warps win.
-  const bool strided = !a.items && grid <= 152;
+  // A launch of a wave or two lasts as long as its slowest warps.  The sources of a chunk
+  // near its own targets take the series; with consecutive targets per warp they are all
+  // one warp's, with strided ones they are shared: U/J of 50 to 2,000 particles 3 to 4 µs
+  // shorter, a dynamic-SFS step of 4,000 / 6,000 322 -> 312 / 473 -> 460 µs.  In a longer
+  // launch the SMs are full and compact warps win (U/J of 20,000: 597 -> 560 µs).
+  const bool strided = !a.items && grid <= 10 * 152;
   PairFn f = pick_kernel<PASS>(kernel, precision, s, strided);
   if (!f) return cudaErrorInvalidConfiguration;
   if (grid <= 0) return cudaSuccess;

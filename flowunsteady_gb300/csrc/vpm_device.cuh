@@ -492,9 +492,9 @@ constexpr double kGaussAScale = -3.0;
 // All T targets take the erf-free form, and a warp vote sends the rare warps
 // holding a pair with ρ² < 3/2 (or the self pair) through the series.  With
 // VOTE, a first warp vote takes the far form (q = 1/r³, p = -3/r⁵; see the
-// far-field notes below) when every pair of the warp has ρ² >= 50; the caller
-// uses it only for warps whose targets are compact enough for the vote to pay
-// (it splits the straight-line code that overlaps the exp/rcp latencies).
+// far-field notes below) when every pair of the warp has ρ² >= 50 (the
+// treecode's near field; it splits the straight-line code that overlaps the
+// exp/rcp latencies).
 template <int T, bool VOTE>
 __device__ __forceinline__ void uj_source_gauss(const float4 sa, const float4 sb,
                                                 const float (&tx)[T], const float (&ty)[T],
@@ -1108,29 +1108,6 @@ __device__ __forceinline__ void ujd_source_gauss_far(const float4 sa, const floa
     const float p = q * ri2;
     const float k3e = k3 * ex2_ftz(r2 * ea);
     accum_pair_d(dx, dy, dz, q, p, -k3e, k3e * is2, sb.x, sb.y, sb.z, acc[k]);
-  }
-}
-
-// FP64 α-derivatives of one pair (zero when r² == 0).
-//   Winckelmans: a = σ², b = 3/2 σ²;  Gaussian-erf: a = 1/σ², b = 1/σ.
-template <int KERNEL>
-__device__ inline void pair_dqp_f64(double r2, double a, double b, double& dq, double& dp) {
-  if (KERNEL == VPM_KERNEL_WINCKELMANS) {
-    const double s = r2 + a;
-    const double rs = rsqrt(s);
-    const double rs2 = rs * rs;
-    const double rs7 = rs2 * rs2 * rs2 * rs;
-    dq = -7.5 * a * a * rs7;
-    dp = -17.5 * a * a * rs7 * rs2;
-  } else {
-    const double e = exp(-0.5 * r2 * a);
-    const double k3 = kSqrt2overPi * b * b * b;
-    dq = -k3 * e;
-    dp = k3 * e * a;
-  }
-  if (!(r2 > 0.0)) {
-    dq = 0.0;
-    dp = 0.0;
   }
 }
 
