@@ -153,11 +153,12 @@ __device__ __forceinline__ double exp2_f64(double r2, double a2048, const double
   const double v = __hiloint2double(__double2hiint(s) + (low ? ex + 128 : ex) * (1 << 20),
                                     __double2loint(s));
   const double r = fma(v, g, v);
-  // The high word of t is that of 1.5·2^52 or one less for -2^32 <= n <= 0 (a low word
-  // above 0 is an n below -2^31); larger for NaN, whose low word is 0.
+  // In range are n = 0 .. -2^31: the high word of t is that of 1.5·2^52 at n = 0 and one
+  // less below it, where the low word is n itself (above 0 for n < -2^31, and 0 again,
+  // with that lower high word, at n = -2^32).  A NaN is out of range: 0, as for r = 0.
   // A vote, so that the product by 2^-128 is not formed for every pair (an FP64 ring step
   // 22.2 -> 21.6 ms): all 32 lanes call this together.
-  const bool in = __double2hiint(t) >= 0x4337ffff && n <= 0;
+  const bool in = n <= 0 && __double2hiint(t) == 0x43380000 + (n >> 31);
   if (!__any_sync(0xffffffffu, low || !in)) return r;
   if (!in || ex < -1100) return 0.0;
   return low ? r * 0x1p-128 : r;
