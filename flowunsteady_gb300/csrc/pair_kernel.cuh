@@ -202,20 +202,16 @@ __device__ __forceinline__ void finish_f32_sums(double* v) {
   }
 }
 
-// FP64 U/J passes: likewise, Gaussian-erf A sums hold p/(-3).
+// FP64 U/J passes: likewise, Gaussian-erf A sums hold p/(-3).  (All nine are summed.)
 template <int PASS, int KERNEL>
 __device__ __forceinline__ void finish_f64_sums(double* v, bool fd) {
-  if constexpr (PASS == PASS_UJ || PASS == PASS_UJD) {
-    if constexpr (KERNEL == VPM_KERNEL_GAUSSIANERF) {
+  if constexpr ((PASS == PASS_UJ || PASS == PASS_UJD) && KERNEL == VPM_KERNEL_GAUSSIANERF) {
 #pragma unroll
-      for (int w = 3; w < 11; ++w) v[w] *= -3.0;
-      if (PASS == PASS_UJD && fd) {   // differences of the same sums
+    for (int w = 3; w < 12; ++w) v[w] *= -3.0;
+    if (PASS == PASS_UJD && fd) {   // differences of the same sums
 #pragma unroll
-        for (int w = 15; w < 23; ++w) v[w] *= -3.0;
-      }
+      for (int w = 15; w < 24; ++w) v[w] *= -3.0;
     }
-    v[11] = -(v[3] + v[7]);
-    if constexpr (PASS == PASS_UJD) v[23] = -(v[15] + v[19]);
   }
 }
 
@@ -852,7 +848,7 @@ __global__ void __launch_bounds__(BLOCK, (min_blocks<PASS, PREC, BLOCK, T>()))
                 const R e0 = dp * c0, e1 = dp * c1, e2 = dp * c2;
                 acc[k][15] += e0 * dx; acc[k][16] += e0 * dy; acc[k][17] += e0 * dz;
                 acc[k][18] += e1 * dx; acc[k][19] += e1 * dy; acc[k][20] += e1 * dz;
-                acc[k][21] += e2 * dx; acc[k][22] += e2 * dy;
+                acc[k][21] += e2 * dx; acc[k][22] += e2 * dy; acc[k][23] += e2 * dz;
                 acc[k][24] += dq * gx; acc[k][25] += dq * gy; acc[k][26] += dq * gz;
               }
             }
