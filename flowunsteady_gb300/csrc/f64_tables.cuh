@@ -18,6 +18,12 @@
 // Exponential.  2^(i/2048), i = 0..2047, from the double-double Taylor series.
 #pragma once
 
+#ifdef __CUDACC__
+#define VPM_HOST_DEVICE __host__ __device__
+#else   // the tables and tests on words are plain C++ for a host compiler
+#define VPM_HOST_DEVICE
+#endif
+
 namespace vpm {
 
 struct DD {   // hi + lo
@@ -50,6 +56,11 @@ constexpr DD dd_div(DD a, double b) {
 constexpr int kCoreRows = 721;    // x_i = 0, 1/8, .., 90
 constexpr int kCoreCoef = 8;
 constexpr int kExp2Rows = 2048;
+
+// Whether u = x/2, given by its high word, is below 45, the end of the core table.  As an
+// unsigned number, so that everything with a sign, a NaN's among it (CUDA's own is
+// 0xfff8000000000000), is past the end: the low word of a NaN would be the index.
+VPM_HOST_DEVICE constexpr bool core_near_word(unsigned hi) { return hi < 0x40468000u; }
 
 struct CoreTable {
   double v[kCoreRows * kCoreCoef];

@@ -114,8 +114,10 @@ __device__ __forceinline__ double core_f1(double u, const double* __restrict__ t
   return b;
 }
 
-// u = x/2 below kFarRho2D/2 = 45 (u >= 0; NaN counts as far): by the high words.
-__device__ __forceinline__ bool core_is_near(double u) { return __double2hiint(u) < 0x40468000; }
+// u = x/2 below kFarRho2D/2 = 45 (u >= 0; any NaN counts as far): by the high words.
+__device__ __forceinline__ bool core_is_near(double u) {
+  return core_near_word(unsigned(__double2hiint(u)));
+}
 
 // q = g/r³ and p/(-3), p = q'/r, of a Gaussian-erf pair; h2 = 1/(2σ²), c3 = 1/σ³,
 // c5 = 1/(3σ⁵).  The pair is dropped when r² == 0.
