@@ -157,18 +157,17 @@ size_t ffv_plan(int64_t nb, int64_t nf, int num_sms, int64_t* chunk, int* n_chun
 }
 
 template <int KERNEL>
-void ffv_start(int grid, int64_t nb, const double* xb, const double* gb, const double* sb,
-               int64_t ldb, int64_t nf, const double* xf, const double* gf, int64_t ldf,
-               int64_t chunk, int n_tb, double* part, double* M, int64_t ldm, int n_chunk,
-               cudaStream_t st) {
+cudaError_t ffv_start(int grid, int64_t nb, const double* xb, const double* gb, const double* sb,
+                      int64_t ldb, int64_t nf, const double* xf, const double* gf, int64_t ldf,
+                      int64_t chunk, int n_tb, double* part, double* M, int64_t ldm, int n_chunk,
+                      cudaStream_t st) {
   const size_t smem = KERNEL == VPM_KERNEL_GAUSSIANERF ? sizeof(CoreTable) : 0;
-  static const bool once = [smem] {
-    cudaFuncSetAttribute(ffv_kernel<KERNEL>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
-    return true;
-  }();
-  (void)once;
+  static PerContext done;
+  const cudaError_t e = allow_smem(done, ffv_kernel<KERNEL>, smem);
+  if (e != cudaSuccess) return e;
   ffv_kernel<KERNEL><<<grid, kFfvBlock, smem, st>>>(nb, xb, gb, sb, ldb, nf, xf, gf, ldf, chunk,
                                                     n_tb, part, M, ldm, n_chunk);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_ffv(int kernel, int64_t nb, const double* xb, const double* gb,
@@ -181,13 +180,10 @@ cudaError_t launch_ffv(int kernel, int64_t nb, const double* xb, const double* g
   ffv_plan(nb, nf, num_sms, &chunk, &n_chunk);
   const int n_tb = int(ceil_div(nb, kFfvBlock));
   const int grid = n_tb * n_chunk;
-  if (kernel == VPM_KERNEL_WINCKELMANS)
-    ffv_start<VPM_KERNEL_WINCKELMANS>(grid, nb, xb, gb, sb, ldb, nf, xf, gf, ldf, chunk, n_tb, part,
-                                      M, ldm, n_chunk, st);
-  else
-    ffv_start<VPM_KERNEL_GAUSSIANERF>(grid, nb, xb, gb, sb, ldb, nf, xf, gf, ldf, chunk, n_tb, part,
-                                      M, ldm, n_chunk, st);
-  cudaError_t e = cudaGetLastError();
+  auto start = kernel == VPM_KERNEL_WINCKELMANS ? ffv_start<VPM_KERNEL_WINCKELMANS>
+                                                : ffv_start<VPM_KERNEL_GAUSSIANERF>;
+  const cudaError_t e = start(grid, nb, xb, gb, sb, ldb, nf, xf, gf, ldf, chunk, n_tb, part, M, ldm,
+                              n_chunk, st);
   if (e != cudaSuccess || n_chunk <= 1) return e;
   ffv_reduce_kernel<<<int(ceil_div(nb, kFfvRed)), dim3(kFfvRed, kFfvNval, kFfvSegs), 0, st>>>(
       nb, gb, ldb, part, n_chunk, M, ldm);

@@ -5,6 +5,7 @@
 #include <stdint.h>
 
 #include "../../include/vpm_gpu.h"
+#include "per_context.h"
 
 namespace vpm {
 
@@ -104,6 +105,28 @@ struct Shape {
   int block;   // threads per CTA
   int tpt;     // targets per thread
 };
+
+// Unique id of the current driver context (0 when none is current or the driver entry
+// points are unavailable).  A context replaced by cudaDeviceReset gets a new id.
+unsigned long long current_context_id();
+
+// Gives `kernel` `smem` bytes of dynamic shared memory (and cluster sizes above 8) in
+// every context it is launched in; the same bytes on every call with one `done`.
+template <class Kernel>
+cudaError_t allow_smem(PerContext& done, Kernel kernel, size_t smem, bool clusters = false) {
+  // Launches below the limit of every kernel (48 KB with their static arrays) need nothing.
+  if (smem <= 40 * 1024 && !clusters) return cudaSuccess;
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess) dev = -1;
+  const int e = done.ensure(dev, current_context_id(), [&] {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
+    if (e == cudaSuccess && clusters)
+      e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) cudaGetLastError();   // reported by the caller
+    return int(e);
+  });
+  return cudaError_t(e);
+}
 
 // Launch one pair pass (grid chosen by the caller through args/n_items).
 cudaError_t launch_pair(int pass, int kernel, int precision, Shape shape, const PairArgs& a,

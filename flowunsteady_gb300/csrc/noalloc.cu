@@ -31,25 +31,7 @@
 
 using namespace vpm;
 
-namespace {
-
-// Partial sums of a split source range: n_chunk x 15 FP64 values per target.
-constexpr int64_t kScratchDoubles = int64_t(1) << 19;          // 4 MiB
-// Largest target count accepted: two source chunks of 15 values per target fit.
-constexpr int64_t kMaxTargets = 16384;
-static_assert((2 * kNvalUJ + 1) * kMaxTargets <= kScratchDoubles, "scratch too small");
-
-static __device__ __align__(256) double g_uj_scratch[kScratchDoubles];
-
-constexpr int kMaxDevices = 64;
-std::mutex g_mu;
-double* g_scratch_addr[kMaxDevices] = {};
-unsigned long long g_scratch_ctx[kMaxDevices] = {};   // context id the address belongs to
-
-// Unique id of the current driver context (0 when none is current or the
-// driver entry points are unavailable).  A context replaced by
-// cudaDeviceReset gets a new id, so a cached symbol address is re-checked.
-unsigned long long current_context_id() {
+unsigned long long vpm::current_context_id() {
   typedef CUresult (*GetCurrent)(CUcontext*);
   typedef CUresult (*GetId)(CUcontext, unsigned long long*);
   static GetCurrent get_current = nullptr;
@@ -74,8 +56,23 @@ unsigned long long current_context_id() {
   return id;
 }
 
+namespace {
+
+// Partial sums of a split source range: n_chunk x 15 FP64 values per target.
+constexpr int64_t kScratchDoubles = int64_t(1) << 19;          // 4 MiB
+// Largest target count accepted: two source chunks of 15 values per target fit.
+constexpr int64_t kMaxTargets = 16384;
+static_assert((2 * kNvalUJ + 1) * kMaxTargets <= kScratchDoubles, "scratch too small");
+
+static __device__ __align__(256) double g_uj_scratch[kScratchDoubles];
+
+std::mutex g_mu;
+double* g_scratch_addr[kMaxDevices] = {};
+unsigned long long g_scratch_ctx[kMaxDevices] = {};   // context id the address belongs to
+
 // Device address of g_uj_scratch on the current device `dev`: looked up once
-// per device context, with the device current.
+// per device context, with the device current (a context replaced by cudaDeviceReset
+// has another id).
 int scratch_address(int dev, double** out) {
   if (dev < 0 || dev >= kMaxDevices)
     return set_error(nullptr, VPM_ERR_UNSUPPORTED, "device index too large for the static scratch table");

@@ -1111,20 +1111,13 @@ __global__ void __launch_bounds__(reduce_threads(nval_of(PASS), SEGS),
 // ---------------------------------------------------------------- dispatch --
 typedef void (*PairFn)(const PairArgs);
 
+// The kernel, ready to be launched in the current context (null: it cannot be made so).
 template <int PASS, int KERNEL, int PREC, int BLOCK, int T, bool CLU = false, bool STRIDED = false>
 PairFn fn_ready() {
-  static bool once = [] {
-    cudaFuncSetAttribute(pair_kernel<PASS, KERNEL, PREC, BLOCK, T, CLU, STRIDED>,
-                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(smem_bytes<PASS, KERNEL, PREC>(BLOCK, T)));
-    // Clusters of up to 16 CTAs (beyond the portable 8) for the split-source form.
-    if (CLU)
-      cudaFuncSetAttribute(pair_kernel<PASS, KERNEL, PREC, BLOCK, T, CLU, STRIDED>,
-                           cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    return true;
-  }();
-  (void)once;
-  return pair_kernel<PASS, KERNEL, PREC, BLOCK, T, CLU, STRIDED>;
+  static PerContext done;
+  const PairFn f = pair_kernel<PASS, KERNEL, PREC, BLOCK, T, CLU, STRIDED>;
+  // Clusters of up to 16 CTAs (beyond the portable 8) for the split-source form.
+  return allow_smem(done, f, smem_bytes<PASS, KERNEL, PREC>(BLOCK, T), CLU) == cudaSuccess ? f : nullptr;
 }
 
 // The same with a warp's targets a block apart where `strided` asks for it: the FP32

@@ -1085,17 +1085,15 @@ __global__ void __launch_bounds__(kNearThreads, NearShape<PASS>::kMinBlocks) nea
 }
 
 template <int KERNEL, int PASS>
-void launch_near(int ngroups, int64_t items, const FmmWork* w, const float* vw, int64_t ldv,
-                 int64_t n, unsigned long long* pairs, cudaStream_t st) {
-  static const bool once = [] {
-    cudaFuncSetAttribute(near_tile_kernel<KERNEL, PASS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(NearShape<PASS>::kSmem));
-    return true;
-  }();
-  (void)once;
+cudaError_t launch_near(int ngroups, int64_t items, const FmmWork* w, const float* vw, int64_t ldv,
+                        int64_t n, unsigned long long* pairs, cudaStream_t st) {
+  static PerContext done;
+  const cudaError_t e = allow_smem(done, near_tile_kernel<KERNEL, PASS>, NearShape<PASS>::kSmem);
+  if (e != cudaSuccess) return e;
   near_tile_kernel<KERNEL, PASS><<<int(items), kNearThreads, NearShape<PASS>::kSmem, st>>>(
       ngroups, w->gbase, w->gtot, w->totals, w->near_list, w->rec, vw, ldv, w->near_raw, n,
       w->counters, pairs);
+  return cudaSuccess;   // (a failed launch is the caller's cudaGetLastError)
 }
 
 // Raw sums [K0, K0 + K) of target t of a group: its near items in order, all K loads
@@ -1722,16 +1720,14 @@ int launch_upward(FmmWork* w, int nleaves, int last_gen, bool f64, int64_t ldw, 
 }
 
 template <int P, int Q>
-void launch_m2l(FmmWork* w, int ngroups, int ncells, cudaStream_t st) {
-  static const bool once = [] {
-    cudaFuncSetAttribute(m2l_kernel<P, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         int(M2lShape<P, Q>::kSmem));
-    return true;
-  }();
-  (void)once;
+cudaError_t launch_m2l(FmmWork* w, int ngroups, int ncells, cudaStream_t st) {
+  static PerContext done;
+  const cudaError_t e = allow_smem(done, m2l_kernel<P, Q>, M2lShape<P, Q>::kSmem);
+  if (e != cudaSuccess) return e;
   m2l_kernel<P, Q><<<ngroups, kM2lThreads, M2lShape<P, Q>::kSmem, st>>>(
       ngroups, w->gbase, w->gtot, w->loc_list, w->geom, w->momf, w->ggeom, ncells, w->loc,
       w->counters);
+  return cudaSuccess;   // (a failed launch is the caller's cudaGetLastError)
 }
 
 template <int P>
@@ -1992,10 +1988,11 @@ cudaError_t fmm_eval(vpm_ctx* c, int kernel, int prec, int p, int ncrit, double 
     if (e == cudaSuccess) e = cudaStreamWaitEvent(w->aux[k], w->fork, 0);
   if (e != cudaSuccess) return e;
   stage = "far field";
+  cudaError_t le = cudaSuccess, ne = cudaSuccess;   // of the launches; the streams rejoin in any case
   if (p == 2) launch_far<2>(w, f64, n, ngroups, ncells, ldw, w->aux[0]);
   else if (p == 4) launch_far<4>(w, f64, n, ngroups, ncells, ldw, w->aux[0]);
   else launch_far<6>(w, f64, n, ngroups, ncells, ldw, w->aux[0]);
-  if (local) launch_m2l<4, kLocalOrder>(w, ngroups, ncells, w->aux[1]);
+  if (local) le = launch_m2l<4, kLocalOrder>(w, ngroups, ncells, w->aux[1]);
   if (f64) {
     if (kernel == VPM_KERNEL_WINCKELMANS)
       near_f64_kernel<VPM_KERNEL_WINCKELMANS><<<ngroups, kTreeBlock, 0, st>>>(
@@ -2004,13 +2001,15 @@ cudaError_t fmm_eval(vpm_ctx* c, int kernel, int prec, int p, int ncrit, double 
       near_f64_kernel<VPM_KERNEL_GAUSSIANERF><<<ngroups, kTreeBlock, 0, st>>>(
           ngroups, w->gbase, w->gtot, w->near_list, w->sorted, ldw, w->near_raw, n, w->counters);
   } else if (dj) {
-    launch_near<VPM_KERNEL_GAUSSIANERF, PASS_UJD>(ngroups, items, w, nullptr, 0, n, w->pairs, st);
+    ne = launch_near<VPM_KERNEL_GAUSSIANERF, PASS_UJD>(ngroups, items, w, nullptr, 0, n, w->pairs, st);
   } else if (kernel == VPM_KERNEL_WINCKELMANS) {
-    launch_near<VPM_KERNEL_WINCKELMANS, PASS_UJ>(ngroups, items, w, nullptr, 0, n, w->pairs, st);
+    ne = launch_near<VPM_KERNEL_WINCKELMANS, PASS_UJ>(ngroups, items, w, nullptr, 0, n, w->pairs, st);
   } else {
-    launch_near<VPM_KERNEL_GAUSSIANERF, PASS_UJ>(ngroups, items, w, nullptr, 0, n, w->pairs, st);
+    ne = launch_near<VPM_KERNEL_GAUSSIANERF, PASS_UJ>(ngroups, items, w, nullptr, 0, n, w->pairs, st);
   }
-  const cudaError_t le = launched(2 + local);
+  if (le == cudaSuccess) le = ne;
+  if ((ne = launched(2 + local)) != cudaSuccess) le = ne;
+  else if (le != cudaSuccess) *why = stage;
   // The other streams always rejoin, whatever failed.
   for (int k = 0; k < 2; ++k) {
     cudaError_t je = cudaEventRecord(w->join[k], w->aux[k]);
@@ -2071,17 +2070,19 @@ cudaError_t fmm_zeta(vpm_ctx* c, bool d, const double* vs, const double* ws, dou
   gather_rows_f32_kernel<<<grid, 256, 0, st>>>(n, 3, w->perm, vs, c->ld, w->vw, ldw);
   if (d)
     gather_rows_f32_kernel<<<grid, 256, 0, st>>>(n, 3, w->perm, ws, c->ld, w->vw + 3 * ldw, ldw);
+  cudaError_t ne;
   if (d) {
-    launch_near<VPM_KERNEL_GAUSSIANERF, PASS_ZETAD>(ngroups, items, w, w->vw, ldw, n, nullptr, st);
+    ne = launch_near<VPM_KERNEL_GAUSSIANERF, PASS_ZETAD>(ngroups, items, w, w->vw, ldw, n, nullptr, st);
     zeta_scatter_kernel<12><<<ngroups, kTreeBlock, 0, st>>>(n, ngroups, w->gbase, w->totals,
                                                             w->near_raw, w->perm, out, c->ld);
   } else {
-    launch_near<VPM_KERNEL_GAUSSIANERF, PASS_ZETA>(ngroups, items, w, w->vw, ldw, n, nullptr, st);
+    ne = launch_near<VPM_KERNEL_GAUSSIANERF, PASS_ZETA>(ngroups, items, w, w->vw, ldw, n, nullptr, st);
     zeta_scatter_kernel<6><<<ngroups, kTreeBlock, 0, st>>>(n, ngroups, w->gbase, w->totals,
                                                            w->near_raw, w->perm, out, c->ld);
   }
   c->launches += d ? 4 : 3;
-  return cudaGetLastError();
+  const cudaError_t e = cudaGetLastError();
+  return ne != cudaSuccess ? ne : e;
 }
 
 }  // namespace vpm
