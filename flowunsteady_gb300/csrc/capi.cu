@@ -802,8 +802,7 @@ cudaError_t ctx_pair(vpm_ctx* c, int pass, int kernel, int prec, int64_t t0, int
   pc.u = u; pc.j = j; pc.ldo = c->ld;
   pc.ws = ws; pc.dj = dj;
   pc.status = c->status;
-  const bool packed = c->rec_pass == pass && c->rec_scale == scale;   // by the update before
-  if (!c->dry) c->rec_pass = -1;
+  const bool packed = !c->dry && c->packed.take(pass, scale);   // by the update before
   pc.post = c->post;
   pc.fine = c->fine;
   if (prec != VPM_PREC_FP64 && (pass == PASS_UJ || pass == PASS_UJD)) {
@@ -915,10 +914,7 @@ static cudaError_t pass_then(vpm_ctx* c, int kernel, const PostArgs& p, int rec_
     if (e2 != cudaSuccess) return e2;
     c->launches += 1;
   }
-  if (rec_pass >= 0) {
-    c->rec_pass = rec_pass;
-    c->rec_scale = p.rec_scale;
-  }
+  c->packed.hold(rec_pass, p.rec_scale);
   return cudaSuccess;
 }
 
@@ -1047,7 +1043,7 @@ static cudaError_t enqueue_stage(vpm_ctx* c, const vpm_scheme* s, double dt, dou
 static cudaError_t enqueue_step(vpm_ctx* c, const vpm_scheme* s, double dt, bool relax) {
   static const double A[3] = {0.0, -5.0 / 9.0, -153.0 / 128.0};
   static const double B[3] = {1.0 / 3.0, 15.0 / 16.0, 8.0 / 15.0};
-  c->rec_pass = -1;   // the particles may have changed since the last step
+  const PackedRecords::Scope scope(c->packed);   // the particles may change between calls
   if (s->integration == VPM_INTEGRATION_RK3) {
     for (int st = 0; st < 3; ++st) ENQP(c, enqueue_stage(c, s, dt, A[st], B[st], st));
   } else {
@@ -1061,7 +1057,6 @@ static cudaError_t enqueue_step(vpm_ctx* c, const vpm_scheme* s, double dt, bool
     update_range(c, &nf, &stat);
     ENQ(c, launch_relax(nf, stat, c->ld, c->J, c->G, s->relax_factor, c->st));
   }
-  c->rec_pass = -1;
   return cudaSuccess;
 }
 
@@ -1473,9 +1468,10 @@ int vpm_eval_sfs(vpm_ctx* c, const vpm_scheme* s) {
   enqueue_uj_sfs(c, s, 0);
   c->dry = false;
   if ((rc = ensure_part(c, c->part_need))) return rc;
-  c->rec_pass = -1;
-  CTX_CK(c, enqueue_uj_sfs(c, s, 0));
-  c->rec_pass = -1;
+  {
+    const PackedRecords::Scope scope(c->packed);
+    CTX_CK(c, enqueue_uj_sfs(c, s, 0));
+  }
   if (s->sfs_flags & VPM_SFS_CLIP_BACKSCATTER) {
     // A step applies the backscatter clipping inside its update kernel; here
     // it is applied on its own, so C_d comes back as the SFS model leaves it.

@@ -7,6 +7,7 @@
 #include <vector>
 
 #include "internal.h"
+#include "packed_records.h"
 #include "update.h"
 #include "vpm_device.cuh"
 
@@ -197,12 +198,11 @@ struct vpm_ctx {
   bool share_sort = false, sort_fresh = false;
   const int* sort_perm = nullptr;
   // Operations that may follow the pass being enqueued within its reduction, whether
-  // they did, and the pass whose packed records are in rec already (-1: none).
+  // they did, and what rec holds for the pass after it.
   const vpm::PostArgs* post = nullptr;
   bool post_taken = false;
   bool fine = false;              // PairCall::fine of the pass being enqueued
-  int rec_pass = -1;
-  double rec_scale = 1.0;
+  vpm::PackedRecords packed;
   double fd_alpha = 0.0;          // of the pair passes being enqueued (PairArgs::fd_alpha)
   double* srt = nullptr;          // Morton-ordered inputs: X3 Γ3 σ1 v3 w3 (13 rows of ld)
   double* sout = nullptr;         // Morton-ordered outputs: U3 J9 DJ9 or ζ sums (21 rows of ld)
