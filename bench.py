@@ -51,7 +51,7 @@ L2_FLUSH_BYTES = 256 << 20
 # last CTA of each tile sums the chunks' partial sums from L2 and drops
 # them there; what still reaches DRAM is partial sums evicted before their tile
 # was complete.  (With a separate reduction launch the partial sums took 1.8 GB.)
-PAIR_KERNEL_TRAFFIC = {(262144, "128x4"): 64656640 + 138696448}
+PAIR_KERNEL_TRAFFIC = {(262144, "128x4"): 43684608 + 112076032}
 
 
 def parse():

@@ -185,10 +185,10 @@ static int plan_cluster(int device, const PairCall& pc, Shape sh, int64_t n_tb,
 constexpr int kSmallWaves = 8;
 constexpr int kLargeWaves = 64;
 constexpr int64_t kLargeField = 131072;
-// Largest field whose reduction takes the particles' updates along: one block of 32
-// particles per SM.  With the updates one block fits on an SM, where the plain sum has
-// three; a larger field's reduction is bound by reading its partial sums and wants
-// those.  A step without SFS at 3,001 / 4,001 / 5,001 particles, launches of their own
+// Largest field whose reduction takes the particles' updates along: 128 blocks of 32
+// particles, less than one per SM.  With the updates one block fits on an SM, where the
+// plain sum has three; a larger field's reduction is bound by reading its partial sums and
+// wants those.  A step without SFS at 3,001 / 4,001 / 5,001 particles, launches of their own
 // against this: 103 / 145 / 186 and 100 / 137 / 203 µs.
 constexpr int64_t kPostInReduce = 4096;
 // Targets whose slots are summed in runs side by side (kReduceSegs): one block of 16

@@ -13,8 +13,8 @@
 //   - the far-field, coincidence and range tests on the bit patterns;
 //   - constants of the source staged once per tile.
 // Measured on GB300 (FP64 Gaussian-erf, two rings of 7,600 particles): U/J pass
-// 5.65 -> 4.09 ms, ζ pass 3.45 -> 2.18 ms; Winckelmans U/J of 4,096 particles 1.45 ->
-// 1.21 ms.
+// 5.63 -> 4.19 ms, ζ pass 3.46 -> 2.00 ms; Winckelmans U/J of 4,096 particles 1.45 ->
+// 1.23 ms.
 #pragma once
 
 #include "f64_tables.cuh"

@@ -21,13 +21,13 @@
 //      boxes), then it is evaluated from its moments; otherwise its leaves are
 //      summed directly, consecutive leaves merged into one range of particles
 //      (two passes: count, fill); with local expansions, far cells at least
-//      as large as the group are marked for them;
-//   5. local expansions (FP32, P = 4): the marked cells' moments turned into
+//      as large as the group go to a list for them;
+//   5. local expansions (FP32, P = 4): that list's moments turned into
 //      one local expansion of ψ per group (M2L, tree.cuh);
 //   6. the direct near field: runs of tiles of a group's near ranges, with the
 //      regularised kernels of the direct sum (FP32 pair routines on positions
 //      relative to the group's first particle, or FP64);
-//   7. the far field: one thread per target over the unmarked far cells of its
+//   7. the far field: one or two targets per thread over the far list of their
 //      group (M2P, tree.cuh); 5 and 7 run beside 6 on streams of their own;
 //   8. near field, far field and the local expansion at every target (L2P)
 //      added, in the original order.
@@ -1239,10 +1239,9 @@ __global__ void __launch_bounds__(kTreeBlock) near_f64_kernel(
 }
 
 // ------------------------------------------------------------ local expansions --
-// Far cells at least as large as their target group are marked in the far
-// list as ~s (negative) when local expansions are on: m2l_kernel turns them
-// into the group's local expansion (tree.cuh), far_kernel evaluates it at each
-// target (L2P) and skips them in its M2P loop.
+// With local expansions on, far cells at least as large as their target group go to a
+// list of their own (LIST_LOC): m2l_kernel turns them into the group's local expansion
+// (tree.cuh), which finish_kernel evaluates at each target (L2P).
 constexpr int kLocalOrder = 7;   // Q for P = 4: L2P within a few per cent of M2P in J (tree.cuh)
 
 // Two warps per target group.  The group's local-expansion cells are taken
